@@ -205,7 +205,8 @@ def run(state):
     if kind == "mixed":  # from the initial state to convergence
         state["h"].levels[0].upload(*state["start"])
         state["h"].solve(drop=1e-12, max_cycles=240, vw=state["vw"], mixed=True)
-        return state["out"]
+        # one vector: the converged flow is smooth, its high modes are small beside the rest
+        return torch.cat([a.reshape(-1) for a in state["out"].values()])
     if kind == "tet":  # sweeps, then the state back to the host (the level's only way out)
         g = state["level"]
         g.iterate(state["sweeps"])
