@@ -1,0 +1,508 @@
+// ins element residual, straight triangles, sum-factorised with one lane per triangle.
+//
+// tri_hp::rsdl's element loop (tri_hp/nstage.cpp:52-73: ugtouht, element_rsdl, lftog) with
+// tri_hp_ins::element_rsdl's straight-element branch (tri_hp/ins/rsdl.cpp:259-433) and the
+// tri_basis operators it calls (proj.cpp:22-119, intgrt.cpp:81-158, derivr / derivs
+// proj.cpp:339-402), FP64 or FP32, plain or correction form.
+//
+// A CTA takes batches of 32 triangles, lane = triangle, and has one warp per eta point j: a
+// thread owns the line (triangle, j) of the tensor-product points. Everything that is not per
+// triangle -- mode, point, table entry -- is then uniform across a warp, so the basis tables are
+// constant-bank operands of the FMAs, shared-memory rows of 32 lanes have no bank conflicts, and
+// no index is computed per lane; the point data of a line stay in its thread's registers.
+//   gather   modes -> U[var][mode][lane] (cp.async, one batch ahead; the connectivity two ahead)
+//   proj     the thread's column sums over the modes (value, d/deta), then its G points
+//   strong   x-direction part of the strong residual in registers; the s fluxes are exchanged
+//            through shared memory for the eta-direction part (warp = x point i there)
+//   SUPG     point by point
+//   intgrtrs per part: x-direction sums of the thread's line -> A, B [var][column][j], exchange,
+//            then every warp sums its share of the modes over j
+//   lftog    results staged [mode][var][lane], written with consecutive threads on
+//            consecutive addresses of the assembly slots (or atomics)
+// Why vector FMAs: on B200 the FP64 tensor instruction runs on the FP64 pipe at its rate (measured
+// 37.0 TFLOP/s against 34.5 for DFMA, and 31 in sum when mixed), so the dense per-point operators
+// that a fragment needs (98k flops per triangle at p = 6 with the padding) lose to the
+// sum-factorised form (about 40k). Measured, FP64, 131k triangles, full residual, against two
+// triangles per warp on mma.m8n8k4.f64: p = 3 157 -> 89 us, p = 4 308 -> 171, p = 5 503 -> 246,
+// p = 6 719 -> 421, p = 8 1884 -> 1108; p = 2 against the scalar warp kernel 197 -> 54. Bound by
+// issue: the FP64 pipe is busy 33 % (p = 6) to 41 % (p = 3) of the time; 7 to 16 warps an SM fit.
+#pragma once
+#include <utility>
+#include "hp_line.h"
+
+namespace hpb {
+
+template <typename R, int P, bool DIFF>
+struct LineCfg {
+    static constexpr int G = P + 1, GG = G * G, X = P + 2, T = (P + 1) * (P + 2) / 2, SM = P - 1,
+                         IM = (P - 1) * (P - 2) / 2, BM = 3 * P, NV = 3;
+    static constexpr int NTHR = 32 * G;
+    static constexpr int U = 0;               // gathered modes [3 T][33]
+    static constexpr int OUT = 3 * T * 33;    // results [3 T][33]
+    static constexpr int EX = 2 * 3 * T * 33; // s fluxes [3][G][G][32], then A, B [3][2][X][G][32]
+    static constexpr int LEN = EX + 6 * X * G * 32;
+    static constexpr int IDX = 15 * 32;       // connectivity of a batch: pnt, seg, sgn, vpos, spos [32][3] each
+    static constexpr int SMEM = LEN * (int)sizeof(R) + 3 * IDX * 4;
+    static constexpr int by_smem = 227 * 1024 / (SMEM + 1024);
+    // CTAs an SM, as many as leave the point data in registers (measured at 131k triangles, FP64:
+    // p = 4 with 1, 2, 3 CTAs 269, 198, 171 us, although 3 spill a little; p = 5 with 1, 2: 347, 246)
+    static constexpr int by_regs = G == 3 ? 5 : G == 4 ? 4 : G == 5 ? 3 : G == 6 ? 2 : 1;
+    static constexpr int MINB = by_smem < by_regs ? (by_smem < 1 ? 1 : by_smem) : by_regs;
+};
+
+template <typename R>
+struct alignas(2 * sizeof(R)) R2 {
+    R x, y;
+};
+
+// Tables of one (precision, p), a kernel parameter. The first index of g and w is the warp's (its
+// eta point; the mode it sums), the others are compile-time. Every entry is used for the three
+// variables at once: an FP64 FMA whose constant is loaded for it alone runs at under half rate
+// (measured: 15 TFLOP/s with one use of each constant, 30 with three).
+template <typename R, int P>
+struct LineTab {
+    static constexpr int G = P + 1, X = P + 2, T = (P + 1) * (P + 2) / 2;
+    R2<R> g[G][T];                     // proj, mode sums: gn, dgn
+    R2<R> w[T][G];                     // intgrtrs, eta-direction: gnwtnn0, dgnwtn, with its minus sign
+    R gx[G][X], dgx[G][X];             // proj, column sums to point i
+    R ar[G][G], as1[G][G], as2[G][G];  // derivr / derivs: 1D derivative operators
+    R dgxw[X][G], gxw[X][G];           // intgrtrs, x-direction
+    R x0[G], n0[G];
+    // intgrtrs, eta-direction: warp w sums items iptr[w] .. iptr[w + 1] - 1; an item is the column
+    // icol and its modes mode[ifst[item] .. ifst[item + 1] - 1]
+    unsigned char iptr[G + 1], icol[G + X], ifst[G + X + 1], mode[T];
+};
+
+template <typename R>
+__device__ __forceinline__ R line_tau0(R c, R gam);
+template <>
+__device__ __forceinline__ double line_tau0<double>(double c, double gam) { return c * rsqrt(gam); }
+template <>
+__device__ __forceinline__ float line_tau0<float>(float c, float gam) { return c / sqrtf(gam); }
+
+// f(0), ..., f(N - 1) with compile-time arguments: the column of a mode is then a constant, so the
+// column sums stay in registers (a loop does not fold ModeCols::col beyond p = 4)
+template <typename F, int... M>
+__device__ __forceinline__ void each_mode(F &&f, std::integer_sequence<int, M...>) {
+    (f(std::integral_constant<int, M>{}), ...);
+}
+
+// An optimisation barrier on a register: what depends on it is computed again.
+__device__ __forceinline__ void opaque(double &x) { asm volatile("" : "+d"(x)); }
+__device__ __forceinline__ void opaque(float &x) { asm volatile("" : "+f"(x)); }
+
+template <int BYTES>
+__device__ __forceinline__ void cp_async(void *dst, const void *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
+                 "n"(BYTES));
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+template <typename R, int P, bool DIFF, bool RE>
+__global__ void __launch_bounds__(LineCfg<R, P, DIFF>::NTHR, LineCfg<R, P, DIFF>::MINB)
+    k_rsdl_ins_line(const __grid_constant__ LineTab<R, P> tab, Mesh mesh, State<R> st, R beta, R omb, R rho, R mu,
+                    double nu2, double adis, int gfloor) {
+    using C = LineCfg<R, P, DIFF>;
+    constexpr int G = C::G, X = C::X, T = C::T, SM = C::SM, IM = C::IM, BM = C::BM, NV = 3, NTHR = C::NTHR;
+    constexpr int IMD = IM > 0 ? IM : 1;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    R *sm = reinterpret_cast<R *>(smem_raw);
+    R *out = sm + C::OUT;
+    int *ring = reinterpret_cast<int *>(sm + C::LEN);
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int j = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    // the thread index anew: the indices of the copy loops are computed in each batch and not kept
+    // in registers across the loop over batches
+    auto fresh_tid = [&]() {
+        int t = tid;
+        asm volatile("" : "+r"(t));
+        return t;
+    };
+    const int nbatch = (mesh.ntri + 31) / 32, last = mesh.ntri - 1;
+    // connectivity of batch b into ring slot s (lanes past the last triangle repeat it)
+    auto fetch_idx = [&](int b, int s) {
+        if (b >= nbatch) return;
+        const int tid = fresh_tid();
+        int *d = ring + s * C::IDX;
+        for (int w = tid; w < C::IDX; w += NTHR) {
+            const int a = w / 96, r = w - a * 96, e = r / 3, c = r - e * 3;
+            const int *src = a == 0 ? mesh.tri_pnt : a == 1 ? mesh.tri_seg : a == 2 ? mesh.tri_sgn : a == 3 ? mesh.vpos : mesh.spos;
+            cp_async<4>(d + w, src + 3 * (size_t)min(b * 32 + e, last) + c);
+        }
+    };
+    // modes of batch b (ugtouht, gtol.cpp:14-55; the signs of the side modes are applied when
+    // they are read), one mode kind per loop, consecutive threads on consecutive values
+    auto fetch_u = [&](int b, int s) {
+        if (b >= nbatch) return;
+        const int tid = fresh_tid();
+        const int *d = ring + s * C::IDX;
+#pragma unroll
+        for (int it = 0; it < (32 * 9 + NTHR - 1) / NTHR; ++it) {
+            const int w = tid + it * NTHR;
+            if (w >= 32 * 9) break;
+            const int e = w / 9, r = w - e * 9, m = r / NV, n = r - m * NV;
+            cp_async<sizeof(R)>(sm + (n * T + m) * 33 + e, st.ugv + (size_t)d[3 * e + m] * NV + n);
+        }
+        constexpr int NS = 96 * SM * NV;
+#pragma unroll
+        for (int it = 0; it < (NS + NTHR - 1) / NTHR; ++it) {
+            const int w = tid + it * NTHR;
+            if (w >= NS) break;
+            const int q = w / (SM * NV), r = w - q * (SM * NV), e = q / 3, i = q - e * 3, k = r / NV, n = r - k * NV;
+            cp_async<sizeof(R)>(sm + (n * T + 3 + i * SM + k) * 33 + e, st.ugs + (size_t)d[96 + q] * (SM * NV) + r);
+        }
+        if constexpr (IM > 0) {
+            constexpr int NI = 32 * IM * NV;
+#pragma unroll
+            for (int it = 0; it < (NI + NTHR - 1) / NTHR; ++it) {
+                const int w = tid + it * NTHR;
+                if (w >= NI) break;
+                const int e = w / (IMD * NV), r = w - e * (IMD * NV), k = r / NV, n = r - k * NV;
+                cp_async<sizeof(R)>(sm + (n * T + BM + k) * 33 + e, st.ugi + (size_t)min(b * 32 + e, last) * (IMD * NV) + r);
+            }
+        }
+    };
+    const int step = gridDim.x;
+    int b = blockIdx.x, slot = 0;
+    fetch_idx(b, 0);
+    fetch_idx(b + step, 1);
+    cp_async_wait();
+    __syncthreads();
+    fetch_u(b, 0);
+    for (; b < nbatch; b += step, slot = slot == 2 ? 0 : slot + 1) {
+        const int *idx = ring + slot * C::IDX;
+        const int t0 = b * 32;
+        // per-triangle constants (Mesh::lgeo): ldcrd, 1 / |J|, tau length scale h, 1 / h
+        const double *lg = mesh.lgeo + (size_t)b * (kLineGeo * 32) + lane;
+        const R d00 = (R)lg[0], d01 = (R)lg[32], d10 = (R)lg[64], d11 = (R)lg[96];
+        const R cm = RE ? (R)(-(double)mu * lg[128]) : (R)0;
+        const R c5 = RE ? (R)(nu2 * lg[192]) : (R)0, c6 = RE ? (R)(adis * lg[160] * lg[128]) : (R)0;
+        R bu[DIFF ? G : 1], bv[DIFF ? G : 1];
+        if constexpr (DIFF) {
+            const R *bp = st.bpt + (size_t)b * (2 * G * G * 32) + lane;
+#pragma unroll
+            for (int i = 0; i < G; ++i) {
+                bu[i] = bp[(i * G + j) * 32];
+                bv[i] = bp[(G * G + i * G + j) * 32];
+            }
+        }
+        cp_async_wait();
+        __syncthreads();
+        R uq[G], vq[G], pq[G], xx[RE ? G : 1], xy[RE ? G : 1], yy[RE ? G : 1];
+        // ---- proj (proj.cpp:22-119): column sums of the thread's line, then its points: u, v, p
+        //      and the viscous stress -mu (2 u_x, u_y + v_x, 2 v_y)
+        {
+            R wu[X], wv[X], wp[X], wu1[X], wv1[X];
+#pragma unroll
+            for (int c = 0; c < X; ++c) wu[c] = wv[c] = wp[c] = wu1[c] = wv1[c] = (R)0;
+            int jl = j;  // anew in each batch: the line's table entries are not kept across the loop
+            asm volatile("" : "+r"(jl));
+            const bool neg[3] = {idx[192 + 3 * lane] < 0, idx[192 + 3 * lane + 1] < 0, idx[192 + 3 * lane + 2] < 0};
+            each_mode([&](auto mm) {
+                constexpr int m = decltype(mm)::value, c = ModeCols<P>::col(m);
+                R x = sm[m * 33 + lane], y = sm[(T + m) * 33 + lane], z = sm[(2 * T + m) * 33 + lane];
+                if constexpr (m >= 3 && m < BM && (((m - 3) % (SM > 0 ? SM : 1)) & 1)) {
+                    const bool ng = neg[(m - 3) / SM];
+                    x = ng ? -x : x;
+                    y = ng ? -y : y;
+                    z = ng ? -z : z;
+                }
+                const R2<R> g = tab.g[jl][m];
+                wu[c] += x * g.x;
+                wv[c] += y * g.x;
+                wp[c] += z * g.x;
+                if constexpr (RE) {
+                    wu1[c] += x * g.y;
+                    wv1[c] += y * g.y;
+                }
+            }, std::make_integer_sequence<int, T>{});
+            const R n0 = tab.n0[j];
+#pragma unroll
+            for (int i = 0; i < G; ++i) {
+                R u = (R)0, v = (R)0, p = (R)0;
+#pragma unroll
+                for (int c = 0; c < X; ++c) {
+                    u += wu[c] * tab.gx[i][c];
+                    v += wv[c] * tab.gx[i][c];
+                    p += wp[c] * tab.gx[i][c];
+                }
+                uq[i] = u;
+                vq[i] = v;
+                pq[i] = p;
+                if constexpr (RE) {
+                    R ur = (R)0, vr = (R)0, us = (R)0, vs = (R)0;
+#pragma unroll
+                    for (int c = 0; c < X; ++c) {
+                        ur += wu[c] * tab.dgx[i][c];
+                        vr += wv[c] * tab.dgx[i][c];
+                        us += wu1[c] * tab.gx[i][c];
+                        vs += wv1[c] * tab.gx[i][c];
+                    }
+                    ur *= n0;
+                    vr *= n0;
+                    us += tab.x0[i] * ur;
+                    vs += tab.x0[i] * vr;
+                    xx[i] = (cm + cm) * (d11 * ur - d10 * us);
+                    xy[i] = cm * ((d00 * us - d01 * ur) + (d11 * vr - d10 * vs));
+                    yy[i] = (cm + cm) * (d00 * vs - d01 * vr);
+                }
+            }
+        }
+        // convective flux (r, s components) of u and v at point i without the pressure, and the
+        // mass flux; correction form: F(b + d) - F(b) with the products expanded
+        auto conv = [&](int i, R &m0, R &m1, R &r0, R &s0, R &r1, R &s1) {
+            const R u = uq[i], v = vq[i];
+            m0 = rho * (d11 * u - d01 * v);
+            m1 = rho * (d00 * v - d10 * u);
+            if constexpr (DIFF) {
+                const R e0 = rho * (d11 * bu[i] - d01 * bv[i]), e1 = rho * (d00 * bv[i] - d10 * bu[i]);
+                const R f0 = bu[i] + u, f1 = bv[i] + v;
+                r0 = f0 * m0 + u * e0;
+                s0 = f0 * m1 + u * e1;
+                r1 = f1 * m0 + v * e0;
+                s1 = f1 * m1 + v * e1;
+            } else {
+                r0 = u * m0;
+                s0 = u * m1;
+                r1 = v * m0;
+                s1 = v * m1;
+            }
+        };
+        R pr[RE ? 3 : 1][RE ? G : 1], ps[RE ? 3 : 1][RE ? G : 1];  // real flux pairs of the line: fr + x0 fs, fs
+        if constexpr (RE) {
+            // ---- strong residual (derivr + derivs of the full fluxes, proj.cpp:339-402):
+            //      res(i, j) = n0(j) (sum_q Ar(i, q) fr(q, j) + As1(i, q) fs(q, j)) + sum_l As2(j, l) fs(i, l)
+            R res[3][G];
+            R *ex = sm + C::EX + j * 32 + lane;  // s flux n at point i: ex[(n G + i) G 32]
+#pragma unroll
+            for (int n = 0; n < 3; ++n)
+#pragma unroll
+                for (int i = 0; i < G; ++i) res[n][i] = (R)0;
+#pragma unroll
+            for (int q = 0; q < G; ++q) {
+                R m0, m1, r0, s0, r1, s1;
+                conv(q, m0, m1, r0, s0, r1, s1);
+                const R px = xx[q] + pq[q], py = yy[q] + pq[q];
+                r0 += d11 * px - d01 * xy[q];
+                s0 += d00 * xy[q] - d10 * px;
+                r1 += d11 * xy[q] - d01 * py;
+                s1 += d00 * py - d10 * xy[q];
+                ex[(q * G) * 32] = s0;
+                ex[((G + q) * G) * 32] = s1;
+                ex[((2 * G + q) * G) * 32] = m1;
+#pragma unroll
+                for (int i = 0; i < G; ++i) {
+                    res[0][i] += tab.ar[i][q] * r0 + tab.as1[i][q] * s0;
+                    res[1][i] += tab.ar[i][q] * r1 + tab.as1[i][q] * s1;
+                    res[2][i] += tab.ar[i][q] * m0 + tab.as1[i][q] * m1;
+                }
+            }
+            __syncthreads();  // (the gathered modes are dead, too)
+            fetch_u(b + step, slot == 2 ? 0 : slot + 1);
+            fetch_idx(b + 2 * step, slot == 0 ? 2 : slot - 1);
+            // eta-direction part, warp = x point: in place on the exchanged rows
+            {
+                R *f = sm + C::EX + (j * G) * 32 + lane;
+                R s[3][G];
+#pragma unroll
+                for (int n = 0; n < 3; ++n)
+#pragma unroll
+                    for (int l = 0; l < G; ++l) s[n][l] = f[(n * G * G + l) * 32];
+#pragma unroll
+                for (int k = 0; k < G; ++k) {
+                    R a[3] = {(R)0, (R)0, (R)0};
+#pragma unroll
+                    for (int l = 0; l < G; ++l)
+#pragma unroll
+                        for (int n = 0; n < 3; ++n) a[n] += tab.as2[k][l] * s[n][l];
+#pragma unroll
+                    for (int n = 0; n < 3; ++n) f[(n * G * G + k) * 32] = a[n];
+                }
+            }
+            __syncthreads();
+            // ---- SUPG (ins/rsdl.cpp:341-431, CALC_TAU2; tau of the base in correction form): real
+            //      pairs, viscous minus SUPG for u, v and the continuity term for p
+            const R n0 = tab.n0[j];
+#pragma unroll
+            for (int i = 0; i < G; ++i) {
+                R u = uq[i], v = vq[i], qv;
+                if constexpr (DIFF) {
+                    qv = bu[i] * bu[i] + bv[i] * bv[i];
+                    u += bu[i];
+                    v += bv[i];
+                } else {
+                    qv = u * u + v * v;
+                }
+                R gam = (R)3 * qv + c5 * c5;
+                if (gfloor) gam = gam > (R)0.1 ? gam : (R)0.1;
+                const R tau0 = line_tau0<R>(c6, gam), tau2 = sqrt(qv) * tau0;
+                const R a0 = tau0 * (n0 * res[0][i] + ex[(i * G) * 32]), a1 = tau0 * (n0 * res[1][i] + ex[((G + i) * G) * 32]),
+                        a2 = tau2 * (n0 * res[2][i] + ex[((2 * G + i) * G) * 32]);
+                // physical SUPG fluxes: x-momentum (2 u a0 + a2, v a0 + u a1), y-momentum
+                // (v a0 + u a1, 2 v a1 + a2), continuity (a0, a1)
+                const R sxx = xx[i] - ((u + u) * a0 + a2), sxy = xy[i] - (v * a0 + u * a1),
+                        syy = yy[i] - ((v + v) * a1 + a2);
+                pr[0][i] = d11 * sxx - d01 * sxy;
+                ps[0][i] = d00 * sxy - d10 * sxx;
+                pr[1][i] = d11 * sxy - d01 * syy;
+                ps[1][i] = d00 * syy - d10 * sxy;
+                pr[2][i] = d01 * a1 - d11 * a0;
+                ps[2][i] = d10 * a0 - d00 * a1;
+#pragma unroll
+                for (int n = 0; n < 3; ++n) pr[n][i] += tab.x0[i] * ps[n][i];
+            }
+            __syncthreads();  // A, B take the place of the exchanged rows
+        }
+        // ---- intgrtrs (intgrt.cpp:81-158): x-direction sums of the three flux pairs, given by
+        //      pair(i, fr + x0 fs, fs), half of the columns at a time (their sums share the registers)
+        auto xsums = [&](auto &&pair) {
+            constexpr int XH = (X + 1) / 2;
+            R *ab = sm + C::EX + j * 32 + lane;  // A of (n, c): row (2 n X + c) G, B X rows further
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                R a[3][XH], bb[3][XH];
+#pragma unroll
+                for (int n = 0; n < 3; ++n)
+#pragma unroll
+                    for (int c = 0; c < XH; ++c) a[n][c] = bb[n][c] = (R)0;
+#pragma unroll
+                for (int i = 0; i < G; ++i) {
+                    R fr[3], fs[3];
+                    pair(i, fr, fs);
+#pragma unroll
+                    for (int c = 0; c < XH; ++c)
+                        if (h * XH + c < X)
+#pragma unroll
+                            for (int n = 0; n < 3; ++n) {
+                                a[n][c] += tab.dgxw[h * XH + c][i] * fr[n];
+                                bb[n][c] += tab.gxw[h * XH + c][i] * fs[n];
+                            }
+                }
+#pragma unroll
+                for (int n = 0; n < 3; ++n)
+#pragma unroll
+                    for (int c = 0; c < XH; ++c)
+                        if (h * XH + c < X) {
+                            ab[((n * 2 * X + h * XH + c) * G) * 32] = a[n][c];
+                            ab[((n * 2 * X + X + h * XH + c) * G) * 32] = bb[n][c];
+                        }
+            }
+        };
+        // eta-direction sums of the warp's modes into the staging rows
+        auto esums = [&](R scale) {
+#pragma unroll 1
+            for (int it = tab.iptr[j]; it < tab.iptr[j + 1]; ++it) {
+                const R *pa = sm + C::EX + (tab.icol[it] * G) * 32 + lane;
+                R a[3][G], bb[3][G];
+#pragma unroll
+                for (int n = 0; n < 3; ++n)
+#pragma unroll
+                    for (int k = 0; k < G; ++k) {
+                        a[n][k] = pa[(n * 2 * X * G + k) * 32];
+                        bb[n][k] = pa[((n * 2 * X + X) * G + k) * 32];
+                    }
+#pragma unroll 1
+                for (int q = tab.ifst[it]; q < tab.ifst[it + 1]; ++q) {
+                    const int m = tab.mode[q];
+                    R s0[3] = {(R)0, (R)0, (R)0}, s1[3] = {(R)0, (R)0, (R)0};
+#pragma unroll
+                    for (int k = 0; k < G; ++k) {
+                        const R2<R> w = tab.w[m][k];
+#pragma unroll
+                        for (int n = 0; n < 3; ++n) {
+                            s0[n] += w.x * a[n][k];
+                            s1[n] += w.y * bb[n][k];
+                        }
+                    }
+#pragma unroll
+                    for (int n = 0; n < 3; ++n) out[(m * NV + n) * 33 + lane] = scale * (s0[n] + s1[n]);
+                }
+            }
+        };
+        xsums([&](int i, R (&fr)[3], R (&fs)[3]) {
+            conv(i, fr[2], fs[2], fr[0], fs[0], fr[1], fs[1]);
+            fr[0] += d11 * pq[i];
+            fs[0] -= d10 * pq[i];
+            fr[1] -= d01 * pq[i];
+            fs[1] += d00 * pq[i];
+#pragma unroll
+            for (int n = 0; n < 3; ++n) fr[n] += tab.x0[i] * fs[n];
+            // the second half of the columns forms the fluxes again instead of keeping them
+            opaque(uq[i]);
+            opaque(vq[i]);
+        });
+        // lftog (gtol.cpp:364-402); curved triangles are done by the curved launch. The interior
+        // values of the imaginary part wait in registers for the real part.
+        constexpr int NKEEP = (32 * IM * NV + NTHR - 1) / NTHR;
+        R keep[NKEEP > 0 ? NKEEP : 1];
+        auto act = [&](int e) { return t0 + e <= last && (!mesh.tri_cv || mesh.tri_cv[t0 + e] < 0); };
+        auto scatter = [&](int part) {
+            const int tid = fresh_tid();
+            R *el = part ? st.elre : st.elim;
+#pragma unroll
+            for (int it = 0; it < (32 * 9 + NTHR - 1) / NTHR; ++it) {
+                const int w = tid + it * NTHR;
+                if (w >= 32 * 9) break;
+                const int e = w / 9, r = w - e * 9, m = r / NV, n = r - m * NV;
+                if (!act(e)) continue;
+                const R val = out[r * 33 + e];
+                if (el) el[(size_t)idx[288 + 3 * e + m] * NV + n] = val;
+                else atomic_add((part ? st.rrv : st.resv) + (size_t)idx[3 * e + m] * NV + n, val);
+            }
+            constexpr int NS = 96 * SM * NV;
+#pragma unroll
+            for (int it = 0; it < (NS + NTHR - 1) / NTHR; ++it) {
+                const int w = tid + it * NTHR;
+                if (w >= NS) break;
+                const int q = w / (SM * NV), r = w - q * (SM * NV), e = q / 3, i = q - e * 3, k = r / NV;
+                if (!act(e)) continue;
+                R val = out[((3 + i * SM) * NV + r) * 33 + e];
+                if ((k & 1) && idx[192 + q] < 0) val = -val;
+                if (el) el[(size_t)3 * mesh.ntri * NV + (size_t)idx[384 + q] * (SM * NV) + r] = val;
+                else atomic_add((part ? st.rrs : st.ress) + (size_t)idx[96 + q] * (SM * NV) + r, val);
+            }
+            if constexpr (IM > 0) {
+#pragma unroll
+                for (int it = 0; it < NKEEP; ++it) {
+                    const int w = tid + it * NTHR;
+                    if (w >= 32 * IM * NV) break;
+                    const int e = w / (IMD * NV), r = w - e * (IMD * NV);
+                    if (!act(e)) continue;
+                    const R val = out[(BM * NV + r) * 33 + e];
+                    const size_t gi = (size_t)t0 * (IMD * NV) + w;
+                    const R rr = omb != (R)0 && (part || !RE) ? st.rri[gi] * omb : (R)0;
+                    if (part) {
+                        st.rri[gi] = rr + val;
+                        st.resi[gi] = keep[it] + (rr + val);
+                    } else {
+                        keep[it] = st.dresi ? val + st.dresi[gi] : val;
+                        if constexpr (!RE) st.resi[gi] = keep[it] + rr;  // res_r unchanged when beta = 0
+                    }
+                }
+            }
+        };
+        __syncthreads();
+        if constexpr (!RE) {
+            fetch_u(b + step, slot == 2 ? 0 : slot + 1);
+            fetch_idx(b + 2 * step, slot == 0 ? 2 : slot - 1);
+        }
+        esums((R)1);
+        __syncthreads();
+        scatter(0);
+        if constexpr (RE) {
+            xsums([&](int i, R (&fr)[3], R (&fs)[3]) {
+#pragma unroll
+                for (int n = 0; n < 3; ++n) {
+                    fr[n] = pr[n][i];
+                    fs[n] = ps[n][i];
+                }
+            });
+            __syncthreads();
+            esums(beta);
+            __syncthreads();
+            scatter(1);
+        }
+    }
+}
+
+}  // namespace hpb

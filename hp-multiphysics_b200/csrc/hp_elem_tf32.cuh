@@ -5,8 +5,8 @@
 // R(b + d) - R(b) + R64(u) about the base state b = fp32(u) (tri_hp::mg_source's shape,
 // tri_hp/nstage.cpp:113-129, with R64 as the source): the convective and pressure fluxes
 // as exact differences F(b + d) - F(b), the viscous flux (linear) of d, the SUPG term with
-// the tau of the base. Same element loop and basis operators as the FP64 tensor-core
-// kernel (hp_elem_mma.cuh; tri_hp/ins/rsdl.cpp:259-433, proj.cpp:22-119,
+// the tau of the base. Same element loop and basis operators as the FP64 line
+// kernel (hp_elem_line.cuh; tri_hp/ins/rsdl.cpp:259-433, proj.cpp:22-119,
 // intgrt.cpp:81-158, proj.cpp:339-402), four triangles per warp: the 16 rows of an
 // m16n8k8 fragment are (triangle, variable) pairs. The contractions round their
 // operands to TF32 (10-bit mantissa) and accumulate in FP32: the smoother's residual is
@@ -18,6 +18,15 @@
 #include "hp_kernels.cuh"
 
 namespace hpb {
+
+// The 1D derivative tables of derivr / derivs and the collapsed-coordinate factors.
+template <typename R, int P>
+struct InsSmall {
+    R dltx[P + 1], dltx1[P + 1][P + 1], dltn[P + 1], dltn1[P + 1][P + 1], dltn2[P + 1][P + 1];
+    R n0[P + 1], x0[P + 1];
+};
+template <int P>
+using InsMmaSmallF = InsSmall<float, P>;
 
 template <int P>
 struct InsTf32 {

@@ -17,9 +17,9 @@
 #include "hp_host.h"
 #include "hp_mlp.h"
 #include "hp_kernels.cuh"
-#include "hp_elem_mma.cuh"
 #include "hp_elem_p1.cuh"
 #include "hp_elem_tf32.cuh"
+#include "hp_line.h"
 
 using namespace hpb;
 
@@ -91,89 +91,8 @@ void fill_tables(const hp_basis_tables &b, DevTables<R, P> &t) {
     t.colstart[X] = c;
 }
 
-// Dense per-point forms of tri_basis::proj (value, d/dr, d/ds; proj.cpp:22-119) and
-// intgrtrs (intgrt.cpp:81-158) for the tensor-core ins kernel, in DMMA fragment order
-// (B operand of mma.m8n8k4 .row.col: lane l holds B[k = l & 3][n = l >> 2]). Point
-// q = i * G + j (i along the x-direction Gauss points, j along eta). With c = the column
-// of mode m in the sum factorisation:
-//   value(q, m) = gn(j, m) gx(i, c)
-//   d/dr (q, m) = n0(j) gn(j, m) dgx(i, c)
-//   d/ds (q, m) = dgn(j, m) gx(i, c) + x0(i) d/dr(q, m)
-//   W_r(q, m)   = -dgxwtx(c, i) gnwtnn0(m, j)
-//   W_s(q, m)   = -(x0(i) dgxwtx(c, i) gnwtnn0(m, j) + gxwtx(c, i) dgnwtn(m, j))
-// so that lf(m) = sum_q flux_r(q) W_r(q, m) + flux_s(q) W_s(q, m) is intgrtrs' result.
-// The 1D derivative operators of derivr / derivs (proj.cpp:339-402) as matrices, so that
-// the strong residual at point (i, j) is
-//   res(i, j) = n0(j) (sum_q Ar(i, q) flux_r(q, j) + sum_q As1(i, q) flux_s(q, j))
-//             + sum_l As2(j, l) flux_s(i, l), with (which = 0: Ar, 1: As1, 2: As2)
-//   Ar(i, q)  = q == i ? dltx(i) sum_{q' != i} dltx1(i, q') : dltx(q) dltx1(i, q)
-//   As1(i, q) = q == i ? dltx(i) sum_{q' != i} dltn1(i, q') : dltx(q) dltn1(i, q)
-//   As2(j, l) = l == j ? dltn(j) sum_{l' != j} dltn2(j, l') : dltn(l) dltn2(j, l).
-inline double deriv_op(const hp_basis_tables &b, int G, int which, int r, int k) {
-    if (r >= G || k >= G) return 0.0;
-    auto tab = [&](int a, int c) {
-        return which == 0 ? b.dltx1[a][c] : (which == 1 ? b.dltn1[a][c] : b.dltn2[a][c]);
-    };
-    const double *dl = which == 2 ? b.dltn : b.dltx;
-    if (k != r) return dl[k] * tab(r, k);
-    double sum = 0.0;
-    for (int c = 0; c < G; ++c)
-        if (c != r) sum += tab(r, c);
-    return dl[r] * sum;
-}
-
-template <int P>
-void build_ins_mma(const hp_basis_tables &b, std::vector<double> &ops, InsMmaSmall<P> &sm) {
-    using M = InsMma<P>;
-    constexpr int G = M::G, GG = M::GG, T = M::T;
-    ops.assign(M::PROJ_LEN + M::INT_LEN + M::DER_LEN, 0.0);
-    for (int op = 0; op < 3; ++op)
-        for (int nt = 0; nt < M::NT; ++nt)
-            for (int ks = 0; ks < M::KS; ++ks)
-                for (int l = 0; l < 32; ++l) {
-                    const int q = nt * 8 + (l >> 2), m = ks * 4 + (l & 3);
-                    if (q >= GG || m >= T) continue;
-                    const int i = q / G, j = q - i * G, c = ModeCols<P>::col(m);
-                    const double dr = b.n0[j] * b.gn[j][m] * b.dgx[i][c];
-                    const double v = op == 0 ? b.gn[j][m] * b.gx[i][c]
-                                             : (op == 1 ? dr : b.dgn[j][m] * b.gx[i][c] + b.x0[i] * dr);
-                    ops[((size_t)(op * M::NT + nt) * M::KS + ks) * 32 + l] = v;
-                }
-    double *ib = ops.data() + M::PROJ_LEN;
-    for (int nt = 0; nt < M::NT2; ++nt)
-        for (int ks = 0; ks < M::KS2; ++ks)
-            for (int l = 0; l < 32; ++l) {
-                const int k = ks * 4 + (l & 3), m = nt * 8 + (l >> 2);
-                if (k >= 2 * GG || m >= T) continue;
-                const int q = k % GG, i = q / G, j = q - i * G, c = ModeCols<P>::col(m);
-                const double w = k < GG ? -b.dgxwtx[c][i] * b.gnwtnn0[m][j]
-                                        : -(b.x0[i] * b.dgxwtx[c][i] * b.gnwtnn0[m][j] + b.gxwtx[c][i] * b.dgnwtn[m][j]);
-                ib[((size_t)nt * M::KS2 + ks) * 32 + l] = w;
-            }
-    // A fragments of the 1D derivative operators (lane l holds A[row = l >> 2][k = l & 3]):
-    // [Ar | As1] per m-tile over 2 KR k-steps, then As2 over KR k-steps
-    double *db = ops.data() + M::PROJ_LEN + M::INT_LEN;
-    for (int mt = 0; mt < M::MT; ++mt)
-        for (int ks = 0; ks < 2 * M::KR; ++ks)
-            for (int l = 0; l < 32; ++l) {
-                const int blk = ks / M::KR, r = mt * 8 + (l >> 2), k = (ks - blk * M::KR) * 4 + (l & 3);
-                db[((size_t)mt * 2 * M::KR + ks) * 32 + l] = deriv_op(b, G, blk, r, k);
-            }
-    double *da = db + M::MT * 2 * M::KR * 32;
-    for (int mt = 0; mt < M::MT; ++mt)
-        for (int ks = 0; ks < M::KR; ++ks)
-            for (int l = 0; l < 32; ++l)
-                da[((size_t)mt * M::KR + ks) * 32 + l] = deriv_op(b, G, 2, mt * 8 + (l >> 2), ks * 4 + (l & 3));
-    for (int i = 0; i < G; ++i) {
-        sm.dltx[i] = b.dltx[i]; sm.dltn[i] = b.dltn[i]; sm.n0[i] = b.n0[i]; sm.x0[i] = b.x0[i];
-        for (int q = 0; q < G; ++q) {
-            sm.dltx1[i][q] = b.dltx1[i][q]; sm.dltn1[i][q] = b.dltn1[i][q]; sm.dltn2[i][q] = b.dltn2[i][q];
-        }
-    }
-}
-
-// The dense operators of the p = 1 point kernel (k_rsdl_ins_p1), the same entries as
-// build_ins_mma's at G = 2, T = 3, indexed by point q = 2 i + j.
+// The dense operators of the p = 1 point kernel (k_rsdl_ins_p1), indexed by point q = 2 i + j, see
+// InsP1Ops.
 template <typename R>
 void build_ins_p1(const hp_basis_tables &b, InsP1Ops<R> &o) {
     constexpr int G = 2;
@@ -208,7 +127,8 @@ float to_tf32(double v) {
     return f;
 }
 
-// The same dense operators as build_ins_mma for the TF32 kernel (mma.m16n8k8 .row.col:
+// Dense per-point forms of tri_basis::proj (value, d/dr, d/ds; proj.cpp:22-119) and intgrtrs
+// (intgrt.cpp:81-158) for the TF32 kernel (mma.m16n8k8 .row.col:
 // lane l holds B[k = l & 3][n = l >> 2] and B[k = (l & 3) + 4][n = l >> 2], stored as one
 // float2 per lane per MMA), rounded to TF32.
 template <int P>
@@ -324,13 +244,14 @@ struct Launchers {
                        const Tune &, cudaStream_t);
     void (*elem_jac)(const void *tab, const Mesh &, const State<R> &, const Phys &, R *K, R *rbar, int nsm,
                      cudaStream_t);
-    // FP64 ins only: the tensor-core element kernel (k_rsdl_ins_mma) with its operators
-    // (mma_build: dense operators in fragment order + the small derivative tables) and
-    // the curved elements through the scalar kernel
-    // (FP64: DMMA k_rsdl_ins_mma; FP32: TF32 k_rsdl_ins_tf32, plain or correction form)
+    // FP32 ins: the tensor-core element kernel (TF32 k_rsdl_ins_tf32) with its operators
+    // (mma_build: dense operators in fragment order + the small derivative tables)
     void (*elem_mma)(const void *ops, const void *small, const void *tab, const Mesh &, const State<R> &,
                      const Phys &, int stage, int zero_rr, int diff, int nsm, const Tune &, cudaStream_t);
     void (*mma_build)(const hp_basis_tables &, std::vector<unsigned char> &ops, std::vector<unsigned char> &small);
+    // the curved elements alone, by the scalar kernel (nothing when the mesh has none)
+    void (*curved)(const void *tab, const Mesh &, const State<R> &, const Phys &, int stage, int zero_rr, int diff,
+                   int nsm, const Tune &, cudaStream_t);
     // FP32 ins: the base state's point values for the correction form (State::bpt)
     void (*base_pts)(const void *tab, const Mesh &, const State<R> &, R *bpt, cudaStream_t);
     int bpt_per_elem;  // 2 GG
@@ -467,28 +388,16 @@ struct LaunchImpl {
             k_minv_vert<R, NV><<<nblk(m.npnt, th), th, 0, st>>>(m, s, mt, sm, im, (R)cfla, upd, fold, slot);
         }
     }
-    static constexpr bool HAS_MMA = PHYS == 1;
     static constexpr bool DBL = std::is_same<R, double>::value;
+    static constexpr bool HAS_MMA = PHYS == 1 && !DBL;
     static int mma_smem() {
-        if constexpr (DBL)
-            return (int)(((sizeof(InsMmaSmall<P>) + 15) / 16) * 16 + (size_t)2 * InsMma<P>::S_EL * InsMma<P>::WPC * 8 +
-                         InsMma<P>::SMEM_GEO + InsMma<P>::SMEM_IDX);
-        else
-            return (int)(((sizeof(InsMmaSmallF<P>) + 15) / 16) * 16 + (size_t)4 * InsTf32<P>::S_EL * InsTf32<P>::WPC * 4 +
-                         InsTf32<P>::SMEM_IDX);
+        return (int)(((sizeof(InsMmaSmallF<P>) + 15) / 16) * 16 + (size_t)4 * InsTf32<P>::S_EL * InsTf32<P>::WPC * 4 +
+                     InsTf32<P>::SMEM_IDX);
     }
     static void elem_mma(const void *ops, const void *small, const void *tab, const Mesh &m, const State<R> &s,
                          const Phys &ph, int stage, int zero_rr, int diff, int nsm, const Tune &tn, cudaStream_t st) {
         if constexpr (HAS_MMA) {
-            if constexpr (DBL) {
-                using MM = InsMma<P>;
-                const double *o = static_cast<const double *>(ops);
-                const long npair = ((long)m.ntri + 1) / 2;
-                const int blocks = (int)std::min<long>((npair + MM::WPC - 1) / MM::WPC, (long)nsm * MM::MINB * 4);
-                k_rsdl_ins_mma<P><<<blocks, MM::WPC * 32, mma_smem(), st>>>(
-                    o, o + MM::PROJ_LEN, o + MM::PROJ_LEN + MM::INT_LEN, *static_cast<const InsMmaSmall<P> *>(small), m,
-                    s, ph, stage, zero_rr);
-            } else {
+            {
                 using MM = InsTf32<P>;
                 const float2 *o = static_cast<const float2 *>(ops);
                 const long nquad = ((long)m.ntri + 3) / 4;
@@ -497,14 +406,15 @@ struct LaunchImpl {
                     o, o + MM::PROJ_LEN / 2, o + (MM::PROJ_LEN + MM::INT_LEN) / 2,
                     *static_cast<const InsMmaSmallF<P> *>(small), m, s, ph, stage, zero_rr, diff);
             }
-            if (m.ncurved > 0) {
-                constexpr int EPC = C::WPC * C::EPW;
-                const int cap = nsm * tn.elem_cap;
-                k_rsdl_elem<R, P, PHYS, true><<<std::min(nblk(m.ncurved, EPC), cap), C::WPC * 32, smem(), st>>>(
-                    reinterpret_cast<const DevTables<R, P> *>(tab), m, s, ph, stage, zero_rr, diff, ElemMat<R>{},
-                    ElemJac<R>{});
-            }
+            curved(tab, m, s, ph, stage, zero_rr, diff, nsm, tn, st);
         }
+    }
+    static void curved(const void *tab, const Mesh &m, const State<R> &s, const Phys &ph, int stage, int zero_rr,
+                       int diff, int nsm, const Tune &tn, cudaStream_t st) {
+        if (m.ncurved == 0) return;
+        constexpr int EPC = C::WPC * C::EPW;
+        k_rsdl_elem<R, P, PHYS, true><<<std::min(nblk(m.ncurved, EPC), nsm * tn.elem_cap), C::WPC * 32, smem(), st>>>(
+            reinterpret_cast<const DevTables<R, P> *>(tab), m, s, ph, stage, zero_rr, diff, ElemMat<R>{}, ElemJac<R>{});
     }
     static constexpr bool HAS_POINT = PHYS == 1 && P == 1;
     static void elem_point(const void *ops, const void *tab, const Mesh &m, const State<R> &s, const Phys &ph,
@@ -514,13 +424,7 @@ struct LaunchImpl {
             const int blocks = (int)std::min<long>(((long)m.ntri + tri_per_cta - 1) / tri_per_cta, (long)nsm * 8);
             k_rsdl_ins_p1<R><<<blocks, 256, 0, st>>>(static_cast<const InsP1Ops<R> *>(ops), m, s, ph, stage, zero_rr,
                                                      diff);
-            if (m.ncurved > 0) {
-                constexpr int EPC = C::WPC * C::EPW;
-                const int cap = nsm * tn.elem_cap;
-                k_rsdl_elem<R, P, PHYS, true><<<std::min(nblk(m.ncurved, EPC), cap), C::WPC * 32, smem(), st>>>(
-                    reinterpret_cast<const DevTables<R, P> *>(tab), m, s, ph, stage, zero_rr, diff, ElemMat<R>{},
-                    ElemJac<R>{});
-            }
+            curved(tab, m, s, ph, stage, zero_rr, diff, nsm, tn, st);
         }
     }
     static void point_build(const hp_basis_tables &b, std::vector<unsigned char> &ops) {
@@ -530,15 +434,7 @@ struct LaunchImpl {
         std::memcpy(ops.data(), &o, sizeof(o));
     }
     static void mma_build(const hp_basis_tables &b, std::vector<unsigned char> &ops, std::vector<unsigned char> &small) {
-        if constexpr (DBL) {
-            InsMmaSmall<P> sm;
-            std::vector<double> o;
-            build_ins_mma<P>(b, o, sm);
-            ops.resize(o.size() * sizeof(double));
-            std::memcpy(ops.data(), o.data(), ops.size());
-            small.resize(sizeof(sm));
-            std::memcpy(small.data(), &sm, sizeof(sm));
-        } else {
+        if constexpr (HAS_MMA) {
             InsMmaSmallF<P> sm;
             std::vector<float> o;
             build_ins_tf32<P>(b, o, sm);
@@ -549,7 +445,7 @@ struct LaunchImpl {
         }
     }
     static void base_pts(const void *tab, const Mesh &m, const State<R> &s, R *bpt, cudaStream_t st) {
-        if constexpr (HAS_MMA && !DBL)
+        if constexpr (HAS_MMA)
             k_base_points<P><<<nblk(2L * m.ntri, 128), 128, 0, st>>>(reinterpret_cast<const DevTables<float, P> *>(tab),
                                                                      m, s.ubv, s.ubs, s.ubi, bpt);
     }
@@ -558,10 +454,7 @@ struct LaunchImpl {
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, smem());
         if (e != cudaSuccess) return e;
         if constexpr (HAS_MMA) {
-            if constexpr (DBL)
-                e = cudaFuncSetAttribute(k_rsdl_ins_mma<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, mma_smem());
-            else
-                e = cudaFuncSetAttribute(k_rsdl_ins_tf32<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, mma_smem());
+            e = cudaFuncSetAttribute(k_rsdl_ins_tf32<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, mma_smem());
             if (e != cudaSuccess) return e;
         }
         return cudaFuncSetAttribute(k_rsdl_elem<R, P, PHYS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem());
@@ -591,10 +484,11 @@ struct LaunchImpl {
         L.emat_apply = &emat_apply;
         L.elem_jac = &elem_jac;
         L.elem_mma = HAS_MMA ? &elem_mma : nullptr;
+        L.curved = &curved;
         L.elem_point = HAS_POINT ? &elem_point : nullptr;
         L.point_build = HAS_POINT ? &point_build : nullptr;
         L.mma_build = HAS_MMA ? &mma_build : nullptr;
-        L.base_pts = (HAS_MMA && !DBL) ? &base_pts : nullptr;
+        L.base_pts = HAS_MMA ? &base_pts : nullptr;
         L.bpt_per_elem = 2 * (P + 1) * (P + 1);
         L.l2err = std::is_same<R, double>::value ? &l2err : nullptr;
         return L;
@@ -684,11 +578,14 @@ struct hp_gpu_ctx {
     int *f2c_tri = nullptr, *c2f_tri = nullptr;
     double *f2c_wt = nullptr, *c2f_wt = nullptr;
     Tune tune[2];  // launch shapes for FP64 [0] and FP32 [1]
-    // FP64 element kernel: HP_ELEM_TENSOR (ins: k_rsdl_ins_mma) or HP_ELEM_SCALAR (k_rsdl_elem)
+    // element kernel: HP_ELEM_TENSOR (ins: FP64 line kernel, FP32 correction form TF32),
+    // HP_ELEM_POINT (ins at p = 1) or HP_ELEM_SCALAR (k_rsdl_elem)
     int elem_kind = 0;
-    void *d_mma = nullptr, *d_mma32 = nullptr;            // dense operators in fragment order (FP64, TF32)
+    void *d_mma32 = nullptr;                              // dense operators in fragment order (TF32)
     void *d_p1 = nullptr, *d_p1_32 = nullptr;             // operators of the p = 1 point kernel (FP64, FP32)
-    std::vector<unsigned char> mma_small, mma_small32;  // derivative tables (kernel parameters)
+    LineLaunch<double> line{};                          // line kernel (ins, p >= 2), its tables
+    std::vector<unsigned char> line_tab;
+    std::vector<unsigned char> mma_small32;             // derivative tables (kernel parameters)
     float *d_bpt32 = nullptr;                           // FP32 base point values (correction form)
     double wtn[HP_MXGP] = {0};                // Gauss-Jacobi weights (l2error)
     double *d_l2part = nullptr;               // l2error per-block partials
@@ -933,6 +830,15 @@ extern "C" int hp_gpu_create(const hp_mesh_desc *m, const hp_basis_tables *b, co
         double *d_g;
         if ((r = upload(c, &d_g, g.data(), g.size()))) return fail(r);
         M.tgeo = d_g;
+        // the same in batches of 32 triangles (Mesh::lgeo)
+        const int nb = (nt + 31) / 32;
+        std::vector<double> lg((size_t)nb * kLineGeo * 32);
+        for (int t = 0; t < nb * 32; ++t)
+            for (int k = 0; k < kLineGeo; ++k)
+                lg[((size_t)(t / 32) * kLineGeo + k) * 32 + t % 32] = g[(size_t)8 * std::min(t, nt - 1) + k];
+        double *d_lg;
+        if ((r = upload(c, &d_lg, lg.data(), lg.size()))) return fail(r);
+        M.lgeo = d_lg;
     }
 
     // curved elements (tri_hp::metric::setinfo, metric.cpp:44-70, for p > 1): the
@@ -987,15 +893,15 @@ extern "C" int hp_gpu_create(const hp_mesh_desc *m, const hp_basis_tables *b, co
     c->L.fill(*b, htab.data());
     if ((r = upload(c, (unsigned char **)&c->d_tab, htab.data(), htab.size()))) return fail(r);
     for (int j = 0; j < b->gpn && j < HP_MXGP; ++j) c->wtn[j] = b->wtn[j];
-    if (c->L.mma_build && c->L32.mma_build) {
-        std::vector<unsigned char> ops, ops32;
-        c->L.mma_build(*b, ops, c->mma_small);
+    if (physics == HP_PHYS_INS) {
+        std::vector<unsigned char> ops32;
         c->L32.mma_build(*b, ops32, c->mma_small32);
-        if ((r = upload(c, (unsigned char **)&c->d_mma, ops.data(), ops.size()))) return fail(r);
         if ((r = upload(c, (unsigned char **)&c->d_mma32, ops32.data(), ops32.size()))) return fail(r);
-        // at p = 1 and 2 the scalar kernel's lane groups (4 and 2 triangles per warp) are
-        // faster than two triangles per tensor-core warp (measured: 0.080 vs 0.153 ms and
-        // 0.205 vs 0.205 ms for 131k triangles); at p = 1 the point kernel is faster still
+        c->line = line_launch<double>(c->p);
+        if (c->line.launch) {
+            c->line.build(*b, c->line_tab);
+            if (c->line.set_smem() != cudaSuccess) { set_err("line kernel: smem attribute rejected"); return fail(HP_ECUDA); }
+        }
         c->elem_kind = c->p >= 3 ? HP_ELEM_TENSOR : HP_ELEM_SCALAR;
     }
     if (c->L.point_build && c->L32.point_build) {
@@ -1149,16 +1055,20 @@ static void launch_elem(hp_gpu_ctx *c, const Launchers<R> &L, const void *tab, c
                         int stage, int zero_rr, int diff) {
     if (c->emat_on && c->emat_built && ph.physics == HP_PHYS_CD && !diff)
         L.emat_apply(emat_of(c, R()), c->mesh, st, ph, stage, zero_rr, c->nsm, tune_of(c, R()), c->stream);
-    // FP64: the DMMA kernel; FP32: the TF32 kernel in correction form only (the operand
-    // rounding to TF32 is ~5e-4 of the fluxes, which a plain-form residual near convergence,
-    // much smaller than its fluxes, would not resolve; the correction form has no such
-    // cancellation)
-    else if (c->elem_kind == HP_ELEM_TENSOR && L.elem_mma &&
-             (std::is_same<R, double>::value ? !diff : (diff && st.bpt != nullptr)))
-        L.elem_mma(std::is_same<R, double>::value ? c->d_mma : c->d_mma32,
-                   std::is_same<R, double>::value ? c->mma_small.data() : c->mma_small32.data(), tab, c->mesh, st, ph,
-                   stage, zero_rr, diff, c->nsm, tune_of(c, R()), c->stream);
-    else if (c->elem_kind == HP_ELEM_POINT && L.elem_point)
+    else if (std::is_same<R, double>::value && c->elem_kind == HP_ELEM_TENSOR && c->line.launch) {
+        if constexpr (std::is_same<R, double>::value)
+            c->line.launch(c->line_tab.data(), c->mesh, st, ph, stage, zero_rr, diff, c->nsm, c->stream);
+        L.curved(tab, c->mesh, st, ph, stage, zero_rr, diff, c->nsm, tune_of(c, R()), c->stream);
+    }
+    // FP32: the TF32 kernel in correction form only (the operand rounding to TF32 is ~5e-4 of the
+    // fluxes, which a plain-form residual near convergence, much smaller than its fluxes, would
+    // not resolve; the correction form has no such cancellation)
+    else if (!std::is_same<R, double>::value && c->elem_kind == HP_ELEM_TENSOR && L.elem_mma && diff &&
+             st.bpt != nullptr)
+        L.elem_mma(c->d_mma32, c->mma_small32.data(), tab, c->mesh, st, ph, stage, zero_rr, diff, c->nsm,
+                   tune_of(c, R()), c->stream);
+    // (p = 1 has no line kernel: HP_ELEM_TENSOR takes the point kernel there)
+    else if ((c->elem_kind == HP_ELEM_POINT || (c->elem_kind == HP_ELEM_TENSOR && !diff)) && L.elem_point)
         L.elem_point(std::is_same<R, double>::value ? c->d_p1 : c->d_p1_32, tab, c->mesh, st, ph, stage, zero_rr, diff,
                      c->nsm, tune_of(c, R()), c->stream);
     else
@@ -1345,7 +1255,7 @@ extern "C" int hp_gpu_l2error(hp_gpu_ctx *c, const hp_field *fld, double *l2, do
 
 extern "C" int hp_gpu_set_element_kernel(hp_gpu_ctx *c, int kind) {
     if (!c || (kind != HP_ELEM_SCALAR && kind != HP_ELEM_TENSOR && kind != HP_ELEM_POINT)) return HP_EINVAL;
-    if (kind == HP_ELEM_TENSOR && !c->d_mma) {
+    if (kind == HP_ELEM_TENSOR && !c->d_mma32) {
         set_err("the tensor-core element kernel is built for ins only");
         return HP_ENOTSUP;
     }

@@ -72,6 +72,9 @@ struct Mesh {
     // per-triangle constants of the straight-element branch [ntri][8]: ldcrd d00, d01, d10,
     // d11, 1 / |J|, the tau length scale h (inscribed radius / (0.25 (p+1)^2)), 1 / h, unused
     const double *tgeo;
+    // the same constants in batches of 32 triangles, [ceil(ntri / 32)][7][32] (the last batch
+    // repeats the last triangle): coalesced for kernels with one lane per triangle
+    const double *lgeo;
 };
 
 // Slot of an element's vertex / side residual in the assembly buffers (State::elim,
@@ -1590,7 +1593,7 @@ __global__ void k_norm_partial(const R *a, size_t n, double *out) {
 
 // History slot bookkeeping for hp_gpu_iterate: maxres of iteration *it goes to
 // hist[*it], then *it advances (all on the device, so one captured graph replays).
-__global__ void k_hist_advance(unsigned long long *slot, double *hist, int *it, int NV, int cap) {
+static __global__ void k_hist_advance(unsigned long long *slot, double *hist, int *it, int NV, int cap) {
     if (threadIdx.x == 0 && blockIdx.x == 0) {
         double mx = 0.0;
         for (int n = 0; n < NV; ++n) {
@@ -1755,7 +1758,7 @@ __global__ void __launch_bounds__(128) k_l2error(const DevTables<double, P> *__r
 
 namespace hpb {
 // Element features of the learned preconditioner (see include/hp_mlp.h).
-__global__ void k_elem_features(Mesh mesh, State<double> st, Phys ph, int NV, int sm, int im, int p, float *feat) {
+static __global__ void k_elem_features(Mesh mesh, State<double> st, Phys ph, int NV, int sm, int im, int p, float *feat) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= mesh.ntri) return;
     float *f = feat + (size_t)t * 17;
@@ -1802,7 +1805,7 @@ __global__ void k_elem_features(Mesh mesh, State<double> st, Phys ph, int NV, in
 }
 
 // Sum of squares of an element's own residual coefficients (vertex, side, interior).
-__global__ void k_elem_resnorm(Mesh mesh, State<double> st, int NV, int sm, int im, double *out) {
+static __global__ void k_elem_resnorm(Mesh mesh, State<double> st, int NV, int sm, int im, double *out) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= mesh.ntri) return;
     double s2 = 0.0;
