@@ -24,8 +24,13 @@
 // that a fragment needs (98k flops per triangle at p = 6 with the padding) lose to the
 // sum-factorised form (about 40k). Measured, FP64, 131k triangles, full residual, against two
 // triangles per warp on mma.m8n8k4.f64: p = 3 157 -> 89 us, p = 4 308 -> 171, p = 5 503 -> 246,
-// p = 6 719 -> 421, p = 8 1884 -> 1108; p = 2 against the scalar warp kernel 197 -> 54. Bound by
+// p = 6 719 -> 403, p = 8 1884 -> 1169; p = 2 against the scalar warp kernel 197 -> 52. Bound by
 // issue: the FP64 pipe is busy 33 % (p = 6) to 41 % (p = 3) of the time; 7 to 16 warps an SM fit.
+// FP32: the same form beats TF32 fragments (mma.m16n8k8, operands rounded to 10 bits), and in
+// full FP32: an update of the FP32 smoother, 131k triangles, p = 3 728 -> 522 us, p = 4 1202 ->
+// 854, p = 6 2625 -> 2031, p = 8 7305 -> 4032, p = 2 against the scalar warp kernel 670 -> 269; in
+// plain form against the scalar warp kernel p = 6 4475 -> 1885. Bound by issue, too: half of the
+// instructions are FMAs.
 #pragma once
 #include <utility>
 #include "hp_line.h"
@@ -41,12 +46,16 @@ struct LineCfg {
     static constexpr int OUT = 3 * T * 33;    // results [3 T][33]
     static constexpr int EX = 2 * 3 * T * 33; // s fluxes [3][G][G][32], then A, B [3][2][X][G][32]
     static constexpr int LEN = EX + 6 * X * G * 32;
-    static constexpr int IDX = 15 * 32;       // connectivity of a batch: pnt, seg, sgn, vpos, spos [32][3] each
+    static constexpr int IDX = 16 * 32;       // connectivity of a batch: pnt, seg, sgn, vpos, spos [32][3] each, tri_cv [32]
+    static constexpr int LPS = SM * NV, LPI = IM * NV;  // values of a side, of a triangle's interior
     static constexpr int SMEM = LEN * (int)sizeof(R) + 3 * IDX * 4;
     static constexpr int by_smem = 227 * 1024 / (SMEM + 1024);
     // CTAs an SM, as many as leave the point data in registers (measured at 131k triangles, FP64:
     // p = 4 with 1, 2, 3 CTAs 269, 198, 171 us, although 3 spill a little; p = 5 with 1, 2: 347, 246)
-    static constexpr int by_regs = G == 3 ? 5 : G == 4 ? 4 : G == 5 ? 3 : G == 6 ? 2 : 1;
+    // FP32, an update at 131k triangles: p = 2 with 4, 6, 8 CTAs 292, 279, 265 us; p = 8 with 1, 2:
+    // 4932, 4052
+    static constexpr int by_regs = sizeof(R) == 8 ? (G == 3 ? 5 : G == 4 ? 4 : G == 5 ? 3 : G == 6 ? 2 : 1)
+                                                  : (G == 3 ? 8 : G <= 5 ? 5 : G == 6 ? 4 : G == 7 ? 3 : 2);
     static constexpr int MINB = by_smem < by_regs ? (by_smem < 1 ? 1 : by_smem) : by_regs;
 };
 
@@ -71,6 +80,7 @@ struct LineTab {
     // intgrtrs, eta-direction: warp w sums items iptr[w] .. iptr[w + 1] - 1; an item is the column
     // icol and its modes mode[ifst[item] .. ifst[item + 1] - 1]
     unsigned char iptr[G + 1], icol[G + X], ifst[G + X + 1], mode[T];
+    unsigned char odd[T];  // the side of an odd side mode, 3 for the other modes
 };
 
 template <typename R>
@@ -91,6 +101,12 @@ __device__ __forceinline__ void each_mode(F &&f, std::integer_sequence<int, M...
 __device__ __forceinline__ void opaque(double &x) { asm volatile("" : "+d"(x)); }
 __device__ __forceinline__ void opaque(float &x) { asm volatile("" : "+f"(x)); }
 
+// x with its sign changed where bit (0 or the sign bit) is set
+__device__ __forceinline__ void flip_if(double &x, int bit) {
+    x = __hiloint2double(__double2hiint(x) ^ bit, __double2loint(x));
+}
+__device__ __forceinline__ void flip_if(float &x, int bit) { x = __int_as_float(__float_as_int(x) ^ bit); }
+
 template <int BYTES>
 __device__ __forceinline__ void cp_async(void *dst, const void *src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
@@ -98,13 +114,49 @@ __device__ __forceinline__ void cp_async(void *dst, const void *src) {
 }
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
+// Point values (u, v) of the base state of the correction form, State::bpt, in batches of 32
+// triangles [ceil(ntri / 32)][2][G^2][32] (lanes past the last triangle repeat it): the projection
+// (proj.cpp:121-186 as dense sums) of the gathered base modes, one thread per (triangle, variable).
+template <int P>
+__global__ void k_base_points(const DevTables<float, P> *__restrict__ tb, Mesh mesh, const float *__restrict__ ubv,
+                              const float *__restrict__ ubs, const float *__restrict__ ubi, float *bpt) {
+    constexpr int G = P + 1, GG = G * G, T = (P + 1) * (P + 2) / 2, SM = (P > 1 ? P - 1 : 1),
+                  IM = (P - 1) * (P - 2) / 2, BM = 3 * P, NV = 3;
+    const long item = (long)blockIdx.x * blockDim.x + threadIdx.x;  // (batch, variable, lane)
+    const int b = (int)(item >> 6), n = (int)(item >> 5) & 1, lane = (int)item & 31;
+    if (b >= (mesh.ntri + 31) / 32) return;
+    const int t = min(b * 32 + lane, mesh.ntri - 1);
+    float lin[T];
+#pragma unroll
+    for (int m = 0; m < T; ++m) {
+        float val;
+        if (m < 3) {
+            val = ubv[mesh.tri_pnt[3 * t + m] * NV + n];
+        } else if (m < BM) {
+            const int i = (m - 3) / SM, k = (m - 3) - i * SM;
+            val = ubs[(mesh.tri_seg[3 * t + i] * SM + k) * NV + n];
+            if ((k & 1) && mesh.tri_sgn[3 * t + i] < 0) val = -val;
+        } else {
+            val = ubi[((size_t)t * IM + (m - BM)) * NV + n];
+        }
+        lin[m] = val;
+    }
+    float *out = bpt + ((size_t)b * 2 + n) * GG * 32 + lane;
+    for (int q = 0; q < GG; ++q) {
+        const int i = q / G, j = q - i * G;
+        float acc = 0.f;
+#pragma unroll
+        for (int m = 0; m < T; ++m) acc += lin[m] * tb->gn[j][m] * tb->gx[i][ModeCols<P>::col(m)];
+        out[q * 32] = acc;
+    }
+}
+
 template <typename R, int P, bool DIFF, bool RE>
 __global__ void __launch_bounds__(LineCfg<R, P, DIFF>::NTHR, LineCfg<R, P, DIFF>::MINB)
     k_rsdl_ins_line(const __grid_constant__ LineTab<R, P> tab, Mesh mesh, State<R> st, R beta, R omb, R rho, R mu,
                     double nu2, double adis, int gfloor) {
     using C = LineCfg<R, P, DIFF>;
     constexpr int G = C::G, X = C::X, T = C::T, SM = C::SM, IM = C::IM, BM = C::BM, NV = 3, NTHR = C::NTHR;
-    constexpr int IMD = IM > 0 ? IM : 1;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     R *sm = reinterpret_cast<R *>(smem_raw);
     R *out = sm + C::OUT;
@@ -125,41 +177,55 @@ __global__ void __launch_bounds__(LineCfg<R, P, DIFF>::NTHR, LineCfg<R, P, DIFF>
         const int tid = fresh_tid();
         int *d = ring + s * C::IDX;
         for (int w = tid; w < C::IDX; w += NTHR) {
-            const int a = w / 96, r = w - a * 96, e = r / 3, c = r - e * 3;
+            const int a = w / 96, r = w - a * 96;
+            if (a == 5) {
+                if (mesh.tri_cv) cp_async<4>(d + w, mesh.tri_cv + min(b * 32 + r, last));
+                continue;
+            }
             const int *src = a == 0 ? mesh.tri_pnt : a == 1 ? mesh.tri_seg : a == 2 ? mesh.tri_sgn : a == 3 ? mesh.vpos : mesh.spos;
-            cp_async<4>(d + w, src + 3 * (size_t)min(b * 32 + e, last) + c);
+            cp_async<4>(d + w, src + min(b * 96 + r, 3 * last + r % 3));
         }
     };
     // modes of batch b (ugtouht, gtol.cpp:14-55; the signs of the side modes are applied when
-    // they are read), one mode kind per loop, consecutive threads on consecutive values
+    // they are read): a thread keeps to one value of the 3 T of a triangle, so its place and its
+    // source are worked out once, and goes through the triangles; consecutive threads are on
+    // consecutive values of a vertex, a side, an interior
     auto fetch_u = [&](int b, int s) {
         if (b >= nbatch) return;
-        const int tid = fresh_tid();
+        constexpr int TPP = NTHR / (3 * T);  // triangles a pass
+        const int tid = fresh_tid(), sub = tid / (3 * T), rr = tid - sub * (3 * T);
+        if (sub >= TPP) return;
         const int *d = ring + s * C::IDX;
-#pragma unroll
-        for (int it = 0; it < (32 * 9 + NTHR - 1) / NTHR; ++it) {
-            const int w = tid + it * NTHR;
-            if (w >= 32 * 9) break;
-            const int e = w / 9, r = w - e * 9, m = r / NV, n = r - m * NV;
-            cp_async<sizeof(R)>(sm + (n * T + m) * 33 + e, st.ugv + (size_t)d[3 * e + m] * NV + n);
+        const R *base;
+        int stride, row;
+        bool inner = false;
+        if (rr < 9) {
+            const int m = rr / 3, n = rr - m * 3;
+            base = st.ugv + n;
+            stride = NV;
+            d += m;
+            row = n * T + m;
+        } else if (rr < 3 * BM) {
+            const int i = (rr - 9) / C::LPS, r = rr - 9 - i * C::LPS, k = r / 3, n = r - k * 3;
+            base = st.ugs + r;
+            stride = C::LPS;
+            d += 96 + i;
+            row = n * T + 3 + i * SM + k;
+        } else {
+            const int r = rr - 3 * BM, k = r / 3, n = r - k * 3;
+            base = st.ugi + r;
+            stride = C::LPI;
+            inner = true;
+            row = n * T + BM + k;
         }
-        constexpr int NS = 96 * SM * NV;
+        R *dst = sm + row * 33;
 #pragma unroll
-        for (int it = 0; it < (NS + NTHR - 1) / NTHR; ++it) {
-            const int w = tid + it * NTHR;
-            if (w >= NS) break;
-            const int q = w / (SM * NV), r = w - q * (SM * NV), e = q / 3, i = q - e * 3, k = r / NV, n = r - k * NV;
-            cp_async<sizeof(R)>(sm + (n * T + 3 + i * SM + k) * 33 + e, st.ugs + (size_t)d[96 + q] * (SM * NV) + r);
-        }
-        if constexpr (IM > 0) {
-            constexpr int NI = 32 * IM * NV;
-#pragma unroll
-            for (int it = 0; it < (NI + NTHR - 1) / NTHR; ++it) {
-                const int w = tid + it * NTHR;
-                if (w >= NI) break;
-                const int e = w / (IMD * NV), r = w - e * (IMD * NV), k = r / NV, n = r - k * NV;
-                cp_async<sizeof(R)>(sm + (n * T + BM + k) * 33 + e, st.ugi + (size_t)min(b * 32 + e, last) * (IMD * NV) + r);
-            }
+        for (int it = 0; it < (32 + TPP - 1) / TPP; ++it) {
+            const int e = sub + it * TPP;
+            if (e >= 32) break;
+            int v = d[3 * e];
+            if (inner) v = min(b * 32 + e, last);
+            cp_async<sizeof(R)>(dst + e, base + (size_t)v * stride);
         }
     };
     const int step = gridDim.x;
@@ -188,6 +254,9 @@ __global__ void __launch_bounds__(LineCfg<R, P, DIFF>::NTHR, LineCfg<R, P, DIFF>
         }
         cp_async_wait();
         __syncthreads();
+        // sign bits of the triangle's sides (tri_sgn < 0): odd side modes change sign
+        const int sbit[3] = {idx[192 + 3 * lane] & (int)0x80000000, idx[192 + 3 * lane + 1] & (int)0x80000000,
+                             idx[192 + 3 * lane + 2] & (int)0x80000000};
         R uq[G], vq[G], pq[G], xx[RE ? G : 1], xy[RE ? G : 1], yy[RE ? G : 1];
         // ---- proj (proj.cpp:22-119): column sums of the thread's line, then its points: u, v, p
         //      and the viscous stress -mu (2 u_x, u_y + v_x, 2 v_y)
@@ -197,15 +266,13 @@ __global__ void __launch_bounds__(LineCfg<R, P, DIFF>::NTHR, LineCfg<R, P, DIFF>
             for (int c = 0; c < X; ++c) wu[c] = wv[c] = wp[c] = wu1[c] = wv1[c] = (R)0;
             int jl = j;  // anew in each batch: the line's table entries are not kept across the loop
             asm volatile("" : "+r"(jl));
-            const bool neg[3] = {idx[192 + 3 * lane] < 0, idx[192 + 3 * lane + 1] < 0, idx[192 + 3 * lane + 2] < 0};
             each_mode([&](auto mm) {
                 constexpr int m = decltype(mm)::value, c = ModeCols<P>::col(m);
                 R x = sm[m * 33 + lane], y = sm[(T + m) * 33 + lane], z = sm[(2 * T + m) * 33 + lane];
                 if constexpr (m >= 3 && m < BM && (((m - 3) % (SM > 0 ? SM : 1)) & 1)) {
-                    const bool ng = neg[(m - 3) / SM];
-                    x = ng ? -x : x;
-                    y = ng ? -y : y;
-                    z = ng ? -z : z;
+                    flip_if(x, sbit[(m - 3) / SM]);
+                    flip_if(y, sbit[(m - 3) / SM]);
+                    flip_if(z, sbit[(m - 3) / SM]);
                 }
                 const R2<R> g = tab.g[jl][m];
                 wu[c] += x * g.x;
@@ -414,8 +481,11 @@ __global__ void __launch_bounds__(LineCfg<R, P, DIFF>::NTHR, LineCfg<R, P, DIFF>
                             s1[n] += w.y * bb[n][k];
                         }
                     }
+                    R sc = scale;  // odd side modes in the side's own direction
+                    const int sd = tab.odd[m];
+                    flip_if(sc, sd == 0 ? sbit[0] : sd == 1 ? sbit[1] : sd == 2 ? sbit[2] : 0);
 #pragma unroll
-                    for (int n = 0; n < 3; ++n) out[(m * NV + n) * 33 + lane] = scale * (s0[n] + s1[n]);
+                    for (int n = 0; n < 3; ++n) out[(m * NV + n) * 33 + lane] = sc * (s0[n] + s1[n]);
                 }
             }
         };
@@ -431,52 +501,60 @@ __global__ void __launch_bounds__(LineCfg<R, P, DIFF>::NTHR, LineCfg<R, P, DIFF>
             opaque(uq[i]);
             opaque(vq[i]);
         });
-        // lftog (gtol.cpp:364-402); curved triangles are done by the curved launch. The interior
-        // values of the imaginary part wait in registers for the real part.
-        constexpr int NKEEP = (32 * IM * NV + NTHR - 1) / NTHR;
-        R keep[NKEEP > 0 ? NKEEP : 1];
-        auto act = [&](int e) { return t0 + e <= last && (!mesh.tri_cv || mesh.tri_cv[t0 + e] < 0); };
+        // lftog (gtol.cpp:364-402), threads as in fetch_u; curved triangles are done by the curved
+        // launch. The interior values of the imaginary part wait in registers for the real part.
+        constexpr int TPS = NTHR / (3 * BM), TPI = NTHR / (IM > 0 ? C::LPI : NTHR);
+        constexpr int NKEEP = IM > 0 ? (32 + TPI - 1) / TPI : 1;
+        R keep[NKEEP];
+        auto act = [&](int e) { return t0 + e <= last && (!mesh.tri_cv || idx[480 + e] < 0); };
         auto scatter = [&](int part) {
             const int tid = fresh_tid();
-            R *el = part ? st.elre : st.elim;
+            {
+                const int sub = tid / (3 * BM), rr = tid - sub * (3 * BM);
+                if (sub < TPS) {
+                    R *el = part ? st.elre : st.elim, *base;
+                    const int *d = idx;
+                    int stride = NV;
+                    if (rr < 9) {
+                        const int m = rr / 3, n = rr - m * 3;
+                        base = (el ? el : part ? st.rrv : st.resv) + n;
+                        d += (el ? 288 : 0) + m;
+                    } else {
+                        const int i = (rr - 9) / C::LPS, r = rr - 9 - i * C::LPS;
+                        base = (el ? el + (size_t)3 * mesh.ntri * NV : part ? st.rrs : st.ress) + r;
+                        d += (el ? 384 : 96) + i;
+                        stride = C::LPS;
+                    }
+                    const R *src = out + rr * 33;
 #pragma unroll
-            for (int it = 0; it < (32 * 9 + NTHR - 1) / NTHR; ++it) {
-                const int w = tid + it * NTHR;
-                if (w >= 32 * 9) break;
-                const int e = w / 9, r = w - e * 9, m = r / NV, n = r - m * NV;
-                if (!act(e)) continue;
-                const R val = out[r * 33 + e];
-                if (el) el[(size_t)idx[288 + 3 * e + m] * NV + n] = val;
-                else atomic_add((part ? st.rrv : st.resv) + (size_t)idx[3 * e + m] * NV + n, val);
-            }
-            constexpr int NS = 96 * SM * NV;
-#pragma unroll
-            for (int it = 0; it < (NS + NTHR - 1) / NTHR; ++it) {
-                const int w = tid + it * NTHR;
-                if (w >= NS) break;
-                const int q = w / (SM * NV), r = w - q * (SM * NV), e = q / 3, i = q - e * 3, k = r / NV;
-                if (!act(e)) continue;
-                R val = out[((3 + i * SM) * NV + r) * 33 + e];
-                if ((k & 1) && idx[192 + q] < 0) val = -val;
-                if (el) el[(size_t)3 * mesh.ntri * NV + (size_t)idx[384 + q] * (SM * NV) + r] = val;
-                else atomic_add((part ? st.rrs : st.ress) + (size_t)idx[96 + q] * (SM * NV) + r, val);
+                    for (int it = 0; it < (32 + TPS - 1) / TPS; ++it) {
+                        const int e = sub + it * TPS;
+                        if (e >= 32) break;
+                        if (!act(e)) continue;
+                        R *p = base + (size_t)d[3 * e] * stride;
+                        if (el) *p = src[e];
+                        else atomic_add(p, src[e]);
+                    }
+                }
             }
             if constexpr (IM > 0) {
+                const int sub = tid / C::LPI, r = tid - sub * C::LPI;
+                if (sub < TPI) {
 #pragma unroll
-                for (int it = 0; it < NKEEP; ++it) {
-                    const int w = tid + it * NTHR;
-                    if (w >= 32 * IM * NV) break;
-                    const int e = w / (IMD * NV), r = w - e * (IMD * NV);
-                    if (!act(e)) continue;
-                    const R val = out[(BM * NV + r) * 33 + e];
-                    const size_t gi = (size_t)t0 * (IMD * NV) + w;
-                    const R rr = omb != (R)0 && (part || !RE) ? st.rri[gi] * omb : (R)0;
-                    if (part) {
-                        st.rri[gi] = rr + val;
-                        st.resi[gi] = keep[it] + (rr + val);
-                    } else {
-                        keep[it] = st.dresi ? val + st.dresi[gi] : val;
-                        if constexpr (!RE) st.resi[gi] = keep[it] + rr;  // res_r unchanged when beta = 0
+                    for (int it = 0; it < NKEEP; ++it) {
+                        const int e = sub + it * TPI;
+                        if (e >= 32) break;
+                        if (!act(e)) continue;
+                        const R val = out[(3 * BM + r) * 33 + e];
+                        const size_t gi = (size_t)(t0 + e) * C::LPI + r;
+                        const R rr = omb != (R)0 && (part || !RE) ? st.rri[gi] * omb : (R)0;
+                        if (part) {
+                            st.rri[gi] = rr + val;
+                            st.resi[gi] = keep[it] + (rr + val);
+                        } else {
+                            keep[it] = st.dresi ? val + st.dresi[gi] : val;
+                            if constexpr (!RE) st.resi[gi] = keep[it] + rr;  // res_r unchanged when beta = 0
+                        }
                     }
                 }
             }

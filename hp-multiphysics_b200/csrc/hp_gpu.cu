@@ -18,7 +18,6 @@
 #include "hp_mlp.h"
 #include "hp_kernels.cuh"
 #include "hp_elem_p1.cuh"
-#include "hp_elem_tf32.cuh"
 #include "hp_line.h"
 
 using namespace hpb;
@@ -116,82 +115,6 @@ void build_ins_p1(const hp_basis_tables &b, InsP1Ops<R> &o) {
     }
 }
 
-// TF32 rounding of an operator entry (round to nearest, ties away from zero, as
-// cvt.rna.tf32.f32 does for the A operands)
-float to_tf32(double v) {
-    float f = (float)v;
-    uint32_t u;
-    std::memcpy(&u, &f, 4);
-    u = (u + 0x1000u) & 0xFFFFE000u;
-    std::memcpy(&f, &u, 4);
-    return f;
-}
-
-// Dense per-point forms of tri_basis::proj (value, d/dr, d/ds; proj.cpp:22-119) and intgrtrs
-// (intgrt.cpp:81-158) for the TF32 kernel (mma.m16n8k8 .row.col:
-// lane l holds B[k = l & 3][n = l >> 2] and B[k = (l & 3) + 4][n = l >> 2], stored as one
-// float2 per lane per MMA), rounded to TF32.
-template <int P>
-void build_ins_tf32(const hp_basis_tables &b, std::vector<float> &ops, InsMmaSmallF<P> &sm) {
-    using M = InsTf32<P>;
-    constexpr int G = M::G, GG = M::GG, T = M::T;
-    ops.assign(M::PROJ_LEN + M::INT_LEN + M::DER_LEN, 0.f);
-    auto proj = [&](int op, int q, int m) -> double {
-        if (q >= GG || m >= T) return 0.0;
-        const int i = q / G, j = q - i * G, c = ModeCols<P>::col(m);
-        const double dr = b.n0[j] * b.gn[j][m] * b.dgx[i][c];
-        return op == 0 ? b.gn[j][m] * b.gx[i][c] : (op == 1 ? dr : b.dgn[j][m] * b.gx[i][c] + b.x0[i] * dr);
-    };
-    auto wgt = [&](int k, int m) -> double {
-        if (k >= 2 * GG || m >= T) return 0.0;
-        const int q = k % GG, i = q / G, j = q - i * G, c = ModeCols<P>::col(m);
-        return k < GG ? -b.dgxwtx[c][i] * b.gnwtnn0[m][j]
-                      : -(b.x0[i] * b.dgxwtx[c][i] * b.gnwtnn0[m][j] + b.gxwtx[c][i] * b.dgnwtn[m][j]);
-    };
-    for (int op = 0; op < 3; ++op)
-        for (int nt = 0; nt < M::NT; ++nt)
-            for (int ks = 0; ks < M::KS; ++ks)
-                for (int l = 0; l < 32; ++l) {
-                    const size_t at = (((size_t)(op * M::NT + nt) * M::KS + ks) * 32 + l) * 2;
-                    const int q = nt * 8 + (l >> 2), m = ks * 8 + (l & 3);
-                    ops[at] = to_tf32(proj(op, q, m));
-                    ops[at + 1] = to_tf32(proj(op, q, m + 4));
-                }
-    float *ib = ops.data() + M::PROJ_LEN;
-    for (int nt = 0; nt < M::NT2; ++nt)
-        for (int ks = 0; ks < M::KS2; ++ks)
-            for (int l = 0; l < 32; ++l) {
-                const size_t at = (((size_t)nt * M::KS2 + ks) * 32 + l) * 2;
-                const int k = ks * 8 + (l & 3), m = nt * 8 + (l >> 2);
-                ib[at] = to_tf32(wgt(k, m));
-                ib[at + 1] = to_tf32(wgt(k + 4, m));
-            }
-    // B fragments of the transposed 1D derivative operators (mma.m16n8k8 .col: lane l holds
-    // B[k = t][n = g], B[k = t + 4][n = g] with g = l >> 2 + 8 nt, t = l & 3 + 8 kb and
-    // B[k][n] = A[n][k]): [Ar | As1]^T in 2 KR k-steps, then As2^T in KR k-steps
-    float *db = ops.data() + M::PROJ_LEN + M::INT_LEN;
-    for (int kk = 0; kk < 3 * M::KR; ++kk)
-        for (int nt = 0; nt < M::NTI; ++nt)
-            for (int l = 0; l < 32; ++l) {
-                const bool part2 = kk >= 2 * M::KR;
-                const int ks = part2 ? kk - 2 * M::KR : kk;
-                const int blk = part2 ? 2 : ks / M::KR, kb = part2 ? ks : ks - (ks / M::KR) * M::KR;
-                const int n = nt * 8 + (l >> 2), k = kb * 8 + (l & 3);
-                float *bb = db + (((size_t)kk * M::NTI + nt) * 32 + l) * 2;
-                bb[0] = to_tf32(deriv_op(b, G, blk, n, k));
-                bb[1] = to_tf32(deriv_op(b, G, blk, n, k + 4));
-            }
-    for (int i = 0; i < G; ++i) {
-        sm.dltx[i] = (float)b.dltx[i]; sm.dltn[i] = (float)b.dltn[i];
-        sm.n0[i] = (float)b.n0[i]; sm.x0[i] = (float)b.x0[i];
-        for (int q = 0; q < G; ++q) {
-            sm.dltx1[i][q] = (float)b.dltx1[i][q];
-            sm.dltn1[i][q] = (float)b.dltn1[i][q];
-            sm.dltn2[i][q] = (float)b.dltn2[i][q];
-        }
-    }
-}
-
 template <typename R>
 void fill_minv(const hp_basis_tables &b, DevMinv<R> &m) {
     std::memset(&m, 0, sizeof(m));
@@ -244,17 +167,9 @@ struct Launchers {
                        const Tune &, cudaStream_t);
     void (*elem_jac)(const void *tab, const Mesh &, const State<R> &, const Phys &, R *K, R *rbar, int nsm,
                      cudaStream_t);
-    // FP32 ins: the tensor-core element kernel (TF32 k_rsdl_ins_tf32) with its operators
-    // (mma_build: dense operators in fragment order + the small derivative tables)
-    void (*elem_mma)(const void *ops, const void *small, const void *tab, const Mesh &, const State<R> &,
-                     const Phys &, int stage, int zero_rr, int diff, int nsm, const Tune &, cudaStream_t);
-    void (*mma_build)(const hp_basis_tables &, std::vector<unsigned char> &ops, std::vector<unsigned char> &small);
     // the curved elements alone, by the scalar kernel (nothing when the mesh has none)
     void (*curved)(const void *tab, const Mesh &, const State<R> &, const Phys &, int stage, int zero_rr, int diff,
                    int nsm, const Tune &, cudaStream_t);
-    // FP32 ins: the base state's point values for the correction form (State::bpt)
-    void (*base_pts)(const void *tab, const Mesh &, const State<R> &, R *bpt, cudaStream_t);
-    int bpt_per_elem;  // 2 GG
     // ins at p = 1: the point kernel (k_rsdl_ins_p1, four lanes per triangle) with its
     // operators (point_build: InsP1Ops<R>), curved triangles through the scalar kernel
     void (*elem_point)(const void *ops, const void *tab, const Mesh &, const State<R> &, const Phys &, int stage,
@@ -388,27 +303,6 @@ struct LaunchImpl {
             k_minv_vert<R, NV><<<nblk(m.npnt, th), th, 0, st>>>(m, s, mt, sm, im, (R)cfla, upd, fold, slot);
         }
     }
-    static constexpr bool DBL = std::is_same<R, double>::value;
-    static constexpr bool HAS_MMA = PHYS == 1 && !DBL;
-    static int mma_smem() {
-        return (int)(((sizeof(InsMmaSmallF<P>) + 15) / 16) * 16 + (size_t)4 * InsTf32<P>::S_EL * InsTf32<P>::WPC * 4 +
-                     InsTf32<P>::SMEM_IDX);
-    }
-    static void elem_mma(const void *ops, const void *small, const void *tab, const Mesh &m, const State<R> &s,
-                         const Phys &ph, int stage, int zero_rr, int diff, int nsm, const Tune &tn, cudaStream_t st) {
-        if constexpr (HAS_MMA) {
-            {
-                using MM = InsTf32<P>;
-                const float2 *o = static_cast<const float2 *>(ops);
-                const long nquad = ((long)m.ntri + 3) / 4;
-                const int blocks = (int)std::min<long>((nquad + MM::WPC - 1) / MM::WPC, (long)nsm * MM::MINB * 4);
-                k_rsdl_ins_tf32<P><<<blocks, MM::WPC * 32, mma_smem(), st>>>(
-                    o, o + MM::PROJ_LEN / 2, o + (MM::PROJ_LEN + MM::INT_LEN) / 2,
-                    *static_cast<const InsMmaSmallF<P> *>(small), m, s, ph, stage, zero_rr, diff);
-            }
-            curved(tab, m, s, ph, stage, zero_rr, diff, nsm, tn, st);
-        }
-    }
     static void curved(const void *tab, const Mesh &m, const State<R> &s, const Phys &ph, int stage, int zero_rr,
                        int diff, int nsm, const Tune &tn, cudaStream_t st) {
         if (m.ncurved == 0) return;
@@ -433,30 +327,10 @@ struct LaunchImpl {
         ops.resize(sizeof(o));
         std::memcpy(ops.data(), &o, sizeof(o));
     }
-    static void mma_build(const hp_basis_tables &b, std::vector<unsigned char> &ops, std::vector<unsigned char> &small) {
-        if constexpr (HAS_MMA) {
-            InsMmaSmallF<P> sm;
-            std::vector<float> o;
-            build_ins_tf32<P>(b, o, sm);
-            ops.resize(o.size() * sizeof(float));
-            std::memcpy(ops.data(), o.data(), ops.size());
-            small.resize(sizeof(sm));
-            std::memcpy(small.data(), &sm, sizeof(sm));
-        }
-    }
-    static void base_pts(const void *tab, const Mesh &m, const State<R> &s, R *bpt, cudaStream_t st) {
-        if constexpr (HAS_MMA)
-            k_base_points<P><<<nblk(2L * m.ntri, 128), 128, 0, st>>>(reinterpret_cast<const DevTables<float, P> *>(tab),
-                                                                     m, s.ubv, s.ubs, s.ubi, bpt);
-    }
     static cudaError_t set_smem_attr() {
         cudaError_t e = cudaFuncSetAttribute(k_rsdl_elem<R, P, PHYS, false>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, smem());
         if (e != cudaSuccess) return e;
-        if constexpr (HAS_MMA) {
-            e = cudaFuncSetAttribute(k_rsdl_ins_tf32<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, mma_smem());
-            if (e != cudaSuccess) return e;
-        }
         return cudaFuncSetAttribute(k_rsdl_elem<R, P, PHYS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem());
     }
     static void l2err(const void *tab, const double *wtn, const Mesh &m, const State<R> &s, int NV,
@@ -483,13 +357,9 @@ struct LaunchImpl {
         L.emat_build = &emat_build;
         L.emat_apply = &emat_apply;
         L.elem_jac = &elem_jac;
-        L.elem_mma = HAS_MMA ? &elem_mma : nullptr;
         L.curved = &curved;
         L.elem_point = HAS_POINT ? &elem_point : nullptr;
         L.point_build = HAS_POINT ? &point_build : nullptr;
-        L.mma_build = HAS_MMA ? &mma_build : nullptr;
-        L.base_pts = HAS_MMA ? &base_pts : nullptr;
-        L.bpt_per_elem = 2 * (P + 1) * (P + 1);
         L.l2err = std::is_same<R, double>::value ? &l2err : nullptr;
         return L;
     }
@@ -578,14 +448,12 @@ struct hp_gpu_ctx {
     int *f2c_tri = nullptr, *c2f_tri = nullptr;
     double *f2c_wt = nullptr, *c2f_wt = nullptr;
     Tune tune[2];  // launch shapes for FP64 [0] and FP32 [1]
-    // element kernel: HP_ELEM_TENSOR (ins: FP64 line kernel, FP32 correction form TF32),
-    // HP_ELEM_POINT (ins at p = 1) or HP_ELEM_SCALAR (k_rsdl_elem)
+    // element kernel: HP_ELEM_TENSOR (ins: line kernel), HP_ELEM_POINT (ins at p = 1) or HP_ELEM_SCALAR (k_rsdl_elem)
     int elem_kind = 0;
-    void *d_mma32 = nullptr;                              // dense operators in fragment order (TF32)
     void *d_p1 = nullptr, *d_p1_32 = nullptr;             // operators of the p = 1 point kernel (FP64, FP32)
-    LineLaunch<double> line{};                          // line kernel (ins, p >= 2), its tables
-    std::vector<unsigned char> line_tab;
-    std::vector<unsigned char> mma_small32;             // derivative tables (kernel parameters)
+    LineLaunch<double> line{};                // line kernel (ins, p >= 2)
+    LineLaunch<float> line32{};
+    std::vector<unsigned char> line_tab, line_tab32;  // its tables (kernel parameters)
     float *d_bpt32 = nullptr;                           // FP32 base point values (correction form)
     double wtn[HP_MXGP] = {0};                // Gauss-Jacobi weights (l2error)
     double *d_l2part = nullptr;               // l2error per-block partials
@@ -894,15 +762,17 @@ extern "C" int hp_gpu_create(const hp_mesh_desc *m, const hp_basis_tables *b, co
     if ((r = upload(c, (unsigned char **)&c->d_tab, htab.data(), htab.size()))) return fail(r);
     for (int j = 0; j < b->gpn && j < HP_MXGP; ++j) c->wtn[j] = b->wtn[j];
     if (physics == HP_PHYS_INS) {
-        std::vector<unsigned char> ops32;
-        c->L32.mma_build(*b, ops32, c->mma_small32);
-        if ((r = upload(c, (unsigned char **)&c->d_mma32, ops32.data(), ops32.size()))) return fail(r);
         c->line = line_launch<double>(c->p);
+        c->line32 = line_launch<float>(c->p);
         if (c->line.launch) {
             c->line.build(*b, c->line_tab);
-            if (c->line.set_smem() != cudaSuccess) { set_err("line kernel: smem attribute rejected"); return fail(HP_ECUDA); }
+            c->line32.build(*b, c->line_tab32);
+            if (c->line.set_smem() != cudaSuccess || c->line32.set_smem() != cudaSuccess) {
+                set_err("line kernel: smem attribute rejected");
+                return fail(HP_ECUDA);
+            }
         }
-        c->elem_kind = c->p >= 3 ? HP_ELEM_TENSOR : HP_ELEM_SCALAR;
+        c->elem_kind = HP_ELEM_TENSOR;
     }
     if (c->L.point_build && c->L32.point_build) {
         std::vector<unsigned char> ops, ops32;
@@ -1048,6 +918,13 @@ static ElemMat<float> emat_of(hp_gpu_ctx *c, float) { return c->em32; }
 static const Tune &tune_of(hp_gpu_ctx *c, double) { return c->tune[0]; }
 static const Tune &tune_of(hp_gpu_ctx *c, float) { return c->tune[1]; }
 
+static void launch_line(hp_gpu_ctx *c, const State<double> &st, const Phys &ph, int stage, int zero_rr, int diff) {
+    c->line.launch(c->line_tab.data(), c->mesh, st, ph, stage, zero_rr, diff, c->nsm, c->stream);
+}
+static void launch_line(hp_gpu_ctx *c, const State<float> &st, const Phys &ph, int stage, int zero_rr, int diff) {
+    c->line32.launch(c->line_tab32.data(), c->mesh, st, ph, stage, zero_rr, diff, c->nsm, c->stream);
+}
+
 // Element part of rsdl(stage): the stored cd element operators once built, else the
 // matrix-free element kernel.
 template <typename R>
@@ -1055,20 +932,12 @@ static void launch_elem(hp_gpu_ctx *c, const Launchers<R> &L, const void *tab, c
                         int stage, int zero_rr, int diff) {
     if (c->emat_on && c->emat_built && ph.physics == HP_PHYS_CD && !diff)
         L.emat_apply(emat_of(c, R()), c->mesh, st, ph, stage, zero_rr, c->nsm, tune_of(c, R()), c->stream);
-    else if (std::is_same<R, double>::value && c->elem_kind == HP_ELEM_TENSOR && c->line.launch) {
-        if constexpr (std::is_same<R, double>::value)
-            c->line.launch(c->line_tab.data(), c->mesh, st, ph, stage, zero_rr, diff, c->nsm, c->stream);
+    else if (c->elem_kind == HP_ELEM_TENSOR && c->line.launch) {
+        launch_line(c, st, ph, stage, zero_rr, diff);
         L.curved(tab, c->mesh, st, ph, stage, zero_rr, diff, c->nsm, tune_of(c, R()), c->stream);
     }
-    // FP32: the TF32 kernel in correction form only (the operand rounding to TF32 is ~5e-4 of the
-    // fluxes, which a plain-form residual near convergence, much smaller than its fluxes, would
-    // not resolve; the correction form has no such cancellation)
-    else if (!std::is_same<R, double>::value && c->elem_kind == HP_ELEM_TENSOR && L.elem_mma && diff &&
-             st.bpt != nullptr)
-        L.elem_mma(c->d_mma32, c->mma_small32.data(), tab, c->mesh, st, ph, stage, zero_rr, diff, c->nsm,
-                   tune_of(c, R()), c->stream);
     // (p = 1 has no line kernel: HP_ELEM_TENSOR takes the point kernel there)
-    else if ((c->elem_kind == HP_ELEM_POINT || (c->elem_kind == HP_ELEM_TENSOR && !diff)) && L.elem_point)
+    else if (c->elem_kind != HP_ELEM_SCALAR && L.elem_point)
         L.elem_point(std::is_same<R, double>::value ? c->d_p1 : c->d_p1_32, tab, c->mesh, st, ph, stage, zero_rr, diff,
                      c->nsm, tune_of(c, R()), c->stream);
     else
@@ -1255,8 +1124,8 @@ extern "C" int hp_gpu_l2error(hp_gpu_ctx *c, const hp_field *fld, double *l2, do
 
 extern "C" int hp_gpu_set_element_kernel(hp_gpu_ctx *c, int kind) {
     if (!c || (kind != HP_ELEM_SCALAR && kind != HP_ELEM_TENSOR && kind != HP_ELEM_POINT)) return HP_EINVAL;
-    if (kind == HP_ELEM_TENSOR && !c->d_mma32) {
-        set_err("the tensor-core element kernel is built for ins only");
+    if (kind == HP_ELEM_TENSOR && c->ph.physics != HP_PHYS_INS) {
+        set_err("the line element kernel is built for ins only");
         return HP_ENOTSUP;
     }
     if (kind == HP_ELEM_POINT && !c->d_p1) {
@@ -1501,10 +1370,10 @@ static int alloc_mixed(hp_gpu_ctx *c) {
     if ((r = dalloc(c, (void **)&f.sprcn, (size_t)c->nseg * c->NV * 4))) return r;
     if ((r = dalloc(c, (void **)&f.tprcn, (size_t)c->ntri * c->NV * 4))) return r;
     if ((r = dalloc(c, (void **)&f.tau, (size_t)c->ntri * c->NV * 4))) return r;
-    // the base state's point values of the TF32 correction-form kernel (refreshed with the
-    // base by base_points); the pointer is fixed here so that captured updates see it
-    if (c->L32.base_pts && c->d_mma32) {
-        if ((r = dalloc(c, (void **)&c->d_bpt32, (size_t)c->ntri * c->L32.bpt_per_elem * 4))) return r;
+    // the base state's point values of the correction form (refreshed with the base by
+    // base_points); the pointer is fixed here so that captured updates see it
+    if (c->line32.base_pts) {
+        if ((r = dalloc(c, (void **)&c->d_bpt32, c->line32.bpt_len(c->ntri) * 4))) return r;
         f.bpt = c->d_bpt32;
     }
     // res_r is scaled by (1 - beta) before it is first written: it must start finite
@@ -1529,7 +1398,7 @@ static void mixed_prcn(hp_gpu_ctx *c) {
 
 // Point values of the FP32 base state (State::bpt) after it changed.
 static void base_points(hp_gpu_ctx *c) {
-    if (c->s32.bpt) c->L32.base_pts(c->d_tab32, c->mesh, c->s32, c->d_bpt32, c->stream);
+    if (c->s32.bpt) c->line32.base_pts(c->d_tab32, c->mesh, c->s32, c->d_bpt32, c->stream);
 }
 
 // Start of one correction cycle: base = fp32(u64), dres = fp32(R64(u64)) (the FP64

@@ -107,8 +107,8 @@ struct State {
     // k_assemble then sums them per vertex and side in a fixed order, so repeated
     // residual evaluations are bitwise identical. NULL: FP64/FP32 atomics.
     R *elim, *elre, *bres;
-    // Correction form on the tensor cores: the base state's point values (u, v)
-    // [ntri][2][GG] (k_base_points), fixed for a correction cycle; NULL: not computed.
+    // Correction form of the line kernel: the base state's point values (u, v) in batches of 32
+    // triangles [ceil(ntri / 32)][2][GG][32] (k_base_points), fixed for a correction cycle.
     const R *bpt;
 };
 

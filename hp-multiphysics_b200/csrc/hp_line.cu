@@ -1,6 +1,7 @@
 // Table builder and launchers of the ins line kernel (hp_elem_line.cuh).
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "hp_line.h"
@@ -33,6 +34,8 @@ void build_tab(const hp_basis_tables &b, LineTab<R, P> &t) {
         }
         t.x0[i] = (R)b.x0[i]; t.n0[i] = (R)b.n0[i];
     }
+    for (int m = 0; m < T; ++m)
+        t.odd[m] = (unsigned char)(m >= 3 && m < 3 * P && ((m - 3) % (P - 1)) % 2 ? (m - 3) / (P - 1) : 3);
     int n = 0, it = 0, col[T];
     for (int c = 0; c < X; ++c)
         for (int m = 0; m < T; ++m)
@@ -54,6 +57,7 @@ void build_tab(const hp_basis_tables &b, LineTab<R, P> &t) {
 
 template <typename R, int P>
 struct Impl {
+    static constexpr bool F32 = std::is_same<R, float>::value;
     static void build(const hp_basis_tables &b, std::vector<unsigned char> &out) {
         out.resize(sizeof(LineTab<R, P>));
         build_tab<R, P>(b, *reinterpret_cast<LineTab<R, P> *>(out.data()));
@@ -68,7 +72,10 @@ struct Impl {
                                     C::SMEM);
     }
     static cudaError_t set_smem() {
-        return smem_attr<false>();
+        const cudaError_t e = smem_attr<false>();
+        if constexpr (F32)
+            if (e == cudaSuccess) return smem_attr<true>();
+        return e;
     }
     template <bool DIFF, bool RE>
     static void go(const void *tab, const Mesh &m, const State<R> &s, const Phys &ph, int stage, int zero_rr, int nsm,
@@ -82,14 +89,34 @@ struct Impl {
     }
     static void launch(const void *tab, const Mesh &m, const State<R> &s, const Phys &ph, int stage, int zero_rr,
                        int diff, int nsm, cudaStream_t st) {
-        if (ph.beta[stage] > 0.0) go<false, true>(tab, m, s, ph, stage, zero_rr, nsm, st);
+        const bool re = ph.beta[stage] > 0.0;
+        if constexpr (F32) {
+            if (diff) {
+                if (re) go<true, true>(tab, m, s, ph, stage, zero_rr, nsm, st);
+                else go<true, false>(tab, m, s, ph, stage, zero_rr, nsm, st);
+                return;
+            }
+        }
+        if (re) go<false, true>(tab, m, s, ph, stage, zero_rr, nsm, st);
         else go<false, false>(tab, m, s, ph, stage, zero_rr, nsm, st);
+    }
+    static void base_pts(const void *tab, const Mesh &m, const State<R> &s, R *bpt, cudaStream_t st) {
+        if constexpr (F32)
+            k_base_points<P><<<(m.ntri + 31) / 32, 64, 0, st>>>(static_cast<const DevTables<float, P> *>(tab), m, s.ubv,
+                                                               s.ubs, s.ubi, bpt);
+    }
+    static size_t bpt_len(int ntri) {
+        return (size_t)((ntri + 31) / 32) * 2 * (P + 1) * (P + 1) * 32;
     }
     static LineLaunch<R> get() {
         LineLaunch<R> l;
         l.build = &build;
         l.set_smem = &set_smem;
         l.launch = &launch;
+        if (F32) {
+            l.base_pts = &base_pts;
+            l.bpt_len = &bpt_len;
+        }
         return l;
     }
 };
@@ -110,5 +137,6 @@ LineLaunch<R> line_launch(int p) {
     return LineLaunch<R>();
 }
 template LineLaunch<double> line_launch<double>(int);
+template LineLaunch<float> line_launch<float>(int);
 
 }  // namespace hpb

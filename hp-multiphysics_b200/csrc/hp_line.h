@@ -38,6 +38,9 @@ struct LineLaunch {
     cudaError_t (*set_smem)() = nullptr;
     void (*launch)(const void *tab, const Mesh &, const State<R> &, const Phys &, int stage, int zero_rr, int diff,
                    int nsm, cudaStream_t) = nullptr;
+    // FP32: the base state's point values of the correction form (State::bpt), their number
+    void (*base_pts)(const void *dev_tables, const Mesh &, const State<R> &, R *bpt, cudaStream_t) = nullptr;
+    size_t (*bpt_len)(int ntri) = nullptr;
 };
 
 // The ins line kernel of p, 2 <= p <= HP_MAXP (launch == nullptr otherwise).

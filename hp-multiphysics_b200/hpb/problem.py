@@ -269,7 +269,7 @@ class GPULevel:
         return K
 
     def element_kernel(self, kind):
-        """Element kernel (hp_gpu_set_element_kernel): "tensor" (ins default at p >= 3),
+        """Element kernel (hp_gpu_set_element_kernel): "tensor" (ins default at p >= 2),
         "point" (ins default at p = 1) or "scalar"."""
         L.check(self.lib.hp_gpu_set_element_kernel(self.h, {"scalar": 0, "tensor": 1, "point": 2}[kind]),
                 "set_element_kernel")

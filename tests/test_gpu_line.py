@@ -49,3 +49,28 @@ def test_line_kernel_matches_oracle_at_batch_edges(kind, n, p):
         o.rsdl(stage)
         assert relerr(g.residual(), o.residual()) < TOL, stage
     g.close()
+
+
+@pytest.mark.parametrize("kind,n,p", [("stair", 1, 2), ("stair", 7, 3)] + [("square", 4, p) for p in range(2, 9)] +
+                         [("square", n, p) for p, n in ((2, 216), (3, 141), (6, 100))])
+def test_fp32_correction_update_matches_fp64_update(kind, n, p):
+    """The FP32 line kernel in correction form (and k_base_points): one update of the FP32 smoother
+    on the correction equation from d = 0 against one FP64 update from the same state.
+
+    Tolerance: the correction is five stages of FP32 residuals, each a sum of at most 290 terms with
+    6e-8 rounding (1.7e-5), cancellation of a factor of 10 between its terms: 1e-3 of the largest
+    correction with the stages together."""
+    pr = _problem(staircase_mesh(n) if kind == "stair" else hpb.square_mesh(n), p)
+    g = pr.gpu()
+    g.element_kernel("tensor")
+    assert g.setup_preconditioner() == 0
+    g.iterate(1)
+    u64 = g.state()
+    g.upload(pr.ugv, pr.ugs, pr.ugi)
+    g.solve(mixed=True, drop=1e-30, max_updates=1, inner=1)
+    u32 = g.state()
+    u0 = (pr.ugv, pr.ugs, pr.ugi)
+    d = np.concatenate([(a - b).ravel() for a, b in zip(u64, u0)])
+    e = np.concatenate([(a - b).ravel() for a, b in zip(u32, u64)])
+    assert np.max(np.abs(e)) < 1e-3 * np.max(np.abs(d))
+    g.close()
