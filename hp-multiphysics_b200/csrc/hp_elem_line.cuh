@@ -1,8 +1,8 @@
-// ins element residual, straight triangles, sum-factorised with one lane per triangle.
+// ins and cd element residual, straight triangles, sum-factorised with one lane per triangle.
 //
 // tri_hp::rsdl's element loop (tri_hp/nstage.cpp:52-73: ugtouht, element_rsdl, lftog) with
-// tri_hp_ins::element_rsdl's straight-element branch (tri_hp/ins/rsdl.cpp:259-433) and the
-// tri_basis operators it calls (proj.cpp:22-119, intgrt.cpp:81-158, derivr / derivs
+// tri_hp_ins::element_rsdl's straight-element branch (tri_hp/ins/rsdl.cpp:259-433) or
+// tri_hp_cd::element_rsdl (tri_hp/cd/rsdl.cpp:14-154, CONST_A) and the tri_basis operators it calls (proj.cpp:22-119, intgrt.cpp:81-158, derivr / derivs
 // proj.cpp:339-402), FP64 or FP32, plain or correction form.
 //
 // A CTA takes batches of 32 triangles, lane = triangle, and has one warp per eta point j: a
@@ -30,32 +30,36 @@
 // full FP32: an update of the FP32 smoother, 131k triangles, p = 3 728 -> 522 us, p = 4 1202 ->
 // 854, p = 6 2625 -> 2031, p = 8 7305 -> 4032, p = 2 against the scalar warp kernel 670 -> 269; in
 // plain form against the scalar warp kernel p = 6 4475 -> 1885. Bound by issue, too: half of the
-// instructions are FMAs.
+// instructions are FMAs. cd against the scalar warp kernel, an FP64 update of 80k triangles: p = 1
+// 126 -> 68 us (with k_vert_p1), p = 2 282 -> 121, p = 4 739 -> 322; p = 6 of 20k 626 -> 330.
 #pragma once
 #include <utility>
 #include "hp_line.h"
 
 namespace hpb {
 
-template <typename R, int P, bool DIFF>
+template <typename R, int P, int PHYS, bool DIFF>
 struct LineCfg {
     static constexpr int G = P + 1, GG = G * G, X = P + 2, T = (P + 1) * (P + 2) / 2, SM = P - 1,
-                         IM = (P - 1) * (P - 2) / 2, BM = 3 * P, NV = 3;
+                         IM = (P - 1) * (P - 2) / 2, BM = 3 * P, NV = PHYS == 1 ? 3 : 1;
     static constexpr int NTHR = 32 * G;
-    static constexpr int U = 0;               // gathered modes [3 T][33]
-    static constexpr int OUT = 3 * T * 33;    // results [3 T][33]
-    static constexpr int EX = 2 * 3 * T * 33; // s fluxes [3][G][G][32], then A, B [3][2][X][G][32]
-    static constexpr int LEN = EX + 6 * X * G * 32;
-    static constexpr int IDX = 16 * 32;       // connectivity of a batch: pnt, seg, sgn, vpos, spos [32][3] each, tri_cv [32]
-    static constexpr int LPS = SM * NV, LPI = IM * NV;  // values of a side, of a triangle's interior
+    static constexpr int U = 0;                // gathered modes [NV T][33]
+    static constexpr int OUT = NV * T * 33;    // results [NV T][33]
+    static constexpr int EX = 2 * NV * T * 33; // s fluxes [NV][G][G][32], then A, B [NV][2][X][G][32]
+    static constexpr int LEN = EX + 2 * NV * X * G * 32;
+    static constexpr int IDX = 16 * 32;        // connectivity of a batch: pnt, seg, sgn, vpos, spos [32][3] each, tri_cv [32]
+    static constexpr int LPS = SM > 0 ? SM * NV : 1, LPI = IM > 0 ? IM * NV : 1;  // values of a side, of an interior
+    static constexpr int XH = NV == 3 ? (X + 1) / 2 : X;  // columns whose x sums share the registers
     static constexpr int SMEM = LEN * (int)sizeof(R) + 3 * IDX * 4;
     static constexpr int by_smem = 227 * 1024 / (SMEM + 1024);
-    // CTAs an SM, as many as leave the point data in registers (measured at 131k triangles, FP64:
-    // p = 4 with 1, 2, 3 CTAs 269, 198, 171 us, although 3 spill a little; p = 5 with 1, 2: 347, 246)
+    // CTAs an SM, as many as leave the point data in registers (ins, 131k triangles, FP64: p = 4 with
+    // 1, 2, 3 CTAs 269, 198, 171 us, although 3 spill a little; p = 5 with 1, 2: 347, 246).
     // FP32, an update at 131k triangles: p = 2 with 4, 6, 8 CTAs 292, 279, 265 us; p = 8 with 1, 2:
     // 4932, 4052
-    static constexpr int by_regs = sizeof(R) == 8 ? (G == 3 ? 5 : G == 4 ? 4 : G == 5 ? 3 : G == 6 ? 2 : 1)
-                                                  : (G == 3 ? 8 : G <= 5 ? 5 : G == 6 ? 4 : G == 7 ? 3 : 2);
+    static constexpr int by_cd = G <= 2 ? 8 : G <= 4 ? 6 : G == 5 ? 5 : G == 6 ? 4 : G == 7 ? 3 : 2;
+    static constexpr int by_regs = PHYS == 0 ? (sizeof(R) == 8 ? by_cd : 2 * by_cd)
+                                 : sizeof(R) == 8 ? (G == 2 ? 8 : G == 3 ? 5 : G == 4 ? 4 : G == 5 ? 3 : G == 6 ? 2 : 1)
+                                                  : (G == 2 ? 12 : G == 3 ? 8 : G <= 5 ? 5 : G == 6 ? 4 : G == 7 ? 3 : 2);
     static constexpr int MINB = by_smem < by_regs ? (by_smem < 1 ? 1 : by_smem) : by_regs;
 };
 
@@ -76,11 +80,18 @@ struct LineTab {
     R gx[G][X], dgx[G][X];             // proj, column sums to point i
     R ar[G][G], as1[G][G], as2[G][G];  // derivr / derivs: 1D derivative operators
     R dgxw[X][G], gxw[X][G];           // intgrtrs, x-direction
-    R x0[G], n0[G];
+    R x0[G], n0[G], src[T];            // src: intgrt of 1 against the modes
     // intgrtrs, eta-direction: warp w sums items iptr[w] .. iptr[w + 1] - 1; an item is the column
     // icol and its modes mode[ifst[item] .. ifst[item + 1] - 1]
     unsigned char iptr[G + 1], icol[G + X], ifst[G + X + 1], mode[T];
     unsigned char odd[T];  // the side of an odd side mode, 3 for the other modes
+};
+
+// What the kernel takes of Phys. ins: rho, mu, nu2 = 2 mu / rho, adis, gfloor (mu + bd0 == 0); cd:
+// rhocv, kcond, the velocity, the source.
+struct LinePar {
+    double beta, omb, rho, mu, nu2, adis, rhocv, kcond, ax, ay, src;
+    int gfloor;
 };
 
 template <typename R>
@@ -151,12 +162,13 @@ __global__ void k_base_points(const DevTables<float, P> *__restrict__ tb, Mesh m
     }
 }
 
-template <typename R, int P, bool DIFF, bool RE>
-__global__ void __launch_bounds__(LineCfg<R, P, DIFF>::NTHR, LineCfg<R, P, DIFF>::MINB)
-    k_rsdl_ins_line(const __grid_constant__ LineTab<R, P> tab, Mesh mesh, State<R> st, R beta, R omb, R rho, R mu,
-                    double nu2, double adis, int gfloor) {
-    using C = LineCfg<R, P, DIFF>;
-    constexpr int G = C::G, X = C::X, T = C::T, SM = C::SM, IM = C::IM, BM = C::BM, NV = 3, NTHR = C::NTHR;
+template <typename R, int P, int PHYS, bool DIFF, bool RE>
+__global__ void __launch_bounds__(LineCfg<R, P, PHYS, DIFF>::NTHR, LineCfg<R, P, PHYS, DIFF>::MINB)
+    k_rsdl_line(const __grid_constant__ LineTab<R, P> tab, Mesh mesh, State<R> st, LinePar par) {
+    using C = LineCfg<R, P, PHYS, DIFF>;
+    constexpr int G = C::G, X = C::X, T = C::T, SM = C::SM, IM = C::IM, BM = C::BM, NV = C::NV, NTHR = C::NTHR;
+    constexpr bool INS = PHYS == 1;
+    const R beta = (R)par.beta, omb = (R)par.omb, rho = (R)par.rho;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     R *sm = reinterpret_cast<R *>(smem_raw);
     R *out = sm + C::OUT;
@@ -192,27 +204,27 @@ __global__ void __launch_bounds__(LineCfg<R, P, DIFF>::NTHR, LineCfg<R, P, DIFF>
     // consecutive values of a vertex, a side, an interior
     auto fetch_u = [&](int b, int s) {
         if (b >= nbatch) return;
-        constexpr int TPP = NTHR / (3 * T);  // triangles a pass
-        const int tid = fresh_tid(), sub = tid / (3 * T), rr = tid - sub * (3 * T);
+        constexpr int TPP = NTHR / (NV * T);  // triangles a pass
+        const int tid = fresh_tid(), sub = tid / (NV * T), rr = tid - sub * (NV * T);
         if (sub >= TPP) return;
         const int *d = ring + s * C::IDX;
         const R *base;
         int stride, row;
         bool inner = false;
-        if (rr < 9) {
-            const int m = rr / 3, n = rr - m * 3;
+        if (rr < 3 * NV) {
+            const int m = rr / NV, n = rr - m * NV;
             base = st.ugv + n;
             stride = NV;
             d += m;
             row = n * T + m;
-        } else if (rr < 3 * BM) {
-            const int i = (rr - 9) / C::LPS, r = rr - 9 - i * C::LPS, k = r / 3, n = r - k * 3;
+        } else if (rr < NV * BM) {
+            const int i = (rr - 3 * NV) / C::LPS, r = rr - 3 * NV - i * C::LPS, k = r / NV, n = r - k * NV;
             base = st.ugs + r;
             stride = C::LPS;
             d += 96 + i;
             row = n * T + 3 + i * SM + k;
         } else {
-            const int r = rr - 3 * BM, k = r / 3, n = r - k * 3;
+            const int r = rr - NV * BM, k = r / NV, n = r - k * NV;
             base = st.ugi + r;
             stride = C::LPI;
             inner = true;
@@ -241,8 +253,20 @@ __global__ void __launch_bounds__(LineCfg<R, P, DIFF>::NTHR, LineCfg<R, P, DIFF>
         // per-triangle constants (Mesh::lgeo): ldcrd, 1 / |J|, tau length scale h, 1 / h
         const double *lg = mesh.lgeo + (size_t)b * (kLineGeo * 32) + lane;
         const R d00 = (R)lg[0], d01 = (R)lg[32], d10 = (R)lg[64], d11 = (R)lg[96];
-        const R cm = RE ? (R)(-(double)mu * lg[128]) : (R)0;
-        const R c5 = RE ? (R)(nu2 * lg[192]) : (R)0, c6 = RE ? (R)(adis * lg[160] * lg[128]) : (R)0;
+        // ins: -mu / |J|, 2 nu / h, adis h / |J|
+        const R cm = INS && RE ? (R)(-par.mu * lg[128]) : (R)0;
+        const R c5 = INS && RE ? (R)(par.nu2 * lg[192]) : (R)0, c6 = INS && RE ? (R)(par.adis * lg[160] * lg[128]) : (R)0;
+        // cd: the velocity's r and s components, the diffusion tensor, -|J| src, tau
+        const R sr = INS ? (R)0 : d11 * (R)par.ax - d01 * (R)par.ay, ss = INS ? (R)0 : d00 * (R)par.ay - d10 * (R)par.ax;
+        R k00 = (R)0, k01 = (R)0, k11 = (R)0, msrc = (R)0, taue = (R)0;
+        if constexpr (!INS && RE) {
+            const R kc = (R)(par.kcond * lg[128]);
+            k00 = -kc * (d11 * d11 + d01 * d01);
+            k11 = -kc * (d10 * d10 + d00 * d00);
+            k01 = kc * (d11 * d10 + d01 * d00);
+            msrc = -(d00 * d11 - d10 * d01) * (R)par.src;
+            taue = st.tau[min(t0 + lane, last)];
+        }
         R bu[DIFF ? G : 1], bv[DIFF ? G : 1];
         if constexpr (DIFF) {
             const R *bp = st.bpt + (size_t)b * (2 * G * G * 32) + lane;
@@ -257,30 +281,38 @@ __global__ void __launch_bounds__(LineCfg<R, P, DIFF>::NTHR, LineCfg<R, P, DIFF>
         // sign bits of the triangle's sides (tri_sgn < 0): odd side modes change sign
         const int sbit[3] = {idx[192 + 3 * lane] & (int)0x80000000, idx[192 + 3 * lane + 1] & (int)0x80000000,
                              idx[192 + 3 * lane + 2] & (int)0x80000000};
-        R uq[G], vq[G], pq[G], xx[RE ? G : 1], xy[RE ? G : 1], yy[RE ? G : 1];
-        // ---- proj (proj.cpp:22-119): column sums of the thread's line, then its points: u, v, p
-        //      and the viscous stress -mu (2 u_x, u_y + v_x, 2 v_y)
+        // ---- proj (proj.cpp:22-119): column sums of the thread's line, then its points: u, v, p and
+        //      the viscous stress -mu (2 u_x, u_y + v_x, 2 v_y); cd: u and the diffusive r, s fluxes
+        constexpr int GV = INS ? G : 1;
+        R uq[G], vq[GV], pq[GV], xx[RE ? G : 1], xy[RE ? G : 1], yy[RE && INS ? G : 1];
+        if constexpr (!INS) vq[0] = pq[0] = (R)0;
         {
-            R wu[X], wv[X], wp[X], wu1[X], wv1[X];
+            constexpr int XV = INS ? X : 1;
+            R wu[X], wv[XV], wp[XV], wu1[X], wv1[XV];
 #pragma unroll
-            for (int c = 0; c < X; ++c) wu[c] = wv[c] = wp[c] = wu1[c] = wv1[c] = (R)0;
+            for (int c = 0; c < X; ++c) wu[c] = wu1[c] = (R)0;
+#pragma unroll
+            for (int c = 0; c < XV; ++c) wv[c] = wp[c] = wv1[c] = (R)0;
             int jl = j;  // anew in each batch: the line's table entries are not kept across the loop
             asm volatile("" : "+r"(jl));
             each_mode([&](auto mm) {
                 constexpr int m = decltype(mm)::value, c = ModeCols<P>::col(m);
-                R x = sm[m * 33 + lane], y = sm[(T + m) * 33 + lane], z = sm[(2 * T + m) * 33 + lane];
-                if constexpr (m >= 3 && m < BM && (((m - 3) % (SM > 0 ? SM : 1)) & 1)) {
-                    flip_if(x, sbit[(m - 3) / SM]);
-                    flip_if(y, sbit[(m - 3) / SM]);
-                    flip_if(z, sbit[(m - 3) / SM]);
-                }
+                constexpr bool odd = m >= 3 && m < BM && (((m - 3) % (SM > 0 ? SM : 1)) & 1);
+                const int bit = odd ? sbit[odd ? (m - 3) / (SM > 0 ? SM : 1) : 0] : 0;
                 const R2<R> g = tab.g[jl][m];
+                R x = sm[m * 33 + lane];
+                if constexpr (odd) flip_if(x, bit);
                 wu[c] += x * g.x;
-                wv[c] += y * g.x;
-                wp[c] += z * g.x;
-                if constexpr (RE) {
-                    wu1[c] += x * g.y;
-                    wv1[c] += y * g.y;
+                if constexpr (RE) wu1[c] += x * g.y;
+                if constexpr (INS) {
+                    R y = sm[(T + m) * 33 + lane], z = sm[(2 * T + m) * 33 + lane];
+                    if constexpr (odd) {
+                        flip_if(y, bit);
+                        flip_if(z, bit);
+                    }
+                    wv[c] += y * g.x;
+                    wp[c] += z * g.x;
+                    if constexpr (RE) wv1[c] += y * g.y;
                 }
             }, std::make_integer_sequence<int, T>{});
             const R n0 = tab.n0[j];
@@ -290,35 +322,47 @@ __global__ void __launch_bounds__(LineCfg<R, P, DIFF>::NTHR, LineCfg<R, P, DIFF>
 #pragma unroll
                 for (int c = 0; c < X; ++c) {
                     u += wu[c] * tab.gx[i][c];
-                    v += wv[c] * tab.gx[i][c];
-                    p += wp[c] * tab.gx[i][c];
+                    if constexpr (INS) {
+                        v += wv[c] * tab.gx[i][c];
+                        p += wp[c] * tab.gx[i][c];
+                    }
                 }
                 uq[i] = u;
-                vq[i] = v;
-                pq[i] = p;
+                if constexpr (INS) {
+                    vq[i] = v;
+                    pq[i] = p;
+                }
                 if constexpr (RE) {
                     R ur = (R)0, vr = (R)0, us = (R)0, vs = (R)0;
 #pragma unroll
                     for (int c = 0; c < X; ++c) {
                         ur += wu[c] * tab.dgx[i][c];
-                        vr += wv[c] * tab.dgx[i][c];
                         us += wu1[c] * tab.gx[i][c];
-                        vs += wv1[c] * tab.gx[i][c];
+                        if constexpr (INS) {
+                            vr += wv[c] * tab.dgx[i][c];
+                            vs += wv1[c] * tab.gx[i][c];
+                        }
                     }
                     ur *= n0;
-                    vr *= n0;
                     us += tab.x0[i] * ur;
-                    vs += tab.x0[i] * vr;
-                    xx[i] = (cm + cm) * (d11 * ur - d10 * us);
-                    xy[i] = cm * ((d00 * us - d01 * ur) + (d11 * vr - d10 * vs));
-                    yy[i] = (cm + cm) * (d00 * vs - d01 * vr);
+                    if constexpr (INS) {
+                        vr *= n0;
+                        vs += tab.x0[i] * vr;
+                        xx[i] = (cm + cm) * (d11 * ur - d10 * us);
+                        xy[i] = cm * ((d00 * us - d01 * ur) + (d11 * vr - d10 * vs));
+                        yy[i] = (cm + cm) * (d00 * vs - d01 * vr);
+                    } else {
+                        xx[i] = k00 * ur + k01 * us;
+                        xy[i] = k01 * ur + k11 * us;
+                    }
                 }
             }
         }
+        const R cr = (R)par.rhocv * sr, cs = (R)par.rhocv * ss;  // cd: convective flux = (cr, cs) u
         // convective flux (r, s components) of u and v at point i without the pressure, and the
         // mass flux; correction form: F(b + d) - F(b) with the products expanded
         auto conv = [&](int i, R &m0, R &m1, R &r0, R &s0, R &r1, R &s1) {
-            const R u = uq[i], v = vq[i];
+            const R u = uq[i], v = vq[INS ? i : 0];
             m0 = rho * (d11 * u - d01 * v);
             m1 = rho * (d00 * v - d10 * u);
             if constexpr (DIFF) {
@@ -335,34 +379,36 @@ __global__ void __launch_bounds__(LineCfg<R, P, DIFF>::NTHR, LineCfg<R, P, DIFF>
                 s1 = v * m1;
             }
         };
-        R pr[RE ? 3 : 1][RE ? G : 1], ps[RE ? 3 : 1][RE ? G : 1];  // real flux pairs of the line: fr + x0 fs, fs
+        R pr[RE ? NV : 1][RE ? G : 1], ps[RE ? NV : 1][RE ? G : 1];  // real flux pairs of the line: fr + x0 fs, fs
         if constexpr (RE) {
             // ---- strong residual (derivr + derivs of the full fluxes, proj.cpp:339-402):
             //      res(i, j) = n0(j) (sum_q Ar(i, q) fr(q, j) + As1(i, q) fs(q, j)) + sum_l As2(j, l) fs(i, l)
-            R res[3][G];
+            R res[NV][G];
             R *ex = sm + C::EX + j * 32 + lane;  // s flux n at point i: ex[(n G + i) G 32]
 #pragma unroll
-            for (int n = 0; n < 3; ++n)
+            for (int n = 0; n < NV; ++n)
 #pragma unroll
                 for (int i = 0; i < G; ++i) res[n][i] = (R)0;
 #pragma unroll
             for (int q = 0; q < G; ++q) {
-                R m0, m1, r0, s0, r1, s1;
-                conv(q, m0, m1, r0, s0, r1, s1);
-                const R px = xx[q] + pq[q], py = yy[q] + pq[q];
-                r0 += d11 * px - d01 * xy[q];
-                s0 += d00 * xy[q] - d10 * px;
-                r1 += d11 * xy[q] - d01 * py;
-                s1 += d00 * py - d10 * xy[q];
-                ex[(q * G) * 32] = s0;
-                ex[((G + q) * G) * 32] = s1;
-                ex[((2 * G + q) * G) * 32] = m1;
-#pragma unroll
-                for (int i = 0; i < G; ++i) {
-                    res[0][i] += tab.ar[i][q] * r0 + tab.as1[i][q] * s0;
-                    res[1][i] += tab.ar[i][q] * r1 + tab.as1[i][q] * s1;
-                    res[2][i] += tab.ar[i][q] * m0 + tab.as1[i][q] * m1;
+                R r[NV], f[NV];
+                if constexpr (INS) {
+                    conv(q, r[2], f[2], r[0], f[0], r[1], f[1]);
+                    const R px = xx[q] + pq[q], py = yy[q] + pq[q];
+                    r[0] += d11 * px - d01 * xy[q];
+                    f[0] += d00 * xy[q] - d10 * px;
+                    r[1] += d11 * xy[q] - d01 * py;
+                    f[1] += d00 * py - d10 * xy[q];
+                } else {
+                    r[0] = cr * uq[q] + xx[q];
+                    f[0] = cs * uq[q] + xy[q];
                 }
+#pragma unroll
+                for (int n = 0; n < NV; ++n) ex[((n * G + q) * G) * 32] = f[n];
+#pragma unroll
+                for (int i = 0; i < G; ++i)
+#pragma unroll
+                    for (int n = 0; n < NV; ++n) res[n][i] += tab.ar[i][q] * r[n] + tab.as1[i][q] * f[n];
             }
             __syncthreads();  // (the gathered modes are dead, too)
             fetch_u(b + step, slot == 2 ? 0 : slot + 1);
@@ -370,20 +416,22 @@ __global__ void __launch_bounds__(LineCfg<R, P, DIFF>::NTHR, LineCfg<R, P, DIFF>
             // eta-direction part, warp = x point: in place on the exchanged rows
             {
                 R *f = sm + C::EX + (j * G) * 32 + lane;
-                R s[3][G];
+                R s[NV][G];
 #pragma unroll
-                for (int n = 0; n < 3; ++n)
+                for (int n = 0; n < NV; ++n)
 #pragma unroll
                     for (int l = 0; l < G; ++l) s[n][l] = f[(n * G * G + l) * 32];
 #pragma unroll
                 for (int k = 0; k < G; ++k) {
-                    R a[3] = {(R)0, (R)0, (R)0};
+                    R a[NV];
+#pragma unroll
+                    for (int n = 0; n < NV; ++n) a[n] = (R)0;
 #pragma unroll
                     for (int l = 0; l < G; ++l)
 #pragma unroll
-                        for (int n = 0; n < 3; ++n) a[n] += tab.as2[k][l] * s[n][l];
+                        for (int n = 0; n < NV; ++n) a[n] += tab.as2[k][l] * s[n][l];
 #pragma unroll
-                    for (int n = 0; n < 3; ++n) f[(n * G * G + k) * 32] = a[n];
+                    for (int n = 0; n < NV; ++n) f[(n * G * G + k) * 32] = a[n];
                 }
             }
             __syncthreads();
@@ -392,6 +440,12 @@ __global__ void __launch_bounds__(LineCfg<R, P, DIFF>::NTHR, LineCfg<R, P, DIFF>
             const R n0 = tab.n0[j];
 #pragma unroll
             for (int i = 0; i < G; ++i) {
+                if constexpr (!INS) {
+                    const R tres = taue * (msrc + n0 * res[0][i] + ex[(i * G) * 32]);
+                    const R fs = xy[i] - ss * tres;
+                    pr[0][i] = xx[i] - sr * tres + tab.x0[i] * fs;
+                    ps[0][i] = fs;
+                } else {
                 R u = uq[i], v = vq[i], qv;
                 if constexpr (DIFF) {
                     qv = bu[i] * bu[i] + bv[i] * bv[i];
@@ -401,7 +455,7 @@ __global__ void __launch_bounds__(LineCfg<R, P, DIFF>::NTHR, LineCfg<R, P, DIFF>
                     qv = u * u + v * v;
                 }
                 R gam = (R)3 * qv + c5 * c5;
-                if (gfloor) gam = gam > (R)0.1 ? gam : (R)0.1;
+                if (par.gfloor) gam = gam > (R)0.1 ? gam : (R)0.1;
                 const R tau0 = line_tau0<R>(c6, gam), tau2 = sqrt(qv) * tau0;
                 const R a0 = tau0 * (n0 * res[0][i] + ex[(i * G) * 32]), a1 = tau0 * (n0 * res[1][i] + ex[((G + i) * G) * 32]),
                         a2 = tau2 * (n0 * res[2][i] + ex[((2 * G + i) * G) * 32]);
@@ -417,36 +471,37 @@ __global__ void __launch_bounds__(LineCfg<R, P, DIFF>::NTHR, LineCfg<R, P, DIFF>
                 ps[2][i] = d10 * a0 - d00 * a1;
 #pragma unroll
                 for (int n = 0; n < 3; ++n) pr[n][i] += tab.x0[i] * ps[n][i];
+                }
             }
             __syncthreads();  // A, B take the place of the exchanged rows
         }
-        // ---- intgrtrs (intgrt.cpp:81-158): x-direction sums of the three flux pairs, given by
-        //      pair(i, fr + x0 fs, fs), half of the columns at a time (their sums share the registers)
+        // ---- intgrtrs (intgrt.cpp:81-158): x-direction sums of the flux pairs, given by
+        //      pair(i, fr + x0 fs, fs), XH columns at a time (their sums share the registers)
         auto xsums = [&](auto &&pair) {
-            constexpr int XH = (X + 1) / 2;
+            constexpr int XH = C::XH;
             R *ab = sm + C::EX + j * 32 + lane;  // A of (n, c): row (2 n X + c) G, B X rows further
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                R a[3][XH], bb[3][XH];
+            for (int h = 0; h < (X + XH - 1) / XH; ++h) {
+                R a[NV][XH], bb[NV][XH];
 #pragma unroll
-                for (int n = 0; n < 3; ++n)
+                for (int n = 0; n < NV; ++n)
 #pragma unroll
                     for (int c = 0; c < XH; ++c) a[n][c] = bb[n][c] = (R)0;
 #pragma unroll
                 for (int i = 0; i < G; ++i) {
-                    R fr[3], fs[3];
+                    R fr[NV], fs[NV];
                     pair(i, fr, fs);
 #pragma unroll
                     for (int c = 0; c < XH; ++c)
                         if (h * XH + c < X)
 #pragma unroll
-                            for (int n = 0; n < 3; ++n) {
+                            for (int n = 0; n < NV; ++n) {
                                 a[n][c] += tab.dgxw[h * XH + c][i] * fr[n];
                                 bb[n][c] += tab.gxw[h * XH + c][i] * fs[n];
                             }
                 }
 #pragma unroll
-                for (int n = 0; n < 3; ++n)
+                for (int n = 0; n < NV; ++n)
 #pragma unroll
                     for (int c = 0; c < XH; ++c)
                         if (h * XH + c < X) {
@@ -455,14 +510,14 @@ __global__ void __launch_bounds__(LineCfg<R, P, DIFF>::NTHR, LineCfg<R, P, DIFF>
                         }
             }
         };
-        // eta-direction sums of the warp's modes into the staging rows
-        auto esums = [&](R scale) {
+        // eta-direction sums of the warp's modes into the staging rows; src0: integral of a constant
+        auto esums = [&](R scale, R src0) {
 #pragma unroll 1
             for (int it = tab.iptr[j]; it < tab.iptr[j + 1]; ++it) {
                 const R *pa = sm + C::EX + (tab.icol[it] * G) * 32 + lane;
-                R a[3][G], bb[3][G];
+                R a[NV][G], bb[NV][G];
 #pragma unroll
-                for (int n = 0; n < 3; ++n)
+                for (int n = 0; n < NV; ++n)
 #pragma unroll
                     for (int k = 0; k < G; ++k) {
                         a[n][k] = pa[(n * 2 * X * G + k) * 32];
@@ -471,12 +526,15 @@ __global__ void __launch_bounds__(LineCfg<R, P, DIFF>::NTHR, LineCfg<R, P, DIFF>
 #pragma unroll 1
                 for (int q = tab.ifst[it]; q < tab.ifst[it + 1]; ++q) {
                     const int m = tab.mode[q];
-                    R s0[3] = {(R)0, (R)0, (R)0}, s1[3] = {(R)0, (R)0, (R)0};
+                    R s0[NV], s1[NV];
+#pragma unroll
+                    for (int n = 0; n < NV; ++n) s0[n] = s1[n] = (R)0;
+                    if constexpr (!INS) s0[0] = src0 * tab.src[m];
 #pragma unroll
                     for (int k = 0; k < G; ++k) {
                         const R2<R> w = tab.w[m][k];
 #pragma unroll
-                        for (int n = 0; n < 3; ++n) {
+                        for (int n = 0; n < NV; ++n) {
                             s0[n] += w.x * a[n][k];
                             s1[n] += w.y * bb[n][k];
                         }
@@ -485,42 +543,47 @@ __global__ void __launch_bounds__(LineCfg<R, P, DIFF>::NTHR, LineCfg<R, P, DIFF>
                     const int sd = tab.odd[m];
                     flip_if(sc, sd == 0 ? sbit[0] : sd == 1 ? sbit[1] : sd == 2 ? sbit[2] : 0);
 #pragma unroll
-                    for (int n = 0; n < 3; ++n) out[(m * NV + n) * 33 + lane] = sc * (s0[n] + s1[n]);
+                    for (int n = 0; n < NV; ++n) out[(m * NV + n) * 33 + lane] = sc * (s0[n] + s1[n]);
                 }
             }
         };
-        xsums([&](int i, R (&fr)[3], R (&fs)[3]) {
-            conv(i, fr[2], fs[2], fr[0], fs[0], fr[1], fs[1]);
-            fr[0] += d11 * pq[i];
-            fs[0] -= d10 * pq[i];
-            fr[1] -= d01 * pq[i];
-            fs[1] += d00 * pq[i];
+        xsums([&](int i, R (&fr)[NV], R (&fs)[NV]) {
+            if constexpr (INS) {
+                conv(i, fr[2], fs[2], fr[0], fs[0], fr[1], fs[1]);
+                fr[0] += d11 * pq[i];
+                fs[0] -= d10 * pq[i];
+                fr[1] -= d01 * pq[i];
+                fs[1] += d00 * pq[i];
 #pragma unroll
-            for (int n = 0; n < 3; ++n) fr[n] += tab.x0[i] * fs[n];
-            // the second half of the columns forms the fluxes again instead of keeping them
-            opaque(uq[i]);
-            opaque(vq[i]);
+                for (int n = 0; n < NV; ++n) fr[n] += tab.x0[i] * fs[n];
+                // the second half of the columns forms the fluxes again instead of keeping them
+                opaque(uq[i]);
+                opaque(vq[i]);
+            } else {
+                fs[0] = cs * uq[i];
+                fr[0] = cr * uq[i] + tab.x0[i] * fs[0];
+            }
         });
         // lftog (gtol.cpp:364-402), threads as in fetch_u; curved triangles are done by the curved
         // launch. The interior values of the imaginary part wait in registers for the real part.
-        constexpr int TPS = NTHR / (3 * BM), TPI = NTHR / (IM > 0 ? C::LPI : NTHR);
+        constexpr int TPS = NTHR / (NV * BM), TPI = NTHR / (IM > 0 ? C::LPI : NTHR);
         constexpr int NKEEP = IM > 0 ? (32 + TPI - 1) / TPI : 1;
         R keep[NKEEP];
         auto act = [&](int e) { return t0 + e <= last && (!mesh.tri_cv || idx[480 + e] < 0); };
         auto scatter = [&](int part) {
             const int tid = fresh_tid();
             {
-                const int sub = tid / (3 * BM), rr = tid - sub * (3 * BM);
+                const int sub = tid / (NV * BM), rr = tid - sub * (NV * BM);
                 if (sub < TPS) {
                     R *el = part ? st.elre : st.elim, *base;
                     const int *d = idx;
                     int stride = NV;
-                    if (rr < 9) {
-                        const int m = rr / 3, n = rr - m * 3;
+                    if (rr < 3 * NV) {
+                        const int m = rr / NV, n = rr - m * NV;
                         base = (el ? el : part ? st.rrv : st.resv) + n;
                         d += (el ? 288 : 0) + m;
                     } else {
-                        const int i = (rr - 9) / C::LPS, r = rr - 9 - i * C::LPS;
+                        const int i = (rr - 3 * NV) / C::LPS, r = rr - 3 * NV - i * C::LPS;
                         base = (el ? el + (size_t)3 * mesh.ntri * NV : part ? st.rrs : st.ress) + r;
                         d += (el ? 384 : 96) + i;
                         stride = C::LPS;
@@ -545,7 +608,7 @@ __global__ void __launch_bounds__(LineCfg<R, P, DIFF>::NTHR, LineCfg<R, P, DIFF>
                         const int e = sub + it * TPI;
                         if (e >= 32) break;
                         if (!act(e)) continue;
-                        const R val = out[(3 * BM + r) * 33 + e];
+                        const R val = out[(NV * BM + r) * 33 + e];
                         const size_t gi = (size_t)(t0 + e) * C::LPI + r;
                         const R rr = omb != (R)0 && (part || !RE) ? st.rri[gi] * omb : (R)0;
                         if (part) {
@@ -564,19 +627,19 @@ __global__ void __launch_bounds__(LineCfg<R, P, DIFF>::NTHR, LineCfg<R, P, DIFF>
             fetch_u(b + step, slot == 2 ? 0 : slot + 1);
             fetch_idx(b + 2 * step, slot == 0 ? 2 : slot - 1);
         }
-        esums((R)1);
+        esums((R)1, (R)0);
         __syncthreads();
         scatter(0);
         if constexpr (RE) {
-            xsums([&](int i, R (&fr)[3], R (&fs)[3]) {
+            xsums([&](int i, R (&fr)[NV], R (&fs)[NV]) {
 #pragma unroll
-                for (int n = 0; n < 3; ++n) {
+                for (int n = 0; n < NV; ++n) {
                     fr[n] = pr[n][i];
                     fs[n] = ps[n][i];
                 }
             });
             __syncthreads();
-            esums(beta);
+            esums(beta, msrc);
             __syncthreads();
             scatter(1);
         }

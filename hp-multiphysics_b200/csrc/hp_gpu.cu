@@ -17,8 +17,8 @@
 #include "hp_host.h"
 #include "hp_mlp.h"
 #include "hp_kernels.cuh"
-#include "hp_elem_p1.cuh"
 #include "hp_line.h"
+#include "hp_p1.h"
 
 using namespace hpb;
 
@@ -90,31 +90,6 @@ void fill_tables(const hp_basis_tables &b, DevTables<R, P> &t) {
     t.colstart[X] = c;
 }
 
-// The dense operators of the p = 1 point kernel (k_rsdl_ins_p1), indexed by point q = 2 i + j, see
-// InsP1Ops.
-template <typename R>
-void build_ins_p1(const hp_basis_tables &b, InsP1Ops<R> &o) {
-    constexpr int G = 2;
-    for (int q = 0; q < 4; ++q)
-        for (int m = 0; m < 3; ++m) {
-            const int i = q / G, j = q - i * G, c = ModeCols<1>::col(m);
-            const double dr = b.n0[j] * b.gn[j][m] * b.dgx[i][c];
-            o.V[q][m] = (R)(b.gn[j][m] * b.gx[i][c]);
-            o.DR[q][m] = (R)dr;
-            o.DS[q][m] = (R)(b.dgn[j][m] * b.gx[i][c] + b.x0[i] * dr);
-            o.WR[q][m] = (R)(-b.dgxwtx[c][i] * b.gnwtnn0[m][j]);
-            o.WS[q][m] = (R)(-(b.x0[i] * b.dgxwtx[c][i] * b.gnwtnn0[m][j] + b.gxwtx[c][i] * b.dgnwtn[m][j]));
-        }
-    for (int r = 0; r < G; ++r) {
-        for (int k = 0; k < G; ++k) {
-            o.AR[r][k] = (R)deriv_op(b, G, 0, r, k);
-            o.AS1[r][k] = (R)deriv_op(b, G, 1, r, k);
-            o.AS2[r][k] = (R)deriv_op(b, G, 2, r, k);
-        }
-        o.N0[r] = (R)b.n0[r];
-    }
-}
-
 template <typename R>
 void fill_minv(const hp_basis_tables &b, DevMinv<R> &m) {
     std::memset(&m, 0, sizeof(m));
@@ -170,11 +145,6 @@ struct Launchers {
     // the curved elements alone, by the scalar kernel (nothing when the mesh has none)
     void (*curved)(const void *tab, const Mesh &, const State<R> &, const Phys &, int stage, int zero_rr, int diff,
                    int nsm, const Tune &, cudaStream_t);
-    // ins at p = 1: the point kernel (k_rsdl_ins_p1, four lanes per triangle) with its
-    // operators (point_build: InsP1Ops<R>), curved triangles through the scalar kernel
-    void (*elem_point)(const void *ops, const void *tab, const Mesh &, const State<R> &, const Phys &, int stage,
-                       int zero_rr, int diff, int nsm, const Tune &, cudaStream_t);
-    void (*point_build)(const hp_basis_tables &, std::vector<unsigned char> &ops);
     // tri_hp::l2error on the device (FP64): per-block partials into part
     void (*l2err)(const void *tab, const double *wtn, const Mesh &, const State<R> &, int NV, const DevField &,
                   double *part, int blocks, cudaStream_t);
@@ -310,23 +280,6 @@ struct LaunchImpl {
         k_rsdl_elem<R, P, PHYS, true><<<std::min(nblk(m.ncurved, EPC), nsm * tn.elem_cap), C::WPC * 32, smem(), st>>>(
             reinterpret_cast<const DevTables<R, P> *>(tab), m, s, ph, stage, zero_rr, diff, ElemMat<R>{}, ElemJac<R>{});
     }
-    static constexpr bool HAS_POINT = PHYS == 1 && P == 1;
-    static void elem_point(const void *ops, const void *tab, const Mesh &m, const State<R> &s, const Phys &ph,
-                           int stage, int zero_rr, int diff, int nsm, const Tune &tn, cudaStream_t st) {
-        if constexpr (HAS_POINT) {
-            const long tri_per_cta = 256 / 4;
-            const int blocks = (int)std::min<long>(((long)m.ntri + tri_per_cta - 1) / tri_per_cta, (long)nsm * 8);
-            k_rsdl_ins_p1<R><<<blocks, 256, 0, st>>>(static_cast<const InsP1Ops<R> *>(ops), m, s, ph, stage, zero_rr,
-                                                     diff);
-            curved(tab, m, s, ph, stage, zero_rr, diff, nsm, tn, st);
-        }
-    }
-    static void point_build(const hp_basis_tables &b, std::vector<unsigned char> &ops) {
-        InsP1Ops<R> o;
-        build_ins_p1<R>(b, o);
-        ops.resize(sizeof(o));
-        std::memcpy(ops.data(), &o, sizeof(o));
-    }
     static cudaError_t set_smem_attr() {
         cudaError_t e = cudaFuncSetAttribute(k_rsdl_elem<R, P, PHYS, false>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, smem());
@@ -358,8 +311,6 @@ struct LaunchImpl {
         L.emat_apply = &emat_apply;
         L.elem_jac = &elem_jac;
         L.curved = &curved;
-        L.elem_point = HAS_POINT ? &elem_point : nullptr;
-        L.point_build = HAS_POINT ? &point_build : nullptr;
         L.l2err = std::is_same<R, double>::value ? &l2err : nullptr;
         return L;
     }
@@ -448,10 +399,14 @@ struct hp_gpu_ctx {
     int *f2c_tri = nullptr, *c2f_tri = nullptr;
     double *f2c_wt = nullptr, *c2f_wt = nullptr;
     Tune tune[2];  // launch shapes for FP64 [0] and FP32 [1]
-    // element kernel: HP_ELEM_TENSOR (ins: line kernel), HP_ELEM_POINT (ins at p = 1) or HP_ELEM_SCALAR (k_rsdl_elem)
+    // element kernel: HP_ELEM_SCALAR (k_rsdl_elem), else the line kernel
     int elem_kind = 0;
-    void *d_p1 = nullptr, *d_p1_32 = nullptr;             // operators of the p = 1 point kernel (FP64, FP32)
-    LineLaunch<double> line{};                // line kernel (ins, p >= 2)
+    P1Ops<double> *d_p1s = nullptr;           // operators of the fused p = 1 stage and its state buffers
+    P1Ops<float> *d_p1s32 = nullptr;
+    double *d_p1u = nullptr;
+    float *d_p1u32 = nullptr;
+    float *d_elim32 = nullptr, *d_elre32 = nullptr;  // FP32 element slots (p = 1)
+    LineLaunch<double> line{};                // line kernel
     LineLaunch<float> line32{};
     std::vector<unsigned char> line_tab, line_tab32;  // its tables (kernel parameters)
     float *d_bpt32 = nullptr;                           // FP32 base point values (correction form)
@@ -674,7 +629,7 @@ extern "C" int hp_gpu_create(const hp_mesh_desc *m, const hp_basis_tables *b, co
     M.seg_pnt = d_sp; M.seg_tri = d_st; M.seg_loc = d_sl;
     M.vs_ptr = d_vsp; M.vs_idx = d_vsi; M.vt_ptr = d_vtp; M.vt_idx = d_vti;
     M.vess = d_vess; M.sess = d_sess; M.bseg = d_bseg; M.bkind = d_bkind; M.bpibc = d_bpibc;
-    M.tri_cv = nullptr; M.crv_cht = nullptr; M.bcrd = nullptr; M.ncurved = 0; M.crv_tri = nullptr;
+    M.vt_pnt = nullptr; M.tri_cv = nullptr; M.crv_cht = nullptr; M.bcrd = nullptr; M.ncurved = 0; M.crv_tri = nullptr;
     M.seg_bdry = d_sbd; M.vb_idx = d_vbi; M.vpos = d_vpos; M.spos = d_spos;
     {   // per-triangle constants of the straight branch (tri_hp_ins::element_rsdl's ldcrd and
         // the inscribed-radius length scale of tau, tri_mesh/tprims.cpp:224-241)
@@ -761,26 +716,30 @@ extern "C" int hp_gpu_create(const hp_mesh_desc *m, const hp_basis_tables *b, co
     c->L.fill(*b, htab.data());
     if ((r = upload(c, (unsigned char **)&c->d_tab, htab.data(), htab.size()))) return fail(r);
     for (int j = 0; j < b->gpn && j < HP_MXGP; ++j) c->wtn[j] = b->wtn[j];
-    if (physics == HP_PHYS_INS) {
-        c->line = line_launch<double>(c->p);
-        c->line32 = line_launch<float>(c->p);
-        if (c->line.launch) {
-            c->line.build(*b, c->line_tab);
-            c->line32.build(*b, c->line_tab32);
-            if (c->line.set_smem() != cudaSuccess || c->line32.set_smem() != cudaSuccess) {
-                set_err("line kernel: smem attribute rejected");
-                return fail(HP_ECUDA);
-            }
-        }
-        c->elem_kind = HP_ELEM_TENSOR;
+    c->line = line_launch<double>(c->p, physics);
+    c->line32 = line_launch<float>(c->p, physics);
+    c->line.build(*b, c->line_tab);
+    c->line32.build(*b, c->line_tab32);
+    if (c->line.set_smem() != cudaSuccess || c->line32.set_smem() != cudaSuccess) {
+        set_err("line kernel: smem attribute rejected");
+        return fail(HP_ECUDA);
     }
-    if (c->L.point_build && c->L32.point_build) {
-        std::vector<unsigned char> ops, ops32;
-        c->L.point_build(*b, ops);
-        c->L32.point_build(*b, ops32);
-        if ((r = upload(c, (unsigned char **)&c->d_p1, ops.data(), ops.size()))) return fail(r);
-        if ((r = upload(c, (unsigned char **)&c->d_p1_32, ops32.data(), ops32.size()))) return fail(r);
-        c->elem_kind = HP_ELEM_POINT;
+    c->elem_kind = HP_ELEM_TENSOR;
+    if (c->p == 1) {
+        P1Ops<double> o;
+        P1Ops<float> o32;
+        p1_ops<double>(*b, o);
+        p1_ops<float>(*b, o32);
+        std::vector<int> vt_pnt(9 * (size_t)nt);
+        for (size_t j = 0; j < vt_idx.size(); ++j)
+            for (int k = 0; k < 3; ++k) vt_pnt[3 * j + k] = m->tri_pnt[3 * (vt_idx[j] >> 2) + k];
+        int *d_vtp3;
+        if ((r = upload(c, &c->d_p1s, &o, 1)) || (r = upload(c, &c->d_p1s32, &o32, 1)) ||
+            (r = upload(c, &d_vtp3, vt_pnt.data(), vt_pnt.size())) ||
+            (r = dalloc(c, (void **)&c->d_p1u, (size_t)np * c->NV * 8)))
+            return fail(r);
+        CK(cudaStreamSynchronize(c->stream));  // the host arrays end here
+        M.vt_pnt = d_vtp3;
     }
     DevMinv<double> hm;
     fill_minv<double>(*b, hm);
@@ -932,14 +891,10 @@ static void launch_elem(hp_gpu_ctx *c, const Launchers<R> &L, const void *tab, c
                         int stage, int zero_rr, int diff) {
     if (c->emat_on && c->emat_built && ph.physics == HP_PHYS_CD && !diff)
         L.emat_apply(emat_of(c, R()), c->mesh, st, ph, stage, zero_rr, c->nsm, tune_of(c, R()), c->stream);
-    else if (c->elem_kind == HP_ELEM_TENSOR && c->line.launch) {
+    else if (c->elem_kind != HP_ELEM_SCALAR) {
         launch_line(c, st, ph, stage, zero_rr, diff);
         L.curved(tab, c->mesh, st, ph, stage, zero_rr, diff, c->nsm, tune_of(c, R()), c->stream);
     }
-    // (p = 1 has no line kernel: HP_ELEM_TENSOR takes the point kernel there)
-    else if (c->elem_kind != HP_ELEM_SCALAR && L.elem_point)
-        L.elem_point(std::is_same<R, double>::value ? c->d_p1 : c->d_p1_32, tab, c->mesh, st, ph, stage, zero_rr, diff,
-                     c->nsm, tune_of(c, R()), c->stream);
     else
         L.elem(tab, c->mesh, st, ph, stage, zero_rr, diff, c->nsm, tune_of(c, R()), c->stream);
 }
@@ -947,7 +902,7 @@ static void launch_elem(hp_gpu_ctx *c, const Launchers<R> &L, const void *tab, c
 // Stream-ordered body of rsdl(stage) (no sync, capturable), either precision.
 template <typename R>
 static void enqueue_rsdl_t(hp_gpu_ctx *c, const Launchers<R> &L, const void *tab, const State<R> &st, const Phys &ph,
-                           int stage, int diff) {
+                           int stage, int diff, int fold = 0) {
     const int nstage = ph.nstage;
     const int zero_rr = (stage >= nstage) ? 1 : 0;
     const double omb = zero_rr ? 0.0 : 1.0 - ph.beta[stage];
@@ -959,7 +914,7 @@ static void enqueue_rsdl_t(hp_gpu_ctx *c, const Launchers<R> &L, const void *tab
         const long n = (long)c->npnt + (long)c->nseg * c->sm;
         const int with_b = (ph.physics == HP_PHYS_INS && c->nbseg > 0) ? 1 : 0;
         k_assemble<R><<<std::min(nblk(n, 256), c->nsm * 16), 256, 0, c->stream>>>(
-            c->mesh, st, c->NV, c->sm, (R)omb, zero_rr, ph.beta[stage] > 0.0 ? 1 : 0, with_b);
+            c->mesh, st, c->NV, c->sm, (R)omb, zero_rr, ph.beta[stage] > 0.0 ? 1 : 0, with_b, fold);
         return;
     }
     const long n = (long)(c->lv + c->ls);
@@ -967,8 +922,80 @@ static void enqueue_rsdl_t(hp_gpu_ctx *c, const Launchers<R> &L, const void *tab
                                                                            st.rrv, st.rrs, (R)omb, zero_rr);
     launch_elem<R>(c, L, tab, st, ph, stage, zero_rr, diff);
     L.bflux(tab, c->mesh, st, ph, diff, c->stream);
+    if (fold) {
+        const long nf = (long)(c->lv + c->ls);
+        k_rsdl_fold<R><<<nblk(nf, 256), 256, 0, c->stream>>>((int)c->lv, (int)c->ls, st.resv, st.rrv, st.ress, st.rrs,
+                                                             st.dresv, st.dress);
+    }
 }
-static void enqueue_rsdl(hp_gpu_ctx *c, int stage) { enqueue_rsdl_t<double>(c, c->L, c->d_tab, c->st, c->ph, stage, 0); }
+
+// The fused p = 1 stage (hp_stage_p1.cuh), unless the scalar element kernel was asked for.
+static bool p1_fused(const hp_gpu_ctx *c) { return c->p == 1 && c->elem_kind != HP_ELEM_SCALAR; }
+static const P1Ops<double> *p1_ops_of(hp_gpu_ctx *c, double) { return c->d_p1s; }
+static const P1Ops<float> *p1_ops_of(hp_gpu_ctx *c, float) { return c->d_p1s32; }
+static double *p1_buf_of(hp_gpu_ctx *c, double) { return c->d_p1u; }
+static float *p1_buf_of(hp_gpu_ctx *c, float) { return c->d_p1u32; }
+
+static void p1_slots(hp_gpu_ctx *, State<double> &) {}
+static void p1_slots(hp_gpu_ctx *c, State<float> &st) {
+    st.elim = c->d_elim32;
+    st.elre = c->d_elre32;
+}
+
+// One p = 1 stage of the state `in`: with `out`, the update's stage from its start u0; without, the
+// residual with res_r and the source folded in.
+template <typename R>
+static void enqueue_p1_stage(hp_gpu_ctx *c, const Launchers<R> &L, const void *tab, const State<R> &st0, const Phys &ph,
+                             int stage, int diff, R *in, const R *u0, R *out, R *res, unsigned long long *slot) {
+    State<R> st = st0;
+    P1Stage<R> s;
+    s.u_in = in;
+    s.u0 = u0;
+    s.u_out = out;
+    s.res = res;
+    s.rr = st.rrv;
+    s.vprcn = st.vprcn;
+    s.dres = st.dresv;
+    s.ub = st.ubv;
+    s.tau = st.tau;
+    s.beta = (R)ph.beta[stage];
+    s.omb = stage >= ph.nstage ? (R)0 : (R)1 - (R)ph.beta[stage];
+    s.cfla = (R)(ph.alpha[stage] * ph.cfl);
+    s.re = ph.beta[stage] > 0.0 ? 1 : 0;
+    s.slot = slot;
+    if (p1_small<R>(c->mesh, c->nsm)) {
+        p1_stage<R>(p1_ops_of(c, R()), c->mesh, s, ph, diff, c->nsm, c->stream);
+        return;
+    }
+    p1_slots(c, st);
+    st.ugv = in;
+    launch_elem<R>(c, L, tab, st, ph, stage, stage >= ph.nstage, diff);
+    p1_vert<R>(p1_ops_of(c, R()), c->mesh, st.elim, st.elre, s, ph, diff, c->stream);
+}
+
+// rsdl(stage) with res_r and the source folded into res (nstage.cpp:76-82)
+template <typename R>
+static void enqueue_rsdl_folded(hp_gpu_ctx *c, const Launchers<R> &L, const void *tab, const State<R> &st,
+                                const Phys &ph, int stage, int diff) {
+    if (p1_fused(c))
+        enqueue_p1_stage<R>(c, L, tab, st, ph, stage, diff, st.ugv, (const R *)nullptr, (R *)nullptr, st.resv, nullptr);
+    else enqueue_rsdl_t<R>(c, L, tab, st, ph, stage, diff, 1);
+}
+
+// The multistage update of a p = 1 level: the state goes ug -> u0v -> buffer -> u0v ... and back to
+// ug in the last stage; ug itself is the update's ug0 until then (one stage: its copy is).
+template <typename R>
+static void enqueue_p1_update(hp_gpu_ctx *c, const Launchers<R> &L, const void *tab, const State<R> &st, const Phys &ph,
+                              int diff, unsigned long long *slot) {
+    const int ns = ph.nstage;
+    R *a = st.ugv, *b = st.u0v, *d = p1_buf_of(c, R());
+    if (ns == 1) cudaMemcpyAsync(b, a, c->lv * sizeof(R), cudaMemcpyDeviceToDevice, c->stream);
+    for (int k = 0; k < ns; ++k) {
+        const bool last = k == ns - 1;
+        enqueue_p1_stage<R>(c, L, tab, st, ph, k, diff, ns == 1 ? b : k == 0 ? a : (k & 1) ? b : d, ns == 1 ? b : a,
+                            last ? a : (k & 1) ? d : b, last ? st.resv : (R *)nullptr, last ? slot : nullptr);
+    }
+}
 
 // minvrt (+ update of ug with cflalpha when upd) ; maxres into slot when slot != NULL
 template <typename R>
@@ -986,13 +1013,14 @@ static void enqueue_minvrt(hp_gpu_ctx *c, double cfla, int upd, int fold, unsign
 template <typename R>
 static void enqueue_update_t(hp_gpu_ctx *c, const Launchers<R> &L, const void *tab, const State<R> &st,
                              const DevMinv<R> *mt, const Phys &ph, int diff, unsigned long long *slot) {
-    cudaMemcpyAsync(st.u0v, st.ugv, c->lv * sizeof(R), cudaMemcpyDeviceToDevice, c->stream);
-    if (c->ls) cudaMemcpyAsync(st.u0s, st.ugs, c->ls * sizeof(R), cudaMemcpyDeviceToDevice, c->stream);
-    if (c->li) cudaMemcpyAsync(st.u0i, st.ugi, c->li * sizeof(R), cudaMemcpyDeviceToDevice, c->stream);
+    if (p1_fused(c)) {
+        enqueue_p1_update<R>(c, L, tab, st, ph, diff, slot);
+        return;
+    }
     for (int stage = 0; stage < ph.nstage; ++stage) {
         enqueue_rsdl_t<R>(c, L, tab, st, ph, stage, diff);
         const double cfla = ph.alpha[stage] * ph.cfl;
-        enqueue_minvrt_t<R>(c, L, st, mt, cfla, 1, 1, stage == ph.nstage - 1 ? slot : nullptr);
+        enqueue_minvrt_t<R>(c, L, st, mt, cfla, stage == 0 ? 2 : 1, 1, stage == ph.nstage - 1 ? slot : nullptr);
     }
 }
 
@@ -1032,12 +1060,7 @@ extern "C" int hp_gpu_enqueue_rsdl(hp_gpu_ctx *c, int stage) {
     }
     int r = fas_first(c);
     if (r) return r;
-    enqueue_rsdl(c, stage);
-    // the reference's rsdl leaves res = res + res_r (nstage.cpp:76-82); the element kernel
-    // already folded the interiors, fold vertices and sides here for the caller
-    const long n = (long)(c->lv + c->ls);
-    k_rsdl_fold<double><<<nblk(n, 256), 256, 0, c->stream>>>((int)c->lv, (int)c->ls, c->st.resv, c->st.rrv, c->st.ress,
-                                                             c->st.rrs, c->st.dresv, c->st.dress);
+    enqueue_rsdl_folded<double>(c, c->L, c->d_tab, c->st, c->ph, stage, 0);
     return check_launch(c);
 }
 
@@ -1085,10 +1108,7 @@ extern "C" int hp_gpu_rsdl(hp_gpu_ctx *c, int stage, int precision) {
     } else {
         f.dresv = f.dress = f.dresi = nullptr;
     }
-    enqueue_rsdl_t<float>(c, c->L32, c->d_tab32, f, c->ph, stage, 0);
-    const long n = (long)(c->lv + c->ls);
-    k_rsdl_fold<float><<<nblk(n, 256), 256, 0, c->stream>>>((int)c->lv, (int)c->ls, f.resv, f.rrv, f.ress, f.rrs,
-                                                            f.dresv, f.dress);
+    enqueue_rsdl_folded<float>(c, c->L32, c->d_tab32, f, c->ph, stage, 0);
     conv(c, (long)c->lv, (const float *)f.resv, c->st.resv);
     conv(c, (long)c->ls, (const float *)f.ress, c->st.ress);
     conv(c, (long)c->li, (const float *)f.resi, c->st.resi);
@@ -1128,8 +1148,8 @@ extern "C" int hp_gpu_set_element_kernel(hp_gpu_ctx *c, int kind) {
         set_err("the line element kernel is built for ins only");
         return HP_ENOTSUP;
     }
-    if (kind == HP_ELEM_POINT && !c->d_p1) {
-        set_err("the point element kernel is built for ins at p = 1 only");
+    if (kind == HP_ELEM_POINT && (c->ph.physics != HP_PHYS_INS || c->p != 1)) {
+        set_err("HP_ELEM_POINT is for ins at p = 1 only");
         return HP_ENOTSUP;
     }
     if (c->elem_kind != kind) {  // captured updates hold the old kernel
@@ -1375,6 +1395,12 @@ static int alloc_mixed(hp_gpu_ctx *c) {
     if (c->line32.base_pts) {
         if ((r = dalloc(c, (void **)&c->d_bpt32, c->line32.bpt_len(c->ntri) * 4))) return r;
         f.bpt = c->d_bpt32;
+    }
+    if (c->p == 1) {
+        const size_t nsl = (size_t)3 * c->ntri * c->NV;
+        if ((r = dalloc(c, (void **)&c->d_p1u32, c->lv * 4)) || (r = dalloc(c, (void **)&c->d_elim32, nsl * 4)) ||
+            (r = dalloc(c, (void **)&c->d_elre32, nsl * 4)))
+            return r;
     }
     // res_r is scaled by (1 - beta) before it is first written: it must start finite
     CK(cudaMemsetAsync(f.rrv, 0, c->lv * 4, c->stream));
@@ -1687,10 +1713,7 @@ static int mg_source_enqueue(hp_gpu_ctx *c) {
     c->fas_pending = false;
     State<double> plain = c->st;
     plain.dresv = plain.dress = plain.dresi = nullptr;
-    enqueue_rsdl_t<double>(c, c->L, c->d_tab, plain, c->ph, c->ph.nstage, 0);
-    const long n2 = (long)(c->lv + c->ls);
-    k_rsdl_fold<double><<<nblk(n2, 256), 256, 0, c->stream>>>((int)c->lv, (int)c->ls, c->st.resv, c->st.rrv,
-                                                              c->st.ress, c->st.rrs, nullptr, nullptr);
+    enqueue_rsdl_folded<double>(c, c->L, c->d_tab, plain, c->ph, c->ph.nstage, 0);
     const int g2 = c->nsm * 8;
     k_fas_source<double><<<g2, 256, 0, c->stream>>>((long)c->lv, c->fadd, c->res0v, c->st.resv, c->fasv);
     if (c->ls) k_fas_source<double><<<g2, 256, 0, c->stream>>>((long)c->ls, c->fadd, c->res0s, c->st.ress, c->fass);
@@ -1969,10 +1992,7 @@ static void rsdl32_folded(hp_gpu_ctx *c, bool with_src) {
     State<float> st = c->s32;
     if (!with_src) st.dresv = st.dress = st.dresi = nullptr;
     const int diff = (c->ph.physics == HP_PHYS_INS) ? 1 : 0;
-    enqueue_rsdl_t<float>(c, c->L32, c->d_tab32, st, phys32(c), c->ph.nstage, diff);
-    const long n = (long)(c->lv + c->ls);
-    k_rsdl_fold<float><<<nblk(n, 256), 256, 0, c->stream>>>((int)c->lv, (int)c->ls, st.resv, st.rrv, st.ress, st.rrs,
-                                                            st.dresv, st.dress);
+    enqueue_rsdl_folded<float>(c, c->L32, c->d_tab32, st, phys32(c), c->ph.nstage, diff);
 }
 
 static int mg_restrict32(hp_gpu_ctx *c) {

@@ -51,6 +51,7 @@ struct Mesh {
     const int *seg_pnt, *seg_tri, *seg_loc;  // [nseg][2]
     const int *vs_ptr, *vs_idx;  // vertex -> (seg*2+end)
     const int *vt_ptr, *vt_idx;  // vertex -> (tri*4+local)
+    const int *vt_pnt;           // p = 1: the triangles' vertices in incidence order [3 ntri][3]
     const int *vess, *sess;      // essential masks
     const int *bseg, *bkind;
     const double *bpibc;  // [nbseg][G]
@@ -943,9 +944,11 @@ __global__ void k_bdry_flux_ins(const DevTables<R, P> *__restrict__ tb, Mesh mes
 // (+ the boundary fluxes, hp_edge_bdry::rsdl), res_r = (1 - beta) res_r + sum of their
 // real parts (nstage.cpp:21-49; zero_rr: res_r = sum). A vertex sums its triangles in
 // vertex-incidence order, a side its two triangles in seg.tri order, so the result does
-// not depend on the scheduling. One thread per vertex, then one per (side, mode).
+// not depend on the scheduling. One thread per vertex, then one per (side, mode). fold: res +=
+// res_r (+ dres), as the stand-alone rsdl leaves it (nstage.cpp:76-82).
 template <typename R>
-__global__ void k_assemble(Mesh mesh, State<R> st, int NV, int SM, R omb, int zero_rr, int with_re, int with_b) {
+__global__ void k_assemble(Mesh mesh, State<R> st, int NV, int SM, R omb, int zero_rr, int with_re, int with_b,
+                           int fold) {
     const size_t soff = (size_t)3 * mesh.ntri * NV;  // side section of the buffers
     const long nitems = (long)mesh.npnt + (long)mesh.nseg * SM;
     for (long k = (long)blockIdx.x * blockDim.x + threadIdx.x; k < nitems; k += (long)gridDim.x * blockDim.x) {
@@ -963,9 +966,9 @@ __global__ void k_assemble(Mesh mesh, State<R> st, int NV, int SM, R omb, int ze
                         if (b >= 0 && (mesh.bkind[b >> 1] & (0xF << 8)) == (1 << 8))
                             sim += st.bres[((size_t)(b >> 1) * (SM + 2) + (b & 1)) * NV + n];
                     }
-                st.resv[v * NV + n] = sim;
-                const R r0 = zero_rr ? (R)0 : st.rrv[v * NV + n] * omb;
-                st.rrv[v * NV + n] = with_re ? r0 + sre : r0;
+                const R r0 = zero_rr ? (R)0 : st.rrv[v * NV + n] * omb, rr = with_re ? r0 + sre : r0;
+                st.rrv[v * NV + n] = rr;
+                st.resv[v * NV + n] = fold ? sim + (rr + (st.dresv ? st.dresv[v * NV + n] : (R)0)) : sim;
             }
         } else {
             const long q = k - mesh.npnt;
@@ -982,9 +985,9 @@ __global__ void k_assemble(Mesh mesh, State<R> st, int NV, int SM, R omb, int ze
                 }
                 if (bf) sim += st.bres[((size_t)e * (SM + 2) + 2 + kk) * NV + n];
                 const size_t g = ((size_t)sd * SM + kk) * NV + n;
-                st.ress[g] = sim;
-                const R r0 = zero_rr ? (R)0 : st.rrs[g] * omb;
-                st.rrs[g] = with_re ? r0 + sre : r0;
+                const R r0 = zero_rr ? (R)0 : st.rrs[g] * omb, rr = with_re ? r0 + sre : r0;
+                st.rrs[g] = rr;
+                st.ress[g] = fold ? sim + (rr + (st.dress ? st.dress[g] : (R)0)) : sim;
             }
         }
     }
@@ -1026,6 +1029,15 @@ __device__ __forceinline__ unsigned long long ord_key(float v) { return (unsigne
 // minvrt (setup_preconditioner.cpp:102-373) fused with the stage update
 // (nstage.cpp:387-409).
 // ---------------------------------------------------------------------------
+// Stage update of one unknown: ug = ug0 - d. upd 2: the update's first stage, whose ug is the
+// update's ug0 and is kept as such (no copy of the state before the update).
+template <typename R>
+__device__ __forceinline__ void stage_update(R *ug, R *u0, size_t g, R d, int upd) {
+    const R a = upd == 2 ? ug[g] : u0[g];
+    if (upd == 2) u0[g] = a;
+    ug[g] = a - d;
+}
+
 // Vertex phase: assemble res.v + res_r.v, remove side and interior parts, apply
 // the vertex preconditioner and Dirichlet zeroing, update ug.v, maxres.
 template <typename R, int NV>
@@ -1060,7 +1072,7 @@ __global__ void k_minv_vert(Mesh mesh, State<R> st, const DevMinv<R> *__restrict
             r[n] *= st.vprcn[v * NV + n];
             if (ess & (1 << n)) r[n] = (R)0;
             st.resv[v * NV + n] = r[n];
-            if (do_update) st.ugv[v * NV + n] = st.u0v[v * NV + n] - cflalpha * r[n];
+            if (do_update) stage_update(st.ugv, st.u0v, v * NV + n, cflalpha * r[n], do_update);
         }
     }
     if (maxres_slot) {
@@ -1137,7 +1149,7 @@ __global__ void k_minv_vert_coop(Mesh mesh, State<R> st, const DevMinv<R> *__res
             x = (x - acc[n]) * st.vprcn[v * NV + n];
             if (ess & (1 << n)) x = (R)0;
             st.resv[v * NV + n] = x;
-            if (do_update) st.ugv[v * NV + n] = st.u0v[v * NV + n] - cflalpha * x;
+            if (do_update) stage_update(st.ugv, st.u0v, v * NV + n, cflalpha * x, do_update);
             r[n] = x;
         }
     }
@@ -1243,7 +1255,7 @@ __global__ void k_minv_side_vn(Mesh mesh, State<R> st, const DevMinv<R> *__restr
         R v = r[0] * (st.sprcn[s * NV + n] * s_sdiag);
         if (mesh.sess[s] & (1 << n)) v = (R)0;
         r[0] = v;
-        if (do_update) st.ugs[g0 + (size_t)MODE * NV] = st.u0s[g0 + (size_t)MODE * NV] - cflalpha * v;
+        if (do_update) stage_update(st.ugs, st.u0s, g0 + (size_t)MODE * NV, cflalpha * v, do_update);
     }
 #pragma unroll
     for (int q = 0; q < NK; ++q) st.ress[g0 + (size_t)(MODE + q) * NV] = r[q];
@@ -1300,7 +1312,7 @@ __global__ void k_minv_int_flat(Mesh mesh, State<R> st, const DevMinv<R> *__rest
     for (int k = 0; k < IM; ++k) {
         const size_t gi = ((size_t)t * IM + k) * NV + n;
         st.resi[gi] = b[k];
-        if (do_update) st.ugi[gi] = st.u0i[gi] - cflalpha * b[k];
+        if (do_update) stage_update(st.ugi, st.u0i, gi, cflalpha * b[k], do_update);
     }
 }
 
@@ -1434,7 +1446,8 @@ __global__ void k_prcn_elem(const DevTables<R, P> *__restrict__ tb, Mesh mesh, S
     }
 }
 
-// res.{v,s} += res_r.{v,s} (nstage.cpp:76-82) for callers of the stand-alone rsdl
+// res.{v,s} += res_r.{v,s} (nstage.cpp:76-82) for callers of the stand-alone rsdl (assembly by
+// atomics; k_assemble folds by itself)
 template <typename R>
 __global__ void k_rsdl_fold(int n1, int n2, R *resv, const R *rrv, R *ress, const R *rrs, const R *dv, const R *ds) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;

@@ -1,4 +1,5 @@
-// Table builder and launchers of the ins line kernel (hp_elem_line.cuh).
+// Table builder and launchers of the line kernel (hp_elem_line.cuh), compiled once for each
+// precision (LINE_R double or float).
 #include <algorithm>
 #include <cstring>
 #include <type_traits>
@@ -16,7 +17,7 @@ namespace {
 // columns (one read of a column's sums costs about as much as one mode).
 template <typename R, int P>
 void build_tab(const hp_basis_tables &b, LineTab<R, P> &t) {
-    constexpr int G = P + 1, X = P + 2, T = (P + 1) * (P + 2) / 2;
+    constexpr int G = P + 1, X = P + 2, T = (P + 1) * (P + 2) / 2, SD = P > 1 ? P - 1 : 1;
     std::memset(&t, 0, sizeof(t));
     for (int i = 0; i < G; ++i) {
         for (int m = 0; m < T; ++m) {
@@ -34,8 +35,14 @@ void build_tab(const hp_basis_tables &b, LineTab<R, P> &t) {
         }
         t.x0[i] = (R)b.x0[i]; t.n0[i] = (R)b.n0[i];
     }
+    for (int m = 0; m < T; ++m) {
+        double s = 0.0;
+        for (int j = 0; j < G; ++j)
+            for (int i = 0; i < G; ++i) s += b.gnwtn[m][j] * b.gxwtx[ModeCols<P>::col(m)][i];
+        t.src[m] = (R)s;
+    }
     for (int m = 0; m < T; ++m)
-        t.odd[m] = (unsigned char)(m >= 3 && m < 3 * P && ((m - 3) % (P - 1)) % 2 ? (m - 3) / (P - 1) : 3);
+        t.odd[m] = (unsigned char)(m >= 3 && m < 3 * P && ((m - 3) % SD) % 2 ? (m - 3) / SD : 3);
     int n = 0, it = 0, col[T];
     for (int c = 0; c < X; ++c)
         for (int m = 0; m < T; ++m)
@@ -55,53 +62,56 @@ void build_tab(const hp_basis_tables &b, LineTab<R, P> &t) {
     t.ifst[it] = (unsigned char)T;
 }
 
-template <typename R, int P>
+template <typename R, int P, int PHYS>
 struct Impl {
-    static constexpr bool F32 = std::is_same<R, float>::value;
+    static constexpr bool F32 = std::is_same<R, float>::value, HAS_DIFF = F32 && PHYS == 1;
     static void build(const hp_basis_tables &b, std::vector<unsigned char> &out) {
         out.resize(sizeof(LineTab<R, P>));
         build_tab<R, P>(b, *reinterpret_cast<LineTab<R, P> *>(out.data()));
     }
     template <bool DIFF>
     static cudaError_t smem_attr() {
-        using C = LineCfg<R, P, DIFF>;
-        cudaError_t e = cudaFuncSetAttribute(k_rsdl_ins_line<R, P, DIFF, true>,
+        using C = LineCfg<R, P, PHYS, DIFF>;
+        cudaError_t e = cudaFuncSetAttribute(k_rsdl_line<R, P, PHYS, DIFF, true>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
         if (e != cudaSuccess) return e;
-        return cudaFuncSetAttribute(k_rsdl_ins_line<R, P, DIFF, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        return cudaFuncSetAttribute(k_rsdl_line<R, P, PHYS, DIFF, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     C::SMEM);
     }
     static cudaError_t set_smem() {
         const cudaError_t e = smem_attr<false>();
-        if constexpr (F32)
+        if constexpr (HAS_DIFF)
             if (e == cudaSuccess) return smem_attr<true>();
         return e;
     }
     template <bool DIFF, bool RE>
-    static void go(const void *tab, const Mesh &m, const State<R> &s, const Phys &ph, int stage, int zero_rr, int nsm,
-                   cudaStream_t st) {
-        using C = LineCfg<R, P, DIFF>;
+    static void go(const void *tab, const Mesh &m, const State<R> &s, const LinePar &par, int nsm, cudaStream_t st) {
+        using C = LineCfg<R, P, PHYS, DIFF>;
         const int nb = (m.ntri + 31) / 32;
-        k_rsdl_ins_line<R, P, DIFF, RE><<<std::min(nb, nsm * C::MINB), C::NTHR, C::SMEM, st>>>(
-            *static_cast<const LineTab<R, P> *>(tab), m, s, (R)ph.beta[stage],
-            zero_rr ? (R)0 : (R)1 - (R)ph.beta[stage], (R)ph.rho, (R)ph.mu, 2. * (ph.mu / ph.rho), ph.adis,
-            ph.mu + ph.bd0 == 0.0 ? 1 : 0);
+        k_rsdl_line<R, P, PHYS, DIFF, RE><<<std::min(nb, nsm * C::MINB), C::NTHR, C::SMEM, st>>>(
+            *static_cast<const LineTab<R, P> *>(tab), m, s, par);
     }
     static void launch(const void *tab, const Mesh &m, const State<R> &s, const Phys &ph, int stage, int zero_rr,
                        int diff, int nsm, cudaStream_t st) {
+        LinePar par;
+        par.beta = ph.beta[stage];
+        par.omb = zero_rr ? 0.0 : (double)((R)1 - (R)ph.beta[stage]);
+        par.rho = ph.rho; par.mu = ph.mu; par.nu2 = 2. * (ph.mu / ph.rho); par.adis = ph.adis;
+        par.rhocv = ph.rhocv; par.kcond = ph.kcond; par.ax = ph.ax; par.ay = ph.ay; par.src = ph.src;
+        par.gfloor = ph.mu + ph.bd0 == 0.0 ? 1 : 0;
         const bool re = ph.beta[stage] > 0.0;
-        if constexpr (F32) {
+        if constexpr (HAS_DIFF) {
             if (diff) {
-                if (re) go<true, true>(tab, m, s, ph, stage, zero_rr, nsm, st);
-                else go<true, false>(tab, m, s, ph, stage, zero_rr, nsm, st);
+                if (re) go<true, true>(tab, m, s, par, nsm, st);
+                else go<true, false>(tab, m, s, par, nsm, st);
                 return;
             }
         }
-        if (re) go<false, true>(tab, m, s, ph, stage, zero_rr, nsm, st);
-        else go<false, false>(tab, m, s, ph, stage, zero_rr, nsm, st);
+        if (re) go<false, true>(tab, m, s, par, nsm, st);
+        else go<false, false>(tab, m, s, par, nsm, st);
     }
     static void base_pts(const void *tab, const Mesh &m, const State<R> &s, R *bpt, cudaStream_t st) {
-        if constexpr (F32)
+        if constexpr (HAS_DIFF)
             k_base_points<P><<<(m.ntri + 31) / 32, 64, 0, st>>>(static_cast<const DevTables<float, P> *>(tab), m, s.ubv,
                                                                s.ubs, s.ubi, bpt);
     }
@@ -113,7 +123,7 @@ struct Impl {
         l.build = &build;
         l.set_smem = &set_smem;
         l.launch = &launch;
-        if (F32) {
+        if (HAS_DIFF) {
             l.base_pts = &base_pts;
             l.bpt_len = &bpt_len;
         }
@@ -121,22 +131,26 @@ struct Impl {
     }
 };
 
-}  // namespace
-
-template <typename R>
-LineLaunch<R> line_launch(int p) {
+template <typename R, int PHYS>
+LineLaunch<R> pick(int p) {
     switch (p) {
-        case 2: return Impl<R, 2>::get();
-        case 3: return Impl<R, 3>::get();
-        case 4: return Impl<R, 4>::get();
-        case 5: return Impl<R, 5>::get();
-        case 6: return Impl<R, 6>::get();
-        case 7: return Impl<R, 7>::get();
-        case 8: return Impl<R, 8>::get();
+        case 1: return Impl<R, 1, PHYS>::get();
+        case 2: return Impl<R, 2, PHYS>::get();
+        case 3: return Impl<R, 3, PHYS>::get();
+        case 4: return Impl<R, 4, PHYS>::get();
+        case 5: return Impl<R, 5, PHYS>::get();
+        case 6: return Impl<R, 6, PHYS>::get();
+        case 7: return Impl<R, 7, PHYS>::get();
+        case 8: return Impl<R, 8, PHYS>::get();
     }
     return LineLaunch<R>();
 }
-template LineLaunch<double> line_launch<double>(int);
-template LineLaunch<float> line_launch<float>(int);
+
+}  // namespace
+
+template <>
+LineLaunch<LINE_R> line_launch<LINE_R>(int p, int physics) {
+    return physics == HP_PHYS_INS ? pick<LINE_R, 1>(p) : pick<LINE_R, 0>(p);
+}
 
 }  // namespace hpb

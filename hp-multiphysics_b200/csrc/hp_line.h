@@ -33,7 +33,7 @@ constexpr int kLineGeo = 7;
 
 template <typename R>
 struct LineLaunch {
-    // tables as the launcher's kernel parameter; shared-memory attributes; k_rsdl_ins_line
+    // tables as the launcher's kernel parameter; shared-memory attributes; k_rsdl_line
     void (*build)(const hp_basis_tables &, std::vector<unsigned char> &tab) = nullptr;
     cudaError_t (*set_smem)() = nullptr;
     void (*launch)(const void *tab, const Mesh &, const State<R> &, const Phys &, int stage, int zero_rr, int diff,
@@ -43,8 +43,12 @@ struct LineLaunch {
     size_t (*bpt_len)(int ntri) = nullptr;
 };
 
-// The ins line kernel of p, 2 <= p <= HP_MAXP (launch == nullptr otherwise).
+// The line kernel of p and physics, 1 <= p <= HP_MAXP.
 template <typename R>
-LineLaunch<R> line_launch(int p);
+LineLaunch<R> line_launch(int p, int physics);
+template <>
+LineLaunch<double> line_launch<double>(int p, int physics);
+template <>
+LineLaunch<float> line_launch<float>(int p, int physics);
 
 }  // namespace hpb

@@ -197,13 +197,13 @@ int hp_gpu_maxres(hp_gpu_ctx *ctx, double *out, double *mx);
 int hp_gpu_resnorm(hp_gpu_ctx *ctx, double *l2, double *linf);
 
 /* Element kernel of rsdl (no counterpart in the reference, which has one CPU loop,
- * tri_hp/nstage.cpp:52-73). HP_ELEM_TENSOR (the default for ins at p >= 2): the line kernel of
- * both precisions, sum-factorised with one lane per triangle and one warp per line of the
- * tensor-product points; HP_ELEM_POINT (the default for ins at p = 1, and what
- * HP_ELEM_TENSOR runs there): four lanes per triangle, one per Gauss point, the point
- * shares of intgrtrs summed by shuffles; HP_ELEM_SCALAR (cd always): the sum-factorised
- * warp kernel. All give the reference's residual up to rounding. HP_ENOTSUP when the
- * kernel is not built for the context's physics and p. */
+ * tri_hp/nstage.cpp:52-73). The default of both physics is the
+ * line kernel, sum-factorised with one lane per triangle and one warp per line of the
+ * tensor-product points; at p = 1 updates and residuals fuse it with the vertex phase, on
+ * small levels vertex by vertex. HP_ELEM_TENSOR selects it for ins, HP_ELEM_POINT for ins
+ * at p = 1; HP_ELEM_SCALAR: the sum-factorised warp kernel, one warp or lane group per
+ * triangle. All give the reference's residual up to rounding. HP_ENOTSUP when the kernel
+ * cannot be selected for the context's physics and p. */
 #define HP_ELEM_SCALAR 0
 #define HP_ELEM_TENSOR 1
 #define HP_ELEM_POINT 2
