@@ -61,6 +61,31 @@ def test_tensor_core_forward_matches_cpu_oracle():
     assert np.max(np.abs(y - yo)) < 2e-2 * np.max(np.abs(yo))
 
 
+@pytest.mark.parametrize("n0,hidden,n", [(17, 3, 1), (17, 3, 31), (17, 3, 32), (17, 3, 33), (1, 1, 100), (16, 2, 129),
+                                         (24, 5, 257), (32, 4, 64), (17, 3, 148 * 3 * 128 + 5)])
+def test_tensor_core_forward_shapes(n0, hidden, n):
+    """k_mlp_forward_mma at the edges of its fragments: samples of a warp (32) and of all CTAs at
+    once, inputs of one and two k-steps, one to five hidden layers. The inputs start at an address
+    that is a multiple of 4 only. The bounds are those of the test above (the same BF16 roundings)."""
+    import torch
+    widths = (n0,) + (64,) * hidden + (1,)
+    net = LR.MLP(widths, seed=3)
+    rng = np.random.default_rng(n)
+    X = rng.normal(size=(n, n0)).astype(np.float32)
+    net.set_norm(np.full(n0, 0.1), np.full(n0, 1.3))
+    Xd = torch.empty(n * n0 + 1, device="cuda")
+    Xd[1:] = torch.from_numpy(X.ravel()).cuda()
+    Y = torch.full((n + 1, 1), np.nan, device="cuda")
+    torch.cuda.synchronize()
+    net.forward(Xd.data_ptr() + 4, Y.data_ptr(), n)
+    torch.cuda.synchronize()
+    y = Y.cpu().numpy()
+    yo = MO.forward(net.params().astype(np.float64), widths, np.full(n0, 0.1), np.full(n0, 1.3), X)[-1]
+    assert np.all(np.isfinite(y[:n])) and np.isnan(y[n, 0])
+    assert np.linalg.norm(y[:n] - yo) < 2e-3 * np.linalg.norm(yo) + 1e-6
+    assert np.max(np.abs(y[:n] - yo)) < 2e-2 * np.max(np.abs(yo))
+
+
 def test_training_reduces_loss():
     rng = np.random.default_rng(1)
     X = rng.normal(size=(4096, 17)).astype(np.float32)
