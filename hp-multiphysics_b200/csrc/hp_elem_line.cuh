@@ -162,9 +162,67 @@ __global__ void k_base_points(const DevTables<float, P> *__restrict__ tb, Mesh m
     }
 }
 
+// Boundary fluxes of bdry_ins::generic (hp_boundary.cpp:973-1049, ins/bdry_ins.h:35-50) of the
+// kernel's share of the boundary edges, 16 lanes an edge: lane k < G evaluates the flux at Gauss
+// point k, lane m < SM + 2 integrates it against the side's function m (end 0, end 1, side modes).
+// It runs in the element kernel before its first batch, whose copies are in flight meanwhile: as a
+// kernel of its own, one thread an edge, it was 7 to 14 us of every stage.
+template <typename R, int P, bool DIFF>
+__device__ __forceinline__ void line_bdry_flux(const DevTables<R, P> *__restrict__ tb, const Mesh &mesh,
+                                               const State<R> &st, R rho) {
+    constexpr int G = P + 1, SM = P - 1, NM = SM + 2;
+    const int l = threadIdx.x & 15, per = blockDim.x >> 4, lg = l < G ? l : 0, lm = l < NM ? l : 0;
+    const unsigned mask = 0xffffu << (threadIdx.x & 16);
+    // from the last CTA on: those have a batch less when the batches do not come out even
+    for (int e = (gridDim.x - 1 - blockIdx.x) * per + (threadIdx.x >> 4); e < mesh.nbseg; e += gridDim.x * per) {
+        if ((mesh.bkind[e] & (0xF << 8)) != (1 << 8)) continue;
+        const int sd = mesh.bseg[e], v0 = mesh.seg_pnt[2 * sd], v1 = mesh.seg_pnt[2 * sd + 1];
+        // normal at the lane's point (straight side, or its position modes: crdtocht1d)
+        R dx = (R)mesh.pnts[2 * v0] * tb->dgx[lg][1] + (R)mesh.pnts[2 * v1] * tb->dgx[lg][2];
+        R dy = (R)mesh.pnts[2 * v0 + 1] * tb->dgx[lg][1] + (R)mesh.pnts[2 * v1 + 1] * tb->dgx[lg][2];
+        if (mesh.bcrd)
+            for (int m = 0; m < SM; ++m) {
+                dx += (R)mesh.bcrd[((size_t)e * SM + m) * 2] * tb->dgx[lg][m + 3];
+                dy += (R)mesh.bcrd[((size_t)e * SM + m) * 2 + 1] * tb->dgx[lg][m + 3];
+            }
+        auto value = [&](const R *uv, const R *us, int n) {
+            R a = uv[(size_t)v0 * 3 + n] * tb->gx[lg][1] + uv[(size_t)v1 * 3 + n] * tb->gx[lg][2];
+#pragma unroll
+            for (int m = 0; m < SM; ++m) a += us[((size_t)sd * SM + m) * 3 + n] * tb->gx[lg][m + 3];
+            return a;
+        };
+        const R u0 = value(st.ugv, st.ugs, 0), u1 = value(st.ugv, st.ugs, 1);
+        const R fm = rho * (u0 * dy - u1 * dx);
+        R f[3] = {(R)0, (R)0, fm};
+        if constexpr (DIFF) {  // F(b + d) - F(b); the boundary pressure cancels
+            const R b0 = value(st.ubv, st.ubs, 0), b1 = value(st.ubv, st.ubs, 1), mb = rho * (b0 * dy - b1 * dx);
+            f[0] = fm * (b0 + u0) + mb * u0;
+            f[1] = fm * (b1 + u1) + mb * u1;
+        } else {
+            const R pb = (R)mesh.bpibc[e * G + lg];
+            f[0] = fm * u0 + pb * dy;
+            f[1] = fm * u1 - pb * dx;
+        }
+        R acc[3] = {(R)0, (R)0, (R)0};
+#pragma unroll
+        for (int k = 0; k < G; ++k) {
+            const R w = tb->gxwtx[lm + 1][k];
+#pragma unroll
+            for (int n = 0; n < 3; ++n) acc[n] += w * __shfl_sync(mask, f[n], k, 16);
+        }
+        if (l < NM)
+            for (int n = 0; n < 3; ++n) {
+                if (st.bres) st.bres[((size_t)e * NM + l) * 3 + n] = acc[n];
+                else if (l < 2) atomic_add(st.resv + (size_t)(l ? v1 : v0) * 3 + n, acc[n]);
+                else atomic_add(st.ress + ((size_t)sd * SM + l - 2) * 3 + n, acc[n]);
+            }
+    }
+}
+
 template <typename R, int P, int PHYS, bool DIFF, bool RE>
 __global__ void __launch_bounds__(LineCfg<R, P, PHYS, DIFF>::NTHR, LineCfg<R, P, PHYS, DIFF>::MINB)
-    k_rsdl_line(const __grid_constant__ LineTab<R, P> tab, Mesh mesh, State<R> st, LinePar par) {
+    k_rsdl_line(const __grid_constant__ LineTab<R, P> tab, const DevTables<R, P> *__restrict__ gtab, Mesh mesh,
+                State<R> st, LinePar par) {
     using C = LineCfg<R, P, PHYS, DIFF>;
     constexpr int G = C::G, X = C::X, T = C::T, SM = C::SM, IM = C::IM, BM = C::BM, NV = C::NV, NTHR = C::NTHR;
     constexpr bool INS = PHYS == 1;
@@ -247,6 +305,7 @@ __global__ void __launch_bounds__(LineCfg<R, P, PHYS, DIFF>::NTHR, LineCfg<R, P,
     cp_async_wait();
     __syncthreads();
     fetch_u(b, 0);
+    if constexpr (INS && P > 1) line_bdry_flux<R, P, DIFF>(gtab, mesh, st, rho);
     for (; b < nbatch; b += step, slot = slot == 2 ? 0 : slot + 1) {
         const int *idx = ring + slot * C::IDX;
         const int t0 = b * 32;

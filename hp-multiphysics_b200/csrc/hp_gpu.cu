@@ -356,6 +356,8 @@ struct hp_gpu_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
     bool own_stream = false;
+    cudaStream_t side = nullptr;  // curved elements, beside the straight ones (meshes that have some)
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     int p = 0, NV = 0, npnt = 0, nseg = 0, ntri = 0, nbseg = 0, sm = 0, im = 0, nsm = 148;
     int ncurved = 0;  // curved elements (tri.info > -1)
     Phys ph{};
@@ -708,6 +710,12 @@ extern "C" int hp_gpu_create(const hp_mesh_desc *m, const hp_basis_tables *b, co
             if ((r = upload(c, &d_ctri, crv_tri.data(), crv_tri.size()))) return fail(r);
             M.tri_cv = d_cv; M.crv_cht = d_cht; M.bcrd = d_bcrd; M.ncurved = ncv; M.crv_tri = d_ctri;
             c->ncurved = ncv;
+            if (cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking) != cudaSuccess ||
+                cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
+                cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming) != cudaSuccess) {
+                set_err("stream of the curved elements");
+                return fail(HP_ECUDA);
+            }
         }
     }
 
@@ -794,6 +802,9 @@ extern "C" int hp_gpu_destroy(hp_gpu_ctx *c) {
     if (c->g_update32) cudaGraphExecDestroy(c->g_update32);
     for (void *p : c->allocs) cudaFreeAsync(p, c->stream);
     if (c->stream) cudaStreamSynchronize(c->stream);
+    if (c->side) cudaStreamDestroy(c->side);
+    if (c->ev_fork) cudaEventDestroy(c->ev_fork);
+    if (c->ev_join) cudaEventDestroy(c->ev_join);
     if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
     delete c;
     return HP_OK;
@@ -878,10 +889,10 @@ static const Tune &tune_of(hp_gpu_ctx *c, double) { return c->tune[0]; }
 static const Tune &tune_of(hp_gpu_ctx *c, float) { return c->tune[1]; }
 
 static void launch_line(hp_gpu_ctx *c, const State<double> &st, const Phys &ph, int stage, int zero_rr, int diff) {
-    c->line.launch(c->line_tab.data(), c->mesh, st, ph, stage, zero_rr, diff, c->nsm, c->stream);
+    c->line.launch(c->line_tab.data(), c->d_tab, c->mesh, st, ph, stage, zero_rr, diff, c->nsm, c->stream);
 }
 static void launch_line(hp_gpu_ctx *c, const State<float> &st, const Phys &ph, int stage, int zero_rr, int diff) {
-    c->line32.launch(c->line_tab32.data(), c->mesh, st, ph, stage, zero_rr, diff, c->nsm, c->stream);
+    c->line32.launch(c->line_tab32.data(), c->d_tab32, c->mesh, st, ph, stage, zero_rr, diff, c->nsm, c->stream);
 }
 
 // Element part of rsdl(stage): the stored cd element operators once built, else the
@@ -892,8 +903,15 @@ static void launch_elem(hp_gpu_ctx *c, const Launchers<R> &L, const void *tab, c
     if (c->emat_on && c->emat_built && ph.physics == HP_PHYS_CD && !diff)
         L.emat_apply(emat_of(c, R()), c->mesh, st, ph, stage, zero_rr, c->nsm, tune_of(c, R()), c->stream);
     else if (c->elem_kind != HP_ELEM_SCALAR) {
+        // the curved triangles beside the straight ones, on a stream of their own (other slots)
+        if (c->side) {
+            cudaEventRecord(c->ev_fork, c->stream);
+            cudaStreamWaitEvent(c->side, c->ev_fork, 0);
+            L.curved(tab, c->mesh, st, ph, stage, zero_rr, diff, c->nsm, tune_of(c, R()), c->side);
+            cudaEventRecord(c->ev_join, c->side);
+        }
         launch_line(c, st, ph, stage, zero_rr, diff);
-        L.curved(tab, c->mesh, st, ph, stage, zero_rr, diff, c->nsm, tune_of(c, R()), c->stream);
+        if (c->side) cudaStreamWaitEvent(c->stream, c->ev_join, 0);
     }
     else
         L.elem(tab, c->mesh, st, ph, stage, zero_rr, diff, c->nsm, tune_of(c, R()), c->stream);
@@ -910,8 +928,8 @@ static void enqueue_rsdl_t(hp_gpu_ctx *c, const Launchers<R> &L, const void *tab
         // assembly by gather: the element and boundary kernels write per-element and
         // per-edge values, k_assemble forms res and res_r of the vertices and sides
         launch_elem<R>(c, L, tab, st, ph, stage, zero_rr, diff);
-        L.bflux(tab, c->mesh, st, ph, diff, c->stream);
-        const long n = (long)c->npnt + (long)c->nseg * c->sm;
+        if (c->elem_kind == HP_ELEM_SCALAR) L.bflux(tab, c->mesh, st, ph, diff, c->stream);
+        const long n = (long)(c->lv + c->ls);
         const int with_b = (ph.physics == HP_PHYS_INS && c->nbseg > 0) ? 1 : 0;
         k_assemble<R><<<std::min(nblk(n, 256), c->nsm * 16), 256, 0, c->stream>>>(
             c->mesh, st, c->NV, c->sm, (R)omb, zero_rr, ph.beta[stage] > 0.0 ? 1 : 0, with_b, fold);
@@ -921,7 +939,7 @@ static void enqueue_rsdl_t(hp_gpu_ctx *c, const Launchers<R> &L, const void *tab
     k_rsdl_pre<R><<<std::min(nblk(n, 256), c->nsm * 8), 256, 0, c->stream>>>((int)c->lv, (int)c->ls, st.resv, st.ress,
                                                                            st.rrv, st.rrs, (R)omb, zero_rr);
     launch_elem<R>(c, L, tab, st, ph, stage, zero_rr, diff);
-    L.bflux(tab, c->mesh, st, ph, diff, c->stream);
+    if (c->elem_kind == HP_ELEM_SCALAR) L.bflux(tab, c->mesh, st, ph, diff, c->stream);
     if (fold) {
         const long nf = (long)(c->lv + c->ls);
         k_rsdl_fold<R><<<nblk(nf, 256), 256, 0, c->stream>>>((int)c->lv, (int)c->ls, st.resv, st.rrv, st.ress, st.rrs,
@@ -1017,10 +1035,16 @@ static void enqueue_update_t(hp_gpu_ctx *c, const Launchers<R> &L, const void *t
         enqueue_p1_update<R>(c, L, tab, st, ph, diff, slot);
         return;
     }
+    // the assembly by gather leaves res complete (res_r and the source added once) and the
+    // preconditioner reads that alone; after atomics it adds them itself
+    const int gathered = st.elim ? 1 : 0;
+    State<R> sm = st;
+    if (gathered) sm.dresv = sm.dress = nullptr;
     for (int stage = 0; stage < ph.nstage; ++stage) {
-        enqueue_rsdl_t<R>(c, L, tab, st, ph, stage, diff);
+        enqueue_rsdl_t<R>(c, L, tab, st, ph, stage, diff, gathered);
         const double cfla = ph.alpha[stage] * ph.cfl;
-        enqueue_minvrt_t<R>(c, L, st, mt, cfla, stage == 0 ? 2 : 1, 1, stage == ph.nstage - 1 ? slot : nullptr);
+        enqueue_minvrt_t<R>(c, L, sm, mt, cfla, stage == 0 ? 2 : 1, !gathered,
+                            stage == ph.nstage - 1 ? slot : nullptr);
     }
 }
 
@@ -1396,6 +1420,8 @@ static int alloc_mixed(hp_gpu_ctx *c) {
         if ((r = dalloc(c, (void **)&c->d_bpt32, c->line32.bpt_len(c->ntri) * 4))) return r;
         f.bpt = c->d_bpt32;
     }
+    // element slots at p = 1 (k_vert_p1 reads them); above, the atomics are the faster assembly in
+    // FP32 (an update of 131k triangles with slots / atomics: p = 3 577 / 522 us, p = 6 2107 / 2031)
     if (c->p == 1) {
         const size_t nsl = (size_t)3 * c->ntri * c->NV;
         if ((r = dalloc(c, (void **)&c->d_p1u32, c->lv * 4)) || (r = dalloc(c, (void **)&c->d_elim32, nsl * 4)) ||
@@ -1756,15 +1782,44 @@ extern "C" int hp_gpu_mg_prolongate(hp_gpu_ctx *coarse) {
     return hp_gpu_sync(coarse->fine);
 }
 
+// Preconditioner set-up inside a cycle: bad elements accumulate in the context's count, which the
+// driver reads once after the cycle (cycle_errors) instead of waiting for the device at every visit.
+static int cycle_prcn(hp_gpu_ctx *c) {
+    const int r = enqueue_prcn(c);
+    if (r) return r;
+    c->prcn_ready = true;
+    return HP_OK;
+}
+
+// HP_ESTATE if a set-up of the cycle met bad elements; the counts start anew.
+static int cycle_errors(hp_gpu_ctx **lv, int n) {
+    std::vector<int> bad(n, 0);
+    for (int l = 0; l < n; ++l) {
+        CK(cudaMemcpyAsync(&bad[l], lv[l]->d_err, 4, cudaMemcpyDeviceToHost, lv[l]->stream));
+        CK(cudaMemsetAsync(lv[l]->d_err, 0, 4, lv[l]->stream));
+    }
+    int any = 0;
+    for (int l = 0; l < n; ++l) {
+        CK(cudaStreamSynchronize(lv[l]->stream));
+        any |= bad[l];
+    }
+    if (any) {
+        set_err("bad elements in a preconditioner set-up");
+        return HP_ESTATE;
+    }
+    return HP_OK;
+}
+static int cycle_begin(hp_gpu_ctx **lv, int n) {
+    for (int l = 0; l < n; ++l) CK(cudaMemsetAsync(lv[l]->d_err, 0, 4, lv[l]->stream));
+    return HP_OK;
+}
+
 // block::cycle (tri_mesh/blocks.cpp:1267-1348) over levels[0] (finest) .. levels[n-1]
 static int cycle(hp_gpu_ctx **lv, int n, int lvl, int vw, int itercrsn, int iterrfne, int eval_prcn) {
     hp_gpu_ctx *c = lv[lvl];
     int r;
     for (int vc = 0; vc < vw; ++vc) {
-        if (eval_prcn) {
-            r = hp_gpu_setup_preconditioner(c);
-            if (r) return r < 0 ? r : HP_ESTATE;
-        }
+        if (eval_prcn && (r = cycle_prcn(c))) return r;
         if ((r = fas_first(c))) return r;
         if ((r = ensure_update_graph(c))) return r;
         for (int it = 0; it < itercrsn; ++it) CK(cudaGraphLaunch(c->g_update, c->stream));
@@ -1773,10 +1828,7 @@ static int cycle(hp_gpu_ctx **lv, int n, int lvl, int vw, int itercrsn, int iter
         if ((r = mg_restrict_enqueue(lv[lvl + 1]))) return r;
         if ((r = cycle(lv, n, lvl + 1, vw, itercrsn, iterrfne, eval_prcn))) return r;
         if ((r = mg_prolong_enqueue(lv[lvl + 1]))) return r;
-        if (eval_prcn && iterrfne) {
-            r = hp_gpu_setup_preconditioner(c);
-            if (r) return r < 0 ? r : HP_ESTATE;
-        }
+        if (eval_prcn && iterrfne && (r = cycle_prcn(c))) return r;
         for (int it = 0; it < iterrfne; ++it) CK(cudaGraphLaunch(c->g_update, c->stream));
     }
     return HP_OK;
@@ -1786,8 +1838,9 @@ extern "C" int hp_gpu_vcycle(hp_gpu_ctx **levels, int nlevels, int vw, int iterc
     if (!levels || nlevels < 1 || vw < 1 || itercrsn < 0 || iterrfne < 0) return HP_EINVAL;
     for (int l = 1; l < nlevels; ++l)
         if (!levels[l] || levels[l]->fine != levels[l - 1]) { set_err("level %d is not attached to level %d", l, l - 1); return HP_EINVAL; }
-    int r = cycle(levels, nlevels, 0, vw, itercrsn, iterrfne, eval_prcn);
-    if (r) return r;
+    int r = cycle_begin(levels, nlevels);
+    if (r || (r = cycle(levels, nlevels, 0, vw, itercrsn, iterrfne, eval_prcn))) return r;
+    if (eval_prcn && (r = cycle_errors(levels, nlevels))) return r;
     return hp_gpu_sync(levels[0]);
 }
 
@@ -1812,7 +1865,8 @@ extern "C" int hp_gpu_solve_mg(hp_gpu_ctx **levels, int nlevels, double drop, in
         // every level's preconditioner is evaluated at its state on the first cycle
         // and then every prcn_every cycles (block::cycle's evaluate_preconditioner)
         const int eval = (nc == 0 || (prcn_every > 0 && nc % prcn_every == 0)) ? 1 : 0;
-        if ((r = cycle(levels, nlevels, 0, vw, itercrsn, iterrfne, eval))) return r;
+        if ((r = cycle_begin(levels, nlevels)) || (r = cycle(levels, nlevels, 0, vw, itercrsn, iterrfne, eval))) return r;
+        if (eval && (r = cycle_errors(levels, nlevels))) return r;
         ++nc;
         if ((r = fp64_norm(f, &rn))) return r;
         const double d = rn / r0;
@@ -1921,7 +1975,9 @@ extern "C" int hp_gpu_solve_mg_graph(hp_gpu_ctx **levels, int nlevels, double dr
     if ((r = fp64_norm(f, &r0))) return r;
     if (hist && nh < hist_cap) hist[nh++] = 1.0;
     // first cycle evaluates every level's preconditioner at its own state
-    if ((r = cycle(levels, nlevels, 0, vw, itercrsn, iterrfne, 1))) return r;
+    if ((r = cycle_begin(levels, nlevels)) || (r = cycle(levels, nlevels, 0, vw, itercrsn, iterrfne, 1)) ||
+        (r = cycle_errors(levels, nlevels)))
+        return r;
     ++nc;
     void *g_frozen = nullptr, *g_eval = nullptr;
     if ((r = hp_gpu_capture_vcycle(levels, nlevels, vw, itercrsn, iterrfne, 0, &g_frozen))) return r;

@@ -944,51 +944,47 @@ __global__ void k_bdry_flux_ins(const DevTables<R, P> *__restrict__ tb, Mesh mes
 // (+ the boundary fluxes, hp_edge_bdry::rsdl), res_r = (1 - beta) res_r + sum of their
 // real parts (nstage.cpp:21-49; zero_rr: res_r = sum). A vertex sums its triangles in
 // vertex-incidence order, a side its two triangles in seg.tri order, so the result does
-// not depend on the scheduling. One thread per vertex, then one per (side, mode). fold: res +=
+// not depend on the scheduling. fold: res +=
 // res_r (+ dres), as the stand-alone rsdl leaves it (nstage.cpp:76-82).
+// One thread per value, so that consecutive threads read consecutive slots: with one thread per
+// vertex and per (side, mode), looping over the variables, the residual of 67k triangles at p = 3
+// spent 15.7 us here, now 8.6.
 template <typename R>
 __global__ void k_assemble(Mesh mesh, State<R> st, int NV, int SM, R omb, int zero_rr, int with_re, int with_b,
                            int fold) {
+    const unsigned nv = (unsigned)mesh.npnt * NV, lps = (unsigned)SM * NV, n0 = nv + (unsigned)mesh.nseg * lps;
     const size_t soff = (size_t)3 * mesh.ntri * NV;  // side section of the buffers
-    const long nitems = (long)mesh.npnt + (long)mesh.nseg * SM;
-    for (long k = (long)blockIdx.x * blockDim.x + threadIdx.x; k < nitems; k += (long)gridDim.x * blockDim.x) {
-        if (k < mesh.npnt) {
-            const int v = (int)k, j0 = mesh.vt_ptr[v], j1 = mesh.vt_ptr[v + 1];
-            for (int n = 0; n < NV; ++n) {
-                R sim = (R)0, sre = (R)0;
-                for (int j = j0; j < j1; ++j) {  // contiguous: the buffers are in incidence order
-                    sim += st.elim[(size_t)j * NV + n];
-                    if (with_re) sre += st.elre[(size_t)j * NV + n];
-                }
-                if (with_b)
-                    for (int q = 0; q < 2; ++q) {
-                        const int b = mesh.vb_idx[2 * v + q];
-                        if (b >= 0 && (mesh.bkind[b >> 1] & (0xF << 8)) == (1 << 8))
-                            sim += st.bres[((size_t)(b >> 1) * (SM + 2) + (b & 1)) * NV + n];
-                    }
-                const R r0 = zero_rr ? (R)0 : st.rrv[v * NV + n] * omb, rr = with_re ? r0 + sre : r0;
-                st.rrv[v * NV + n] = rr;
-                st.resv[v * NV + n] = fold ? sim + (rr + (st.dresv ? st.dresv[v * NV + n] : (R)0)) : sim;
+    for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k < n0; k += gridDim.x * blockDim.x) {
+        R sim = (R)0, sre = (R)0;
+        if (k < nv) {
+            const int v = (int)(k / NV), n = (int)(k - v * NV), j1 = mesh.vt_ptr[v + 1];
+            for (int j = mesh.vt_ptr[v]; j < j1; ++j) {  // contiguous: the buffers are in incidence order
+                sim += st.elim[(size_t)j * NV + n];
+                if (with_re) sre += st.elre[(size_t)j * NV + n];
             }
+            if (with_b)
+                for (int q = 0; q < 2; ++q) {
+                    const int b = mesh.vb_idx[2 * v + q];
+                    if (b >= 0 && (mesh.bkind[b >> 1] & (0xF << 8)) == (1 << 8))
+                        sim += st.bres[((size_t)(b >> 1) * (SM + 2) + (b & 1)) * NV + n];
+                }
+            const R r0 = zero_rr ? (R)0 : st.rrv[k] * omb, rr = with_re ? r0 + sre : r0;
+            st.rrv[k] = rr;
+            st.resv[k] = fold ? sim + (rr + (st.dresv ? st.dresv[k] : (R)0)) : sim;
         } else {
-            const long q = k - mesh.npnt;
-            const int sd = (int)(q / SM), kk = (int)(q - (long)sd * SM);
-            const int e = with_b ? mesh.seg_bdry[sd] : -1;
-            const bool bf = e >= 0 && (mesh.bkind[e] & (0xF << 8)) == (1 << 8);
-            for (int n = 0; n < NV; ++n) {
-                R sim = (R)0, sre = (R)0;
-                for (int side = 0; side < 2; ++side) {
-                    if (mesh.seg_tri[2 * sd + side] < 0) continue;
-                    const size_t idx = soff + ((size_t)(2 * sd + side) * SM + kk) * NV + n;
-                    sim += st.elim[idx];
-                    if (with_re) sre += st.elre[idx];
-                }
-                if (bf) sim += st.bres[((size_t)e * (SM + 2) + 2 + kk) * NV + n];
-                const size_t g = ((size_t)sd * SM + kk) * NV + n;
-                const R r0 = zero_rr ? (R)0 : st.rrs[g] * omb, rr = with_re ? r0 + sre : r0;
-                st.rrs[g] = rr;
-                st.ress[g] = fold ? sim + (rr + (st.dress ? st.dress[g] : (R)0)) : sim;
+            const unsigned g = k - nv;
+            const int sd = (int)(g / lps), r = (int)(g - sd * lps);
+            for (int side = 0; side < 2; ++side) {
+                if (mesh.seg_tri[2 * sd + side] < 0) continue;
+                const size_t idx = soff + (size_t)(2 * sd + side) * lps + r;
+                sim += st.elim[idx];
+                if (with_re) sre += st.elre[idx];
             }
+            const int e = with_b ? mesh.seg_bdry[sd] : -1;
+            if (e >= 0 && (mesh.bkind[e] & (0xF << 8)) == (1 << 8)) sim += st.bres[(size_t)e * (SM + 2) * NV + 2 * NV + r];
+            const R r0 = zero_rr ? (R)0 : st.rrs[g] * omb, rr = with_re ? r0 + sre : r0;
+            st.rrs[g] = rr;
+            st.ress[g] = fold ? sim + (rr + (st.dress ? st.dress[g] : (R)0)) : sim;
         }
     }
 }
@@ -1270,7 +1266,7 @@ __global__ void k_minv_int_flat(Mesh mesh, State<R> st, const DevMinv<R> *__rest
     // the tables in shared memory, staged per block
     __shared__ R s_bfmi[3 + 3 * SM][IM], s_idiag[IM][2];
     for (int x = threadIdx.x; x < (3 + 3 * SM) * IM; x += blockDim.x) s_bfmi[x / IM][x % IM] = mt->bfmi[x / IM][x % IM];
-    for (int x = threadIdx.x; x < 2 * IM; x += blockDim.x) s_idiag[x / 2][x % 2] = mt->idiag[x / 2][x % 2];
+    for (int x = threadIdx.x; x < 2 * IM; x += blockDim.x) s_idiag[x / 2][x % 2] = x % 2 ? (R)1 / mt->idiag[x / 2][1] : mt->idiag[x / 2][0];
     __syncthreads();
     const long gid = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (gid >= (long)mesh.ntri * NV) return;
@@ -1278,19 +1274,20 @@ __global__ void k_minv_int_flat(Mesh mesh, State<R> st, const DevMinv<R> *__rest
     R b[IM];
 #pragma unroll
     for (int k = 0; k < IM; ++k) b[k] = st.resi[((size_t)t * IM + k) * NV + n];
+    // (s_idiag[i][1] holds the reciprocal: a thread had 3 IM divisions)
 #pragma unroll
     for (int i = 0; i < IM; ++i) {
         if (i >= 1) b[i] -= s_idiag[i][0] * b[0];
-        b[i] /= s_idiag[i][1];
+        b[i] *= s_idiag[i][1];
     }
 #pragma unroll
     for (int i = IM - 1; i >= 0; --i) {
-        b[i] /= s_idiag[i][1];
+        b[i] *= s_idiag[i][1];
         if (i >= 1) b[0] -= s_idiag[i][0] * b[i];
     }
-    const R tp = st.tprcn[t * NV + n];
+    const R tp = (R)1 / st.tprcn[t * NV + n];
 #pragma unroll
-    for (int k = 0; k < IM; ++k) b[k] /= tp;
+    for (int k = 0; k < IM; ++k) b[k] *= tp;
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
         const R u = st.resv[mesh.tri_pnt[3 * t + i] * NV + n];

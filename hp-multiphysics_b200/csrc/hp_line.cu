@@ -85,13 +85,13 @@ struct Impl {
         return e;
     }
     template <bool DIFF, bool RE>
-    static void go(const void *tab, const Mesh &m, const State<R> &s, const LinePar &par, int nsm, cudaStream_t st) {
+    static void go(const void *tab, const void *gtab, const Mesh &m, const State<R> &s, const LinePar &par, int nsm, cudaStream_t st) {
         using C = LineCfg<R, P, PHYS, DIFF>;
         const int nb = (m.ntri + 31) / 32;
         k_rsdl_line<R, P, PHYS, DIFF, RE><<<std::min(nb, nsm * C::MINB), C::NTHR, C::SMEM, st>>>(
-            *static_cast<const LineTab<R, P> *>(tab), m, s, par);
+            *static_cast<const LineTab<R, P> *>(tab), static_cast<const DevTables<R, P> *>(gtab), m, s, par);
     }
-    static void launch(const void *tab, const Mesh &m, const State<R> &s, const Phys &ph, int stage, int zero_rr,
+    static void launch(const void *tab, const void *gtab, const Mesh &m, const State<R> &s, const Phys &ph, int stage, int zero_rr,
                        int diff, int nsm, cudaStream_t st) {
         LinePar par;
         par.beta = ph.beta[stage];
@@ -102,13 +102,13 @@ struct Impl {
         const bool re = ph.beta[stage] > 0.0;
         if constexpr (HAS_DIFF) {
             if (diff) {
-                if (re) go<true, true>(tab, m, s, par, nsm, st);
-                else go<true, false>(tab, m, s, par, nsm, st);
+                if (re) go<true, true>(tab, gtab, m, s, par, nsm, st);
+                else go<true, false>(tab, gtab, m, s, par, nsm, st);
                 return;
             }
         }
-        if (re) go<false, true>(tab, m, s, par, nsm, st);
-        else go<false, false>(tab, m, s, par, nsm, st);
+        if (re) go<false, true>(tab, gtab, m, s, par, nsm, st);
+        else go<false, false>(tab, gtab, m, s, par, nsm, st);
     }
     static void base_pts(const void *tab, const Mesh &m, const State<R> &s, R *bpt, cudaStream_t st) {
         if constexpr (HAS_DIFF)

@@ -33,10 +33,11 @@ constexpr int kLineGeo = 7;
 
 template <typename R>
 struct LineLaunch {
-    // tables as the launcher's kernel parameter; shared-memory attributes; k_rsdl_line
+    // tables as the launcher's kernel parameter; shared-memory attributes; k_rsdl_line, with the
+    // level's DevTables on the device (ins at p > 1: the boundary fluxes, too)
     void (*build)(const hp_basis_tables &, std::vector<unsigned char> &tab) = nullptr;
     cudaError_t (*set_smem)() = nullptr;
-    void (*launch)(const void *tab, const Mesh &, const State<R> &, const Phys &, int stage, int zero_rr, int diff,
+    void (*launch)(const void *tab, const void *dev_tables, const Mesh &, const State<R> &, const Phys &, int stage, int zero_rr, int diff,
                    int nsm, cudaStream_t) = nullptr;
     // FP32: the base state's point values of the correction form (State::bpt), their number
     void (*base_pts)(const void *dev_tables, const Mesh &, const State<R> &, R *bpt, cudaStream_t) = nullptr;
