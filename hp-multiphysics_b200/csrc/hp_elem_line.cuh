@@ -38,18 +38,24 @@
 
 namespace hpb {
 
-template <typename R, int P, int PHYS, bool DIFF>
+template <typename R, int P, int PHYS, bool DIFF, bool RE>
 struct LineCfg {
     static constexpr int G = P + 1, GG = G * G, X = P + 2, T = (P + 1) * (P + 2) / 2, SM = P - 1,
                          IM = (P - 1) * (P - 2) / 2, BM = 3 * P, NV = PHYS == 1 ? 3 : 1;
     static constexpr int NTHR = 32 * G;
-    static constexpr int U = 0;                // gathered modes [NV T][33]
-    static constexpr int OUT = NV * T * 33;    // results [NV T][33]
-    static constexpr int EX = 2 * NV * T * 33; // s fluxes [NV][G][G][32], then A, B [NV][2][X][G][32]
+    // FP64, p = 6, a stage without the real part: the modes are gathered into the exchange area, once
+    // that has been read, instead of into an area of their own, so that a second CTA fits an SM (its
+    // 128 registers a thread hold what such a stage keeps; 131k triangles: 246 -> 159 us). With the
+    // real part the point data do not fit: 404 us with two CTAs against 413, 30 against 22 us on 2k
+    // triangles. p = 7, 8 need more than half of the shared memory, p <= 5 have two CTAs as it is.
+    static constexpr bool TIGHT = PHYS == 1 && G == 7 && sizeof(R) == 8 && !RE;
+    static constexpr int OUT = 0;                           // results [NV T][33]
+    static constexpr int U = NV * T * 33;                   // gathered modes [NV T][33]
+    static constexpr int EX = TIGHT ? U : 2 * NV * T * 33;  // s fluxes [NV][G][G][32], then A, B [NV][2][X][G][32]
     static constexpr int LEN = EX + 2 * NV * X * G * 32;
     static constexpr int IDX = 16 * 32;        // connectivity of a batch: pnt, seg, sgn, vpos, spos [32][3] each, tri_cv [32]
     static constexpr int LPS = SM > 0 ? SM * NV : 1, LPI = IM > 0 ? IM * NV : 1;  // values of a side, of an interior
-    static constexpr int XH = NV == 3 ? (X + 1) / 2 : X;  // columns whose x sums share the registers
+    static constexpr int XH = NV == 1 ? X : (X + 1) / 2;  // columns whose x sums share the registers
     static constexpr int SMEM = LEN * (int)sizeof(R) + 3 * IDX * 4;
     static constexpr int by_smem = 227 * 1024 / (SMEM + 1024);
     // CTAs an SM, as many as leave the point data in registers (ins, 131k triangles, FP64: p = 4 with
@@ -58,7 +64,7 @@ struct LineCfg {
     // 4932, 4052
     static constexpr int by_cd = G <= 2 ? 8 : G <= 4 ? 6 : G == 5 ? 5 : G == 6 ? 4 : G == 7 ? 3 : 2;
     static constexpr int by_regs = PHYS == 0 ? (sizeof(R) == 8 ? by_cd : 2 * by_cd)
-                                 : sizeof(R) == 8 ? (G == 2 ? 8 : G == 3 ? 5 : G == 4 ? 4 : G == 5 ? 3 : G == 6 ? 2 : 1)
+                                 : sizeof(R) == 8 ? (G == 2 ? 8 : G == 3 ? 5 : G == 4 ? 4 : G == 5 ? 3 : G == 6 || TIGHT ? 2 : 1)
                                                   : (G == 2 ? 12 : G == 3 ? 8 : G <= 5 ? 5 : G == 6 ? 4 : G == 7 ? 3 : 2);
     static constexpr int MINB = by_smem < by_regs ? (by_smem < 1 ? 1 : by_smem) : by_regs;
 };
@@ -220,10 +226,10 @@ __device__ __forceinline__ void line_bdry_flux(const DevTables<R, P> *__restrict
 }
 
 template <typename R, int P, int PHYS, bool DIFF, bool RE>
-__global__ void __launch_bounds__(LineCfg<R, P, PHYS, DIFF>::NTHR, LineCfg<R, P, PHYS, DIFF>::MINB)
+__global__ void __launch_bounds__(LineCfg<R, P, PHYS, DIFF, RE>::NTHR, LineCfg<R, P, PHYS, DIFF, RE>::MINB)
     k_rsdl_line(const __grid_constant__ LineTab<R, P> tab, const DevTables<R, P> *__restrict__ gtab, Mesh mesh,
                 State<R> st, LinePar par) {
-    using C = LineCfg<R, P, PHYS, DIFF>;
+    using C = LineCfg<R, P, PHYS, DIFF, RE>;
     constexpr int G = C::G, X = C::X, T = C::T, SM = C::SM, IM = C::IM, BM = C::BM, NV = C::NV, NTHR = C::NTHR;
     constexpr bool INS = PHYS == 1;
     const R beta = (R)par.beta, omb = (R)par.omb, rho = (R)par.rho;
@@ -288,7 +294,7 @@ __global__ void __launch_bounds__(LineCfg<R, P, PHYS, DIFF>::NTHR, LineCfg<R, P,
             inner = true;
             row = n * T + BM + k;
         }
-        R *dst = sm + row * 33;
+        R *dst = sm + C::U + row * 33;
 #pragma unroll
         for (int it = 0; it < (32 + TPP - 1) / TPP; ++it) {
             const int e = sub + it * TPP;
@@ -352,6 +358,7 @@ __global__ void __launch_bounds__(LineCfg<R, P, PHYS, DIFF>::NTHR, LineCfg<R, P,
             for (int c = 0; c < X; ++c) wu[c] = wu1[c] = (R)0;
 #pragma unroll
             for (int c = 0; c < XV; ++c) wv[c] = wp[c] = wv1[c] = (R)0;
+            const R *um = sm + C::U + lane;
             int jl = j;  // anew in each batch: the line's table entries are not kept across the loop
             asm volatile("" : "+r"(jl));
             each_mode([&](auto mm) {
@@ -359,12 +366,12 @@ __global__ void __launch_bounds__(LineCfg<R, P, PHYS, DIFF>::NTHR, LineCfg<R, P,
                 constexpr bool odd = m >= 3 && m < BM && (((m - 3) % (SM > 0 ? SM : 1)) & 1);
                 const int bit = odd ? sbit[odd ? (m - 3) / (SM > 0 ? SM : 1) : 0] : 0;
                 const R2<R> g = tab.g[jl][m];
-                R x = sm[m * 33 + lane];
+                R x = um[m * 33];
                 if constexpr (odd) flip_if(x, bit);
                 wu[c] += x * g.x;
                 if constexpr (RE) wu1[c] += x * g.y;
                 if constexpr (INS) {
-                    R y = sm[(T + m) * 33 + lane], z = sm[(2 * T + m) * 33 + lane];
+                    R y = um[(T + m) * 33], z = um[(2 * T + m) * 33];
                     if constexpr (odd) {
                         flip_if(y, bit);
                         flip_if(z, bit);
@@ -606,6 +613,7 @@ __global__ void __launch_bounds__(LineCfg<R, P, PHYS, DIFF>::NTHR, LineCfg<R, P,
                 }
             }
         };
+        if constexpr (C::TIGHT) __syncthreads();  // the gathered modes have been read
         xsums([&](int i, R (&fr)[NV], R (&fs)[NV]) {
             if constexpr (INS) {
                 conv(i, fr[2], fs[2], fr[0], fs[0], fr[1], fs[1]);
@@ -629,6 +637,21 @@ __global__ void __launch_bounds__(LineCfg<R, P, PHYS, DIFF>::NTHR, LineCfg<R, P,
         constexpr int NKEEP = IM > 0 ? (32 + TPI - 1) / TPI : 1;
         R keep[NKEEP];
         auto act = [&](int e) { return t0 + e <= last && (!mesh.tri_cv || idx[480 + e] < 0); };
+        // res_r of the interior values, in a stage without the real part: read ahead of the sums
+        // (FP64: p = 6 165 -> 159 us; FP32 has no registers to hold them, an update 2018 -> 2060 us)
+        constexpr bool RRI = sizeof(R) == 8 && !RE;
+        auto load_rr = [&]() {
+            const int sub = tid / C::LPI, r = tid - sub * C::LPI;
+            if constexpr (RRI && IM > 0) {
+#pragma unroll
+                for (int it = 0; it < NKEEP; ++it) {
+                    const int e = sub + it * TPI;
+                    keep[it] = (R)0;
+                    if (omb != (R)0 && sub < TPI && e < 32 && t0 + e <= last)
+                        keep[it] = st.rri[(size_t)(t0 + e) * C::LPI + r] * omb;
+                }
+            }
+        };
         auto scatter = [&](int part) {
             const int tid = fresh_tid();
             {
@@ -669,7 +692,7 @@ __global__ void __launch_bounds__(LineCfg<R, P, PHYS, DIFF>::NTHR, LineCfg<R, P,
                         if (!act(e)) continue;
                         const R val = out[(NV * BM + r) * 33 + e];
                         const size_t gi = (size_t)(t0 + e) * C::LPI + r;
-                        const R rr = omb != (R)0 && (part || !RE) ? st.rri[gi] * omb : (R)0;
+                        const R rr = RRI ? keep[it] : omb != (R)0 && (part || !RE) ? st.rri[gi] * omb : (R)0;
                         if (part) {
                             st.rri[gi] = rr + val;
                             st.resi[gi] = keep[it] + (rr + val);
@@ -682,12 +705,15 @@ __global__ void __launch_bounds__(LineCfg<R, P, PHYS, DIFF>::NTHR, LineCfg<R, P,
             }
         };
         __syncthreads();
-        if constexpr (!RE) {
+        auto fetch = [&]() {
             fetch_u(b + step, slot == 2 ? 0 : slot + 1);
             fetch_idx(b + 2 * step, slot == 0 ? 2 : slot - 1);
-        }
+        };
+        if constexpr (!RE && !C::TIGHT) fetch();
+        load_rr();
         esums((R)1, (R)0);
         __syncthreads();
+        if constexpr (C::TIGHT) fetch();
         scatter(0);
         if constexpr (RE) {
             xsums([&](int i, R (&fr)[NV], R (&fs)[NV]) {

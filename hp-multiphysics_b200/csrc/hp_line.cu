@@ -71,12 +71,12 @@ struct Impl {
     }
     template <bool DIFF>
     static cudaError_t smem_attr() {
-        using C = LineCfg<R, P, PHYS, DIFF>;
-        cudaError_t e = cudaFuncSetAttribute(k_rsdl_line<R, P, PHYS, DIFF, true>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+        const cudaError_t e = cudaFuncSetAttribute(k_rsdl_line<R, P, PHYS, DIFF, true>,
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   LineCfg<R, P, PHYS, DIFF, true>::SMEM);
         if (e != cudaSuccess) return e;
         return cudaFuncSetAttribute(k_rsdl_line<R, P, PHYS, DIFF, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    C::SMEM);
+                                    LineCfg<R, P, PHYS, DIFF, false>::SMEM);
     }
     static cudaError_t set_smem() {
         const cudaError_t e = smem_attr<false>();
@@ -86,7 +86,7 @@ struct Impl {
     }
     template <bool DIFF, bool RE>
     static void go(const void *tab, const void *gtab, const Mesh &m, const State<R> &s, const LinePar &par, int nsm, cudaStream_t st) {
-        using C = LineCfg<R, P, PHYS, DIFF>;
+        using C = LineCfg<R, P, PHYS, DIFF, RE>;
         const int nb = (m.ntri + 31) / 32;
         k_rsdl_line<R, P, PHYS, DIFF, RE><<<std::min(nb, nsm * C::MINB), C::NTHR, C::SMEM, st>>>(
             *static_cast<const LineTab<R, P> *>(tab), static_cast<const DevTables<R, P> *>(gtab), m, s, par);
