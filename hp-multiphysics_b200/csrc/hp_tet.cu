@@ -12,9 +12,9 @@
 // face and interior sections back to back, each [entity][mode][4 variables]; the
 // dense operators (G^3 x T each) are stored in DMMA fragment order, read through the
 // read-only path and stay in L1 / L2. One warp per pair of tetrahedra: the
-// projections and integrations run on the FP64 tensor cores, lanes own (tetrahedron,
-// point) pairs for the pointwise fluxes, and the per-point arrays live in the warp's
-// shared-memory slice. Boundary faces with a flux take one warp each.
+// projections and integrations run on the FP64 tensor cores, lanes own lines of points
+// for the pointwise fluxes, and the per-point arrays live in the warp's shared-memory
+// slice. Boundary faces with a flux take one warp each.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -172,36 +172,61 @@ __device__ __forceinline__ void tet_gather_kinds(const TetMeshD &mesh, const Tet
     }
 }
 
+template <int BYTES>
+__device__ __forceinline__ void cp_async(void *dst, const void *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
+                 "n"(BYTES));
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // tet_hp::rsdl element loop (res: imaginary terms, res_r: beta-scaled real terms) on the
-// FP64 tensor cores (DMMA, mma.m8n8k4.f64): one warp takes two tetrahedra, so the 8 rows of an A fragment are (tetrahedron, variable) pairs.
+// FP64 tensor cores (DMMA, mma.m8n8k4.f64): one warp takes two tetrahedra, so the 8 rows of an A
+// fragment are (tetrahedron, variable) pairs.
 //   projection:  C[8 x Q] = U[8 x T] * Op^T[T x Q]   for Op = F, DX, DY, DZ
 //   intgrtrst:   C[8 x T] = Flux[8 x 3Q] * WD[3Q x T] (WD = w * (DX; DY; DZ))
 // The B operands are constant: the host stores them in fragment order (one 8-byte
 // coalesced load per lane per MMA). The pointwise fluxes, the strong residual and
-// the SUPG terms stay scalar, lanes owning (tetrahedron, point) pairs.
-template <int P>
+// the SUPG terms stay scalar. The convective fluxes are
+// never stored for the integration: its A fragments are formed from the state at the points.
+//
+// What bounds it: the FP64 pipe (DMMA and DFMA share it) and the warps that fit it, so that the
+// gather, the scatter and the scalar phases of some run under the MMAs of others. One persistent CTA
+// an SM; the indices, modes and coordinates of a warp's next pairs come by cp.async meanwhile
+// (waiting for two dependent loads per kind of mode was 45 % of a stage without the real part);
+// where a mode lies and its sign are looked up (TetLoc), not worked out per value; the phases
+// between the MMAs give a lane a line along x of its own tetrahedron, whose geometry it holds and
+// whose x sums take each value once. Before: two warps a CTA, 8 warps an SM, the convective fluxes
+// in shared memory. 197k tetrahedra, p = 3, full residual 1760 -> 1230 us, without the real part
+// 1100 -> 441; p = 2 763 -> 540 and 436 -> 182; p = 1 219 -> 169 and 124 -> 71; p = 4 (25k) 1221 ->
+// 640 and 585 -> 214; the p = 3 Jacobian diagonal 137 -> 104 ms. The derivatives stay modal: taken
+// from the point values by the 1D operators they would save 120 of 448 MMAs, but their error is
+// 1.6e-15 instead of 4e-17 (the collapsed coordinates amplify it).
+template <int P, bool RE>
 struct TetMma {
     using C = TetCfg<P>;
     static constexpr int KS = (C::T + 3) / 4;        // projection k-steps
     static constexpr int NT = (C::Q + 7) / 8;        // projection n-tiles
-    static constexpr int KS2 = (3 * C::Q + 3) / 4;   // intgrtrst k-steps
+    static constexpr int QK = (C::Q + 3) / 4;        // intgrtrst: point quads, a k-step per component of each
     static constexpr int NT2 = (C::T + 7) / 8;       // intgrtrst n-tiles
-    static constexpr int WPC = 2;
     // strides padded to 4 (mod 16) doubles: the 4 rows (variables) a half-warp reads
     // in one fragment load fall on distinct shared-memory banks
     static constexpr int pad4(int x) { return x + ((4 - x % 16) + 16) % 16; }
-    static constexpr int QP = pad4(C::Q);       // u [NV][QP]
-    static constexpr int VS = pad4(3 * C::Q);   // fim / fre [NV][VS], component c at c * Q
-    // per tetrahedron: uht [NV][T], u [NV][QP], fim [NV][VS], fre [NV][VS]
-    // per tetrahedron: u [3][QP] (u, v, w), fim [NV][VS], fre [NV][VS]; the gathered modes
-    // uht [NV][T] and then the pressure at the points share fre's variable-3 slot, which
-    // holds nothing else until the SUPG phase (uht is read into registers before the
-    // projection stores anything; the pressure values are last read by the pointwise phase)
-    static constexpr int S_EL = 3 * QP + 2 * NV * VS;
-    static_assert(NV * C::T <= VS && C::Q <= VS, "uht / pressure must fit fre's variable-3 slot");
+    static constexpr int QP = pad4(C::Q);       // u, v, w, p at the points [NV][QP]
+    static constexpr int VS = pad4(3 * C::Q);   // fluxes [NV][VS], component c at c * Q
+    // a warp's area: gathered modes [2][NV T], vertex coordinates and tau [2][14], both of the next
+    // pair from the moment this pair's are in registers; u, v, w, p [2][NV][QP]; total fluxes, then
+    // the real ones [2][NV][VS]; indices
+    // of three pairs [3][2][25]
+    static constexpr int U = 0, XY = U + 2 * NV * C::T, UQ = XY + 28, FR = UQ + 2 * NV * QP,
+                         IDX = FR + (RE ? 2 * NV * VS : 0), S_WARP = IDX + 76;
+    static_assert(UQ % 2 == 0 && FR % 2 == 0 && S_WARP % 2 == 0, "pairs of doubles are stored at once");
     static constexpr int NG = NT < 8 ? NT : 8;  // projection n-tiles accumulated together
-    static constexpr int S_WARP = 2 * S_EL;
-    static constexpr size_t PROJ_LEN = (size_t)4 * NT * KS * 32, INT_LEN = (size_t)NT2 * KS2 * 32;
+    static constexpr size_t PROJ_LEN = (size_t)4 * NT * KS * 32, INT_LEN = (size_t)NT2 * QK * 3 * 32;
+    static constexpr int fit = (227 * 1024 / 8) / S_WARP;  // warps an SM, one CTA
+    // as many as fit (12 at p = 3 with the real part: 1640, 1460, 1230 us with 10, 11, 12 at 197k
+    // tetrahedra), up to 16: without the real part 20 are 444 against 441 us at p = 3, 301 against 214
+    // at p = 4 (25k), 16 with it 540 against 556 with 12 at p = 2
+    static constexpr int WPC = fit < 16 ? fit : 16;
     static constexpr size_t SMEM = (size_t)S_WARP * WPC * sizeof(double);
 };
 
@@ -211,120 +236,233 @@ __device__ __forceinline__ void dmma(double &c0, double &c1, double a, double b)
                  : "d"(a), "d"(b));
 }
 
+// Where local mode m of a tetrahedron lies (gtol.cpp:16-82): value n at I[ent] * stride + off + n of
+// a field, I the tetrahedron's indices: vertices 0-3, edges 4-9, faces 10-13, edge signs 14-19,
+// face rotations 20-23, 24 the tetrahedron itself; it is negated where sgn * I[sent] < 0.
+struct TetLoc {
+    int ent, stride, sent, sgn;
+    long off;
+};
+template <int P>
+__device__ __forceinline__ TetLoc tet_loc(const TetFields<double> &g, int m) {
+    using C = TetCfg<P>;
+    constexpr int EM = C::EM > 0 ? C::EM : 1, FM = C::FM > 0 ? C::FM : 1, IM = C::IM > 0 ? C::IM : 1;
+    if (m < 4) return TetLoc{m, NV, 0, 1, 0};
+    if (m < 4 + 6 * C::EM) {
+        const int i = (m - 4) / EM, k = (m - 4) - i * EM;
+        return TetLoc{4 + i, EM * NV, k & 1 ? 14 + i : 0, 1, (g.e - g.v) + k * NV};
+    }
+    if (m < C::BM) {
+        const int r = m - 4 - 6 * C::EM, i = r / FM, idx = r - i * FM;
+        const bool odd = (face_mode_row<C::EM>(idx) - 1) & 1;
+        return TetLoc{10 + i, FM * NV, odd ? 20 + i : 0, odd ? -1 : 1, (g.f - g.v) + idx * NV};
+    }
+    return TetLoc{24, IM * NV, 0, 1, (g.i - g.v) + (m - C::BM) * NV};
+}
+
 // MODE 0: tet_hp::rsdl element loop (res, res_r). MODE 1: the stage-0 element residual
 // lf_re + lf_im of every tetrahedron into rbar [ntet][T][NV]. MODE 2: tet_hp::
 // jacobian_diagonal (tet_hp/jacobi.cpp:32-111): one item per (tetrahedron, mode m,
 // variable n) with uht(n)(m) raised by dw; (lf(n)(m) - rbar) / dw is added, without the
-// edge / face sign (its square is 1), to the global diagonal jd.
-template <int P, int MODE>
-__global__ void __launch_bounds__(TetMma<P>::WPC * 32)
+// edge / face sign (its square is 1), to the global diagonal jd. RE: with the real part (beta > 0).
+template <int P, int MODE, bool RE>
+__global__ void __launch_bounds__(TetMma<P, RE>::WPC * 32, 1)
     k_tet_rsdl_mma(const double *__restrict__ projB, const double *__restrict__ intB, TetSmall<double, P> sm,
                    TetMeshD mesh, TetFields<double> ug, TetFields<double> res, TetFields<double> rr,
                    const double *__restrict__ tau, double rho, double mu, double beta, double *rbar,
                    TetFields<double> jd, const float *__restrict__ lsc, float clampv) {
     using C = TetCfg<P>;
-    using M = TetMma<P>;
-    constexpr int G = C::G, Q = C::Q, T = C::T;
+    using M = TetMma<P, RE>;
+    constexpr int G = C::G, Q = C::Q, T = C::T, QP = M::QP, VS = M::VS;
+    constexpr int EM = C::EM, FM = C::FM, IM = C::IM;
+    constexpr int EMD = EM > 0 ? EM : 1, FMD = FM > 0 ? FM : 1, IMD = IM > 0 ? IM : 1;
     constexpr int NJ = NV * T;  // items per tetrahedron in MODE 2
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ double s1d[RE ? 5 * G * G + 2 * G : 1];  // Ay, By, Az, y0, z0, Ax, Bx: read by lines
+    __shared__ TetLoc locs[T];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int grow = lane >> 2, gcol = lane & 3;  // fragment row / column group
-    double *base = reinterpret_cast<double *>(smem_raw) + warp * M::S_WARP;
-    constexpr int QP = M::QP, VS = M::VS;
-    auto UQ = [&](int e) { return base + e * M::S_EL; };
-    auto FIM = [&](int e) { return base + e * M::S_EL + 3 * QP; };
-    auto FRE = [&](int e) { return base + e * M::S_EL + 3 * QP + NV * VS; };
-    auto UHT = [&](int e) { return FRE(e) + 3 * VS; };
-    auto PV = [&](int e) { return FRE(e) + 3 * VS; };
-    const long nitems = MODE == 2 ? (long)mesh.ntet * NJ : (long)mesh.ntet;
-    const long npair = (nitems + 1) / 2;
-    for (long pr = (long)blockIdx.x * M::WPC + warp; pr < npair; pr += (long)gridDim.x * M::WPC) {
-        const long it0 = 2 * pr;
-        const bool has1 = it0 + 1 < nitems;
-        // tetrahedron of item e (a missing second item repeats the first)
-        int te[2];
-        for (int e = 0; e < 2; ++e) {
-            const long it = (e == 1 && has1) ? it0 + 1 : it0;
-            te[e] = MODE == 2 ? (int)(it / NJ) : (int)it;
+    const int gcol = lane & 3, e = lane >> 4, n = (lane >> 2) & 3;  // fragment: row (e, n), column group
+    double *const base = reinterpret_cast<double *>(smem_raw) + warp * M::S_WARP;
+    int *const ring = reinterpret_cast<int *>(base + M::IDX);
+    if constexpr (RE) {
+        for (int k = threadIdx.x; k < G * G; k += blockDim.x) {
+            s1d[k] = (&sm.Ay[0][0])[k];
+            s1d[G * G + k] = (&sm.By[0][0])[k];
+            s1d[2 * G * G + k] = (&sm.Az[0][0])[k];
+            s1d[3 * G * G + 2 * G + k] = (&sm.Ax[0][0])[k];
+            s1d[4 * G * G + 2 * G + k] = (&sm.Bx[0][0])[k];
+            if (k < G) {
+                s1d[3 * G * G + k] = sm.y0[k];
+                s1d[3 * G * G + G + k] = sm.z0[k];
+            }
         }
-        // ---- gather both tetrahedra (a missing second one gets zeros)
-        tet_gather_kinds<double, P, 2>(
-            mesh, ug, lane, [&](int e) { return e ? te[1] : te[0]; }, [&](int e) { return e == 0 || has1; },
-            [&](int e) { return UHT(e); });
-        double dw[2] = {0.0, 0.0};
-        int jm[2] = {0, 0}, jn[2] = {0, 0};
+    }
+    if (threadIdx.x < T) locs[threadIdx.x] = tet_loc<P>(MODE == 2 ? jd : res, threadIdx.x);
+    __syncthreads();
+    // entries past the last point are read as A values against zeros of B
+    for (int k = lane; k < M::IDX - M::UQ; k += 32) base[M::UQ + k] = 0.0;
+    const long nitems = MODE == 2 ? (long)mesh.ntet * NJ : (long)mesh.ntet;
+    const long npair = (nitems + 1) / 2, step = (long)gridDim.x * M::WPC;
+    // tetrahedron of item ee of pair pr (a missing second item repeats the first)
+    auto tet_of = [&](long pr, int ee) {
+        long it = 2 * pr + ee;
+        if (it >= nitems) it = nitems - 1;
+        return MODE == 2 ? (int)(it / NJ) : (int)it;
+    };
+    auto fetch_idx = [&](long pr, int slot) {
+        if (pr >= npair) return;
+        constexpr int LAST = FM > 0 ? 24 : EM > 0 ? 20 : 4;
+#pragma unroll
+        for (int w = lane; w < 50; w += 32) {
+            const int ee = w / 25, r = w - ee * 25, t = tet_of(pr, ee);
+            if (r == 24) ring[slot * 50 + w] = t;
+            if (r >= LAST || (FM == 0 && r >= 10 && r < 14)) continue;
+            const int *src = r < 4    ? mesh.tp + 4 * (size_t)t + r
+                             : r < 10 ? mesh.ts + 6 * (size_t)t + (r - 4)
+                             : r < 14 ? mesh.tt + 4 * (size_t)t + (r - 10)
+                             : r < 20 ? mesh.tsg + 6 * (size_t)t + (r - 14)
+                                      : mesh.trot + 4 * (size_t)t + (r - 20);
+            cp_async<4>(ring + slot * 50 + w, src);
+        }
+    };
+    // modes (ugtouht, without the signs), vertex coordinates and tau of pair pr
+    auto fetch_u = [&](long pr, int slot) {
+        if (pr >= npair) return;
+        const int *I = ring + slot * 50;
+        double *dst = base + M::U;
+        {
+            const int m = (lane >> 2) & 3, nn = lane & 3;
+            cp_async<8>(dst + (e * NV + nn) * T + m, ug.v + (size_t)I[e * 25 + m] * NV + nn);
+        }
+        if constexpr (EM > 0) {
+            constexpr int NED = 2 * 6 * EM * NV;
+#pragma unroll
+            for (int w = lane; w < NED; w += 32) {
+                const int b = w / (EMD * NV), r = w - b * (EMD * NV), ee = b / 6, i = b - ee * 6, k = r / NV, nn = r - k * NV;
+                cp_async<8>(dst + (ee * NV + nn) * T + 4 + i * EMD + k,
+                            ug.e + (size_t)I[ee * 25 + 4 + i] * (EMD * NV) + r);
+            }
+        }
+        if constexpr (FM > 0) {
+            constexpr int NFC = 2 * 4 * FM * NV;
+#pragma unroll
+            for (int w = lane; w < NFC; w += 32) {
+                const int b = w / (FMD * NV), r = w - b * (FMD * NV), ee = b / 4, i = b - ee * 4, k = r / NV, nn = r - k * NV;
+                cp_async<8>(dst + (ee * NV + nn) * T + 4 + 6 * EM + i * FMD + k,
+                            ug.f + (size_t)I[ee * 25 + 10 + i] * (FMD * NV) + r);
+            }
+        }
+        if constexpr (IM > 0) {
+            for (int w = lane; w < 2 * IM * NV; w += 32) {
+                const int ee = w / (IMD * NV), r = w - ee * (IMD * NV), k = r / NV, nn = r - k * NV;
+                cp_async<8>(dst + (ee * NV + nn) * T + C::BM + k, ug.i + (size_t)tet_of(pr, ee) * (IMD * NV) + r);
+            }
+        }
+        if (lane < 28) {
+            const int ee = lane / 14, r = lane - ee * 14;
+            if (r < 12) cp_async<8>(base + M::XY + lane, mesh.pnts + 3 * (size_t)I[ee * 25 + r / 3] + r % 3);
+            else if (RE) cp_async<8>(base + M::XY + lane, tau + 2 * (size_t)tet_of(pr, ee) + (r - 12));
+        }
+    };
+    // consecutive warps take consecutive pairs; where there are fewer pairs than warps, all SMs take some
+    long pr = npair >= step ? (long)blockIdx.x * M::WPC + warp : blockIdx.x + (long)gridDim.x * warp;
+    int slot = 0;
+    fetch_idx(pr, 0);
+    fetch_idx(pr + step, 1);
+    cp_async_wait();
+    __syncwarp();
+    fetch_u(pr, 0);
+    for (; pr < npair; pr += step, slot = slot == 2 ? 0 : slot + 1) {
+        const long it0 = 2 * pr;
+        const bool ok = e == 0 || it0 + 1 < nitems;  // the lane's row belongs to an item
+        const int te = tet_of(pr, e);
+        const int *I = ring + slot * 50 + e * 25;
+        cp_async_wait();
+        __syncwarp();
+        double *const uht = base + M::U + e * (NV * T);
+        double dw = 0.0;
+        int jm = 0, jn = 0;
         if constexpr (MODE == 2) {
-            __syncwarp();
             // dw = 1e-6 sum over the 4 vertex modes of all variables + 1e-10, the same for
             // every variable (jacobi.cpp:63-67)
-            for (int e = 0; e < 2; ++e) {
-                double sdw = 0.0;
-                for (int n = 0; n < NV; ++n)
-                    for (int i = 0; i < 4; ++i) sdw += fabs(UHT(e)[n * T + i]);
-                dw[e] = sdw * 1.0e-6 + 1.0e-10;
-                const long it = (e == 1 && has1) ? it0 + 1 : it0;
-                const int j = (int)(it - (long)te[e] * NJ);
-                jm[e] = j / NV;
-                jn[e] = j - jm[e] * NV;
-            }
-            __syncwarp();
-            if (lane < 2 && (lane == 0 || has1)) UHT(lane)[jn[lane] * T + jm[lane]] += dw[lane];
+            for (int nn = 0; nn < NV; ++nn)
+                for (int i = 0; i < 4; ++i) dw += fabs(uht[nn * T + i]);
+            dw = dw * 1.0e-6 + 1.0e-10;
+            const long it = ok ? it0 + e : it0;
+            const int j = (int)(it - (long)te * NJ);
+            jm = j / NV;
+            jn = j - jm * NV;
         }
-        // geometry of both (the missing one repeats the first)
-        double d[2][3][3], cj[2];
-        for (int e = 0; e < 2; ++e) {
-            const int t = te[e];
-            const int v0 = mesh.tp[4 * t], v1 = mesh.tp[4 * t + 1], v2 = mesh.tp[4 * t + 2], v3 = mesh.tp[4 * t + 3];
-            double ld[3][3];
-            for (int n = 0; n < 3; ++n) {
-                const double c2 = mesh.pnts[3 * v2 + n];
-                ld[n][0] = 0.5 * (mesh.pnts[3 * v3 + n] - c2);
-                ld[n][1] = 0.5 * (mesh.pnts[3 * v1 + n] - c2);
-                ld[n][2] = 0.5 * (mesh.pnts[3 * v0 + n] - c2);
+        // the row's modes, signs applied
+        double a[M::KS];
+#pragma unroll
+        for (int ks = 0; ks < M::KS; ++ks) {
+            const int m = ks * 4 + gcol;
+            a[ks] = 0.0;
+            if (m < T) {
+                a[ks] = uht[n * T + m];
+                if (locs[m].sgn * I[locs[m].sent] < 0) a[ks] = -a[ks];
+                if constexpr (MODE == 2)
+                    if (m == jm && n == jn) a[ks] += dw;
             }
-            d[e][0][0] = ld[1][1] * ld[2][2] - ld[1][2] * ld[2][1];
-            d[e][0][1] = -ld[0][1] * ld[2][2] + ld[0][2] * ld[2][1];
-            d[e][0][2] = ld[0][1] * ld[1][2] - ld[0][2] * ld[1][1];
-            d[e][1][0] = -ld[1][0] * ld[2][2] + ld[1][2] * ld[2][0];
-            d[e][1][1] = ld[0][0] * ld[2][2] - ld[0][2] * ld[2][0];
-            d[e][1][2] = -ld[0][0] * ld[1][2] + ld[0][2] * ld[1][0];
-            d[e][2][0] = ld[1][0] * ld[2][1] - ld[1][1] * ld[2][0];
-            d[e][2][1] = -ld[0][0] * ld[2][1] + ld[0][1] * ld[2][0];
-            d[e][2][2] = ld[0][0] * ld[1][1] - ld[0][1] * ld[1][0];
-            cj[e] = ld[0][0] * (ld[1][1] * ld[2][2] - ld[1][2] * ld[2][1]) -
-                    ld[0][1] * (ld[1][0] * ld[2][2] - ld[2][0] * ld[1][2]) +
-                    ld[0][2] * (ld[1][0] * ld[2][1] - ld[2][0] * ld[1][1]);
+        }
+        // geometry of the lane's tetrahedron
+        double d[3][3], cj;
+        {
+            const double *xy = base + M::XY + e * 14;
+            double ld[3][3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const double c2 = xy[6 + k];
+                ld[k][0] = 0.5 * (xy[9 + k] - c2);
+                ld[k][1] = 0.5 * (xy[3 + k] - c2);
+                ld[k][2] = 0.5 * (xy[k] - c2);
+            }
+            d[0][0] = ld[1][1] * ld[2][2] - ld[1][2] * ld[2][1];
+            d[0][1] = -ld[0][1] * ld[2][2] + ld[0][2] * ld[2][1];
+            d[0][2] = ld[0][1] * ld[1][2] - ld[0][2] * ld[1][1];
+            d[1][0] = -ld[1][0] * ld[2][2] + ld[1][2] * ld[2][0];
+            d[1][1] = ld[0][0] * ld[2][2] - ld[0][2] * ld[2][0];
+            d[1][2] = -ld[0][0] * ld[1][2] + ld[0][2] * ld[1][0];
+            d[2][0] = ld[1][0] * ld[2][1] - ld[1][1] * ld[2][0];
+            d[2][1] = -ld[0][0] * ld[2][1] + ld[0][1] * ld[2][0];
+            d[2][2] = ld[0][0] * ld[1][1] - ld[0][1] * ld[1][0];
+            cj = ld[0][0] * (ld[1][1] * ld[2][2] - ld[1][2] * ld[2][1]) -
+                 ld[0][1] * (ld[1][0] * ld[2][2] - ld[2][0] * ld[1][2]) +
+                 ld[0][2] * (ld[1][0] * ld[2][1] - ld[2][0] * ld[1][1]);
+        }
+        double tau0 = 0.0, tau3 = 0.0;
+        if constexpr (RE) {
+            tau0 = base[M::XY + e * 14 + 12];
+            tau3 = base[M::XY + e * 14 + 13];
         }
         __syncwarp();
-        // ---- projection on the tensor cores: row (e, n) = (grow >> 2, grow & 3)
-        {
-            const int e = grow >> 2, n = grow & 3;
-            double a[M::KS];
+        fetch_u(pr + step, slot == 2 ? 0 : slot + 1);
+        fetch_idx(pr + 2 * step, slot == 0 ? 2 : slot - 1);
+        // ---- projection: the values and, for the velocity, the derivatives at the points
+#pragma unroll 1
+        for (int op = 0; op < (RE ? 4 : 1); ++op) {
+            double *dst = op == 0 ? base + M::UQ + (e * NV + n) * QP
+                                  : (n < 3 ? base + M::FR + (e * NV + n) * VS + (op - 1) * Q : nullptr);
+#pragma unroll 1
+            for (int nt0 = 0; nt0 < M::NT; nt0 += M::NG) {
+                // NG independent accumulator chains
+                double c[M::NG][2];
 #pragma unroll
-            for (int ks = 0; ks < M::KS; ++ks) {
-                const int m = ks * 4 + gcol;
-                a[ks] = m < T ? UHT(e)[n * T + m] : 0.0;
-            }
-            __syncwarp();  // uht is dead from here: its slot takes the pressure values
-            const bool needd = beta > 0.0;
-            for (int op = 0; op < (needd ? 4 : 1); ++op) {
-                double *dst = op == 0 ? (n < 3 ? UQ(e) + n * QP : PV(e))
-                                      : (n < 3 ? FRE(e) + n * VS + (op - 1) * Q : nullptr);
-                for (int nt0 = 0; nt0 < M::NT; nt0 += M::NG) {
-                    // NG independent accumulator chains
-                    double c[M::NG][2];
+                for (int g = 0; g < M::NG; ++g) c[g][0] = c[g][1] = 0.0;
+                const double *b = projB + ((size_t)(op * M::NT + nt0) * M::KS) * 32 + lane;
 #pragma unroll
-                    for (int g = 0; g < M::NG; ++g) c[g][0] = c[g][1] = 0.0;
-                    const double *b = projB + ((size_t)(op * M::NT + nt0) * M::KS) * 32 + lane;
+                for (int ks = 0; ks < M::KS; ++ks)
 #pragma unroll
-                    for (int ks = 0; ks < M::KS; ++ks)
+                    for (int g = 0; g < M::NG; ++g)
+                        if (nt0 + g < M::NT) dmma(c[g][0], c[g][1], a[ks], __ldg(b + ((size_t)g * M::KS + ks) * 32));
+                if (dst) {
 #pragma unroll
-                        for (int g = 0; g < M::NG; ++g)
-                            if (nt0 + g < M::NT) dmma(c[g][0], c[g][1], a[ks], __ldg(b + ((size_t)g * M::KS + ks) * 32));
-                    if (dst) {
-#pragma unroll
-                        for (int g = 0; g < M::NG; ++g) {
-                            const int q = (nt0 + g) * 8 + gcol * 2;
+                    for (int g = 0; g < M::NG; ++g) {
+                        const int q = (nt0 + g) * 8 + gcol * 2;
+                        if constexpr (Q % 8 == 0) {
+                            *reinterpret_cast<double2 *>(dst + q) = make_double2(c[g][0], c[g][1]);
+                        } else {
                             if (q < Q) dst[q] = c[g][0];
                             if (q + 1 < Q) dst[q + 1] = c[g][1];
                         }
@@ -333,196 +471,191 @@ __global__ void __launch_bounds__(TetMma<P>::WPC * 32)
             }
         }
         __syncwarp();
-        // ---- pointwise fluxes, lanes own (e, q): fim = convective + pressure / continuity;
-        //      fre = viscous flux from the velocity derivatives stored there
-        for (int w = lane; w < 2 * Q; w += 32) {
-            const int e = w / Q, q = w - e * Q;
-            const double *uq = UQ(e);
-            double *fim = FIM(e), *fre = FRE(e);
-            const double uu[4] = {uq[q], uq[QP + q], uq[2 * QP + q], PV(e)[q]};
-            const double fx = rho * uu[0], fy = rho * uu[1], fz = rho * uu[2];
-            double f3[3];
+        if constexpr (RE) {
+            constexpr int GG = G * G;
+            const double *const uq = base + M::UQ + e * NV * QP;
+            double *const fr = base + M::FR + e * NV * VS;
+            const double cjcbi = mu / cj;
+            // the convective and pressure flux of the momentum at a point, f3 the mass flux
+            auto conv = [&](const double (&uu)[4], double (&f3)[3], double (&f)[3][3]) {
+                const double fx = rho * uu[0], fy = rho * uu[1], fz = rho * uu[2];
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                f3[c] = d[e][c][0] * fx + d[e][c][1] * fy + d[e][c][2] * fz;
-                fim[3 * VS + c * Q + q] = f3[c];
+                for (int c = 0; c < 3; ++c) {
+                    f3[c] = d[c][0] * fx + d[c][1] * fy + d[c][2] * fz;
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) f[k][c] = uu[k] * f3[c] + d[c][k] * uu[3];
+                }
+            };
+            constexpr int NL = (GG + 15) / 16;  // x lines of a lane; at p = 1 there are lanes for each half of one
+            constexpr int SP = 2 * GG <= 16 ? 2 : 1, NI = G / SP;
+            const int l16 = lane & 15, i0 = SP > 1 && l16 >= GG ? NI : 0, r0 = SP > 1 && l16 >= GG ? l16 - GG : l16;
+            double rsd[NL][NI][NV];
+            // ---- total fluxes, in the place of the velocity derivatives; lanes own lines along x
+#pragma unroll
+            for (int it = 0; it < NL; ++it) {
+                const int r = r0 + 16 * it;
+                if (SP > 1 ? l16 >= SP * GG : r >= GG) break;
+#pragma unroll
+                for (int ii = 0; ii < NI; ++ii) {
+                    const int q = (i0 + ii) * GG + r;
+                    const double uu[4] = {uq[q], uq[QP + q], uq[2 * QP + q], uq[3 * QP + q]};
+                    double f3[3], f[3][3], du[3][3], h[3][3];
+                    conv(uu, f3, f);
+#pragma unroll
+                    for (int k = 0; k < 3; ++k)
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) du[k][c] = fr[k * VS + c * Q + q];
+                    // sum_ee (d_c . d_ee) du[k][ee] = d_c . h[k], and its transpose
+#pragma unroll
+                    for (int b = 0; b < 3; ++b)
+#pragma unroll
+                        for (int k = 0; k < 3; ++k) h[b][k] = d[0][k] * du[b][0] + d[1][k] * du[b][1] + d[2][k] * du[b][2];
+#pragma unroll
+                    for (int k = 0; k < 3; ++k)
+#pragma unroll
+                        for (int c = 0; c < 3; ++c)
+                            fr[k * VS + c * Q + q] =
+                                f[k][c] - cjcbi * (d[c][0] * (h[k][0] + h[0][k]) + d[c][1] * (h[k][1] + h[1][k]) +
+                                                   d[c][2] * (h[k][2] + h[2][k]));
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) fr[3 * VS + c * Q + q] = f3[c];
+                }
             }
+            __syncwarp();
+            // ---- strong residual at the lane's points
 #pragma unroll
-            for (int n = 0; n < 3; ++n)
+            for (int it = 0; it < NL; ++it) {
+                const int r = r0 + 16 * it;
+                if (SP > 1 ? l16 >= SP * GG : r >= GG) break;
+                const int j = r / G, kk = r - j * G;
+                const double zz = s1d[3 * GG + G + kk], yz = s1d[3 * GG + j] * zz;
 #pragma unroll
-                for (int c = 0; c < 3; ++c) fim[n * VS + c * Q + q] = uu[n] * f3[c] + d[e][c][n] * uu[3];
-            if (beta > 0.0) {
-                double du[3][3];
+                for (int i = 0; i < NI; ++i)
 #pragma unroll
-                for (int n = 0; n < 3; ++n)
+                    for (int m = 0; m < NV; ++m) rsd[it][i][m] = 0.0;
 #pragma unroll
-                    for (int c = 0; c < 3; ++c) du[n][c] = fre[n * VS + c * Q + q];
-                const double cjcbi = mu / cj[e];
-                double h[3][3];
+                for (int l = 0; l < G; ++l)
 #pragma unroll
-                for (int b = 0; b < 3; ++b)
+                    for (int m = 0; m < NV; ++m) {
+                        const double *fx = fr + m * VS + l * GG + r;
+                        const double f0 = fx[0], f12 = fx[Q] + fx[2 * Q];
 #pragma unroll
-                    for (int a = 0; a < 3; ++a)
-                        h[b][a] = d[e][0][a] * du[b][0] + d[e][1][a] * du[b][1] + d[e][2][a] * du[b][2];
-#pragma unroll
-                for (int a = 0; a < 3; ++a)
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        double s = 0.0;
-#pragma unroll
-                        for (int ee = 0; ee < 3; ++ee) {
-                            const double gce = d[e][c][0] * d[e][ee][0] + d[e][c][1] * d[e][ee][1] + d[e][c][2] * d[e][ee][2];
-                            s += gce * du[a][ee];
-                        }
-                        s += d[e][c][0] * h[0][a] + d[e][c][1] * h[1][a] + d[e][c][2] * h[2][a];
-                        fre[a * VS + c * Q + q] = -cjcbi * s;
+                        for (int i = 0; i < NI; ++i)
+                            if constexpr (SP == 1) rsd[it][i][m] += sm.Ax[i][l] * f0 + sm.Bx[i][l] * f12;
+                            else rsd[it][i][m] += s1d[3 * GG + 2 * G + (i0 + i) * G + l] * f0 + s1d[4 * GG + 2 * G + (i0 + i) * G + l] * f12;
                     }
-            }
-        }
-        __syncwarp();
-        if (beta > 0.0) {
-            // ---- strong residual at the owned points
-            constexpr int NW = (2 * Q + 31) / 32;
-            double rsd[NW][NV];
 #pragma unroll
-            for (int k = 0; k < NW; ++k) {
-                const int w = lane + 32 * k;
-                if (w >= 2 * Q) break;
-                const int e = w / Q, q = w - e * Q;
-                const int i = q / (G * G), j = (q / G) % G, kk = q % G;
-                const double yz = sm.y0[j] * sm.z0[kk], zz = sm.z0[kk];
-                const double *fim = FIM(e), *fre = FRE(e);
+                for (int ii = 0; ii < NI; ++ii) {
+                    const int i = i0 + ii;
+                    double ay[NV], az[NV];
 #pragma unroll
-                for (int n = 0; n < NV; ++n) {
-                    auto fl = [&](int c, int i2, int j2, int k2) -> double {
-                        const int q2 = (i2 * G + j2) * G + k2;
-                        return n < 3 ? fim[n * VS + c * Q + q2] + fre[n * VS + c * Q + q2] : fim[3 * VS + c * Q + q2];
-                    };
-                    double ax = 0, bxs = 0, bxt = 0, ays = 0, byt = 0, azt = 0;
+                    for (int m = 0; m < NV; ++m) ay[m] = az[m] = 0.0;
 #pragma unroll
                     for (int l = 0; l < G; ++l) {
-                        ax += sm.Ax[i][l] * fl(0, l, j, kk);
-                        bxs += sm.Bx[i][l] * fl(1, l, j, kk);
-                        bxt += sm.Bx[i][l] * fl(2, l, j, kk);
-                        ays += sm.Ay[j][l] * fl(1, i, l, kk);
-                        byt += sm.By[j][l] * fl(2, i, l, kk);
-                        azt += sm.Az[kk][l] * fl(2, i, j, l);
+                        const double cay = s1d[j * G + l], cby = s1d[GG + j * G + l], caz = s1d[2 * GG + kk * G + l];
+                        const double *fy = fr + (i * G + l) * G + kk, *fz = fr + (i * G + j) * G + l;
+#pragma unroll
+                        for (int m = 0; m < NV; ++m) {
+                            ay[m] += cay * fy[m * VS + Q] + cby * fy[m * VS + 2 * Q];
+                            az[m] += caz * fz[m * VS + 2 * Q];
+                        }
                     }
-                    rsd[k][n] = yz * ax + (yz * bxs + zz * ays) + (yz * bxt + zz * byt + azt);
+#pragma unroll
+                    for (int m = 0; m < NV; ++m) rsd[it][ii][m] = yz * rsd[it][ii][m] + zz * ay[m] + az[m];
                 }
             }
             __syncwarp();
-            // ---- SUPG terms into fre (viscous + SUPG; variable 3: the continuity SUPG term)
+            // ---- viscous + SUPG fluxes (variable 3: the continuity SUPG term)
 #pragma unroll
-            for (int k = 0; k < NW; ++k) {
-                const int w = lane + 32 * k;
-                if (w >= 2 * Q) break;
-                const int e = w / Q, q = w - e * Q;
-                const int t = te[e];
-                const double tau0 = tau[2 * t], tau3 = tau[2 * t + 1];
-                double *fre = FRE(e);
-                const double *uq = UQ(e);
-                double tr[NV], uu[3];
+            for (int it = 0; it < NL; ++it) {
+                const int r = r0 + 16 * it;
+                if (SP > 1 ? l16 >= SP * GG : r >= GG) break;
 #pragma unroll
-                for (int n = 0; n < 3; ++n) {
-                    tr[n] = tau0 * rsd[k][n];
-                    uu[n] = uq[n * QP + q];
-                }
-                tr[3] = tau3 * rsd[k][3];
-#pragma unroll
-                for (int a = 0; a < 3; ++a)
+                for (int ii = 0; ii < NI; ++ii) {
+                    const int q = (i0 + ii) * GG + r;
+                    const double uu[4] = {uq[q], uq[QP + q], uq[2 * QP + q], uq[3 * QP + q]};
+                    const double tr[4] = {tau0 * rsd[it][ii][0], tau0 * rsd[it][ii][1], tau0 * rsd[it][ii][2], tau3 * rsd[it][ii][3]};
+                    double f3[3], f[3][3];
+                    conv(uu, f3, f);
 #pragma unroll
                     for (int c = 0; c < 3; ++c) {
-                        double s2 = d[e][c][a] * (2.0 * uu[a]);
+                        const double du = d[c][0] * uu[0] + d[c][1] * uu[1] + d[c][2] * uu[2];
+                        const double dt = d[c][0] * tr[0] + d[c][1] * tr[1] + d[c][2] * tr[2];
 #pragma unroll
-                        for (int b = 0; b < 3; ++b)
-                            if (b != a) s2 += d[e][c][b] * uu[b];
-                        double r = s2 * tr[a];
-#pragma unroll
-                        for (int b = 0; b < 3; ++b)
-                            if (b != a) r += d[e][c][b] * uu[a] * tr[b];
-                        r += d[e][c][a] * tr[3];
-                        fre[a * VS + c * Q + q] -= r;
+                        for (int m = 0; m < 3; ++m)
+                            fr[m * VS + c * Q + q] = (fr[m * VS + c * Q + q] - f[m][c]) - (du * tr[m] + dt * uu[m] + d[c][m] * tr[3]);
+                        fr[3 * VS + c * Q + q] = -dt;
                     }
-#pragma unroll
-                for (int c = 0; c < 3; ++c)
-                    fre[3 * VS + c * Q + q] = -d[e][c][0] * tr[0] - d[e][c][1] * tr[1] - d[e][c][2] * tr[2];
+                }
             }
             __syncwarp();
         }
-        // ---- intgrtrst on the tensor cores (imaginary into res, real * beta into res_r); with a
-        //      real part both share each operator fragment load
+        // ---- intgrtrst (imaginary into res, real * beta into res_r); both parts share each
+        //      operator fragment load
+        double ci[M::NT2][2], cr[M::NT2][2];
+#pragma unroll
+        for (int nt = 0; nt < M::NT2; ++nt) ci[nt][0] = ci[nt][1] = cr[nt][0] = cr[nt][1] = 0.0;
         {
-            const int e = grow >> 2, n = grow & 3;
-            const bool two = beta > 0.0;
-            double tot[M::NT2][2];
-            const double *fai = FIM(e) + n * VS, *far = FRE(e) + n * VS;  // [3][Q] = k order
-            double ci[M::NT2][2], cr[M::NT2][2];
+            const double *uq = base + M::UQ + e * NV * QP + gcol, *far = base + M::FR + (e * NV + n) * VS + gcol;
+            const double *bq = intB + lane, *ur = base + M::UQ + (e * NV + n) * QP + gcol;
+            double dn[3];
 #pragma unroll
-            for (int nt = 0; nt < M::NT2; ++nt) ci[nt][0] = ci[nt][1] = cr[nt][0] = cr[nt][1] = 0.0;
+            for (int c = 0; c < 3; ++c) dn[c] = n == 0 ? d[c][0] : n == 1 ? d[c][1] : n == 2 ? d[c][2] : 0.0;
 #pragma unroll 2
-            for (int ks = 0; ks < M::KS2; ++ks) {
-                const int k = ks * 4 + gcol;
-                const double ai = k < 3 * Q ? fai[k] : 0.0;
-                const double ar = (two && k < 3 * Q) ? far[k] : 0.0;
+            for (int qq = 0; qq < M::QK; ++qq) {
+                const double u0 = uq[qq * 4], u1 = uq[QP + qq * 4], u2 = uq[2 * QP + qq * 4], p = uq[3 * QP + qq * 4];
+                const double un = n < 3 ? rho * ur[qq * 4] : rho;
 #pragma unroll
-                for (int nt = 0; nt < M::NT2; ++nt) {
-                    const double bf = __ldg(intB + ((size_t)nt * M::KS2 + ks) * 32 + lane);
-                    dmma(ci[nt][0], ci[nt][1], ai, bf);
-                    if (two) dmma(cr[nt][0], cr[nt][1], ar, bf);
-                }
-            }
-            const bool ok = (e == 0 || has1);
+                for (int c = 0; c < 3; ++c) {
+                    const double ai = un * (d[c][0] * u0 + d[c][1] * u1 + d[c][2] * u2) + dn[c] * p;
+                    const double ar = RE ? far[c * Q + qq * 4] : 0.0;
 #pragma unroll
-            for (int nt = 0; nt < M::NT2; ++nt)
-#pragma unroll
-                for (int h2 = 0; h2 < 2; ++h2) {
-                    // row grow = (e, n); columns m = nt*8 + gcol*2 + {0, 1}
-                    const int m = nt * 8 + gcol * 2 + h2;
-                    tot[nt][h2] = 0.0;
-                    if (!ok || m >= T) continue;
-                    const double vi = -ci[nt][h2], vr = -cr[nt][h2];
-                    if constexpr (MODE != 0) {
-                        tot[nt][h2] = two ? vi + beta * vr : vi;
-                    } else {
-                        double sg;
-                        double *dst = mode_slot<double, P>(mesh, res, te[e], m, n, sg);
-                        if (m < C::BM) atomicAdd(dst, sg * vi);
-                        else *dst = vi;
-                        if (two) {
-                            double *dr = mode_slot<double, P>(mesh, rr, te[e], m, n, sg);
-                            if (m < C::BM) atomicAdd(dr, beta * sg * vr);
-                            else *dr += beta * vr;
-                        }
+                    for (int nt = 0; nt < M::NT2; ++nt) {
+                        const double bf = __ldg(bq + ((size_t)(nt * M::QK + qq) * 3 + c) * 32);
+                        dmma(ci[nt][0], ci[nt][1], ai, bf);
+                        if (RE) dmma(cr[nt][0], cr[nt][1], ar, bf);
                     }
                 }
-            if constexpr (MODE != 0) {
-                const bool ok = (e == 0 || has1);
-#pragma unroll
-                for (int nt = 0; nt < M::NT2; ++nt)
-#pragma unroll
-                    for (int h2 = 0; h2 < 2; ++h2) {
-                        const int m = nt * 8 + gcol * 2 + h2;
-                        if (!ok || m >= T) continue;
-                        const size_t rb = ((size_t)te[e] * T + m) * NV + n;
-                        if constexpr (MODE == 1) {
-                            rbar[rb] = tot[nt][h2];
-                        } else {
-                            if (m != jm[e] || n != jn[e]) continue;
-                            double sg;
-                            double *dst = mode_slot<double, P>(mesh, jd, te[e], m, n, sg);
-                            double sc = 1.0;  // learned per-tetrahedron scale of its contribution
-                            if (lsc) {
-                                float c = lsc[te[e]];
-                                c = c > clampv ? clampv : (c < -clampv ? -clampv : c);
-                                if (!(c == c)) c = 0.f;
-                                sc = exp((double)c);
-                            }
-                            atomicAdd(dst, sc * (tot[nt][h2] - rbar[rb]) / dw[e]);
-                        }
-                    }
             }
         }
+#pragma unroll
+        for (int nt = 0; nt < M::NT2; ++nt)
+#pragma unroll
+            for (int h2 = 0; h2 < 2; ++h2) {
+                // row (e, n); columns m = nt*8 + gcol*2 + {0, 1}
+                const int m = nt * 8 + gcol * 2 + h2;
+                if (!ok || m >= T) continue;
+                const double vi = -ci[nt][h2], vr = -cr[nt][h2];
+                if constexpr (MODE == 0) {
+                    // (res and res_r have the same layout)
+                    const TetLoc lc = locs[m];
+                    const bool neg = lc.sgn * I[lc.sent] < 0;
+                    const size_t at = (size_t)I[lc.ent] * lc.stride + lc.off + n;
+                    if (m < C::BM) atomicAdd(res.v + at, neg ? -vi : vi);
+                    else res.v[at] = vi;
+                    if (RE) {
+                        if (m < C::BM) atomicAdd(rr.v + at, beta * (neg ? -vr : vr));
+                        else rr.v[at] += beta * vr;
+                    }
+                } else {
+                    const double tot = RE ? vi + beta * vr : vi;
+                    const size_t rb = ((size_t)te * T + m) * NV + n;
+                    if constexpr (MODE == 1) {
+                        rbar[rb] = tot;
+                    } else {
+                        if (m != jm || n != jn) continue;
+                        double sc = 1.0;  // learned per-tetrahedron scale of its contribution
+                        if (lsc) {
+                            float c = lsc[te];
+                            c = c > clampv ? clampv : (c < -clampv ? -clampv : c);
+                            if (!(c == c)) c = 0.f;
+                            sc = exp((double)c);
+                        }
+                        atomicAdd(jd.v + (size_t)I[locs[m].ent] * locs[m].stride + locs[m].off + n,
+                                  sc * (tot - rbar[rb]) / dw);
+                    }
+                }
+            }
         __syncwarp();
     }
 }
@@ -1202,12 +1335,12 @@ int talloc(hp_tet_ctx *c, void **p, size_t bytes) {
 }
 
 // DMMA B fragments (lane = 4 * group + column): projection B[k = mode][n = point]
-// = Op(q, m) at [op][nt][ks][lane]; intgrtrst B[k = (c, q)][n = mode] = w(q) Dc(q, m)
-// at [nt][ks][lane]; zero beyond T, Q, 3Q.
+// = Op(q, m) at [op][nt][ks][lane]; intgrtrst B[k = q][n = mode] = w(q) Dc(q, m)
+// at [nt][point quad][c][lane]; zero beyond T, Q.
 template <int P>
 void tet_fragments(const hp_tet_tables &b, std::vector<double> &proj, std::vector<double> &intg) {
     using C = TetCfg<P>;
-    using M = TetMma<P>;
+    using M = TetMma<P, true>;
     proj.assign(M::PROJ_LEN, 0.0);
     intg.assign(M::INT_LEN, 0.0);
     const double(*ops[4])[HP_TET_MAXT] = {b.F, b.DX, b.DY, b.DZ};
@@ -1220,26 +1353,42 @@ void tet_fragments(const hp_tet_tables &b, std::vector<double> &proj, std::vecto
                         proj[(((size_t)op * M::NT + nt) * M::KS + ks) * 32 + lane] = ops[op][q][m];
                 }
     for (int nt = 0; nt < M::NT2; ++nt)
-        for (int ks = 0; ks < M::KS2; ++ks)
+        for (int ks = 0; ks < 3 * M::QK; ++ks)
             for (int lane = 0; lane < 32; ++lane) {
-                const int k = ks * 4 + (lane & 3), m = nt * 8 + (lane >> 2);
-                if (k >= 3 * C::Q || m >= C::T) continue;
-                const int c = k / C::Q, q = k - c * C::Q;
-                intg[((size_t)nt * M::KS2 + ks) * 32 + lane] = b.w[q] * ops[1 + c][q][m];
+                const int c = ks % 3, q = ks / 3 * 4 + (lane & 3), m = nt * 8 + (lane >> 2);
+                if (q >= C::Q || m >= C::T) continue;
+                intg[((size_t)nt * 3 * M::QK + ks) * 32 + lane] = b.w[q] * ops[1 + c][q][m];
             }
 }
 
 // dynamic shared memory above 48 KB for every instantiation, once per process
+template <int P, int MODE, bool RE>
+cudaError_t rsdl_attr() {
+    return cudaFuncSetAttribute(k_tet_rsdl_mma<P, MODE, RE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)TetMma<P, RE>::SMEM);
+}
 template <int P>
 int ensure_attrs() {
-    using M = TetMma<P>;
     static bool done = false;
     if (done) return HP_OK;
-    TCK(cudaFuncSetAttribute(k_tet_rsdl_mma<P, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)M::SMEM));
-    TCK(cudaFuncSetAttribute(k_tet_rsdl_mma<P, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)M::SMEM));
-    TCK(cudaFuncSetAttribute(k_tet_rsdl_mma<P, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)M::SMEM));
+    TCK((rsdl_attr<P, 0, false>()));
+    TCK((rsdl_attr<P, 0, true>()));
+    TCK((rsdl_attr<P, 1, false>()));
+    TCK((rsdl_attr<P, 1, true>()));
+    TCK((rsdl_attr<P, 2, false>()));
+    TCK((rsdl_attr<P, 2, true>()));
     done = true;
     return HP_OK;
+}
+
+// one launch over nitems items, one CTA an SM
+template <int P, int MODE, bool RE>
+void go_rsdl(hp_tet_ctx *c, const TetSmall<double, P> &sm, double beta, const float *lsc, float clampv) {
+    using M = TetMma<P, RE>;
+    const long nitems = (long)c->mesh.ntet * (MODE == 2 ? NV * TetCfg<P>::T : 1), npair = (nitems + 1) / 2;
+    k_tet_rsdl_mma<P, MODE, RE><<<(int)std::min<long>(npair, c->nsm), M::WPC * 32, M::SMEM, c->stream>>>(
+        c->projB, c->intB, sm, c->mesh, c->fields(c->U), c->fields(c->RES), c->fields(c->RR), c->tau, c->ph.rho,
+        c->ph.mu, beta, MODE == 0 ? nullptr : c->rbar, MODE == 0 ? TetFields<double>{} : c->fields(c->JD), lsc, clampv);
 }
 
 template <int P>
@@ -1264,14 +1413,9 @@ int launch_rsdl(hp_tet_ctx *c, int stage) {
     if (c->faces.n > 0)
         k_tet_face_flux<P><<<std::min(nblk(c->faces.n, 4), c->nsm * 16), 128, 0, c->stream>>>(
             c->faces, c->ftab, c->mesh, c->fields(c->U), c->fields(c->RES), c->ph.rho);
-    using M = TetMma<P>;
-    const size_t smem2 = (size_t)M::S_WARP * M::WPC * sizeof(double);
     if (int r = ensure_attrs<P>()) return r;
-    const long npair = ((long)c->mesh.ntet + 1) / 2;
-    int blocks = std::min(nblk(npair, M::WPC), c->nsm * 32);
-    k_tet_rsdl_mma<P, 0><<<blocks, M::WPC * 32, smem2, c->stream>>>(
-        c->projB, c->intB, sm, c->mesh, c->fields(c->U), c->fields(c->RES), c->fields(c->RR), c->tau, c->ph.rho,
-        c->ph.mu, beta, nullptr, TetFields<double>{}, nullptr, 0.f);
+    if (beta > 0.0) go_rsdl<P, 0, true>(c, sm, beta, nullptr, 0.f);
+    else go_rsdl<P, 0, false>(c, sm, beta, nullptr, 0.f);
     k_tet_fold<double><<<std::min(nblk((long)c->ltot, 256), c->nsm * 8), 256, 0, c->stream>>>((long)c->ltot, c->RES,
                                                                                             c->RR);
     if (c->fine) {
@@ -1285,8 +1429,6 @@ int launch_rsdl(hp_tet_ctx *c, int stage) {
 
 template <int P>
 int launch_jacdiag(hp_tet_ctx *c) {
-    using C = TetCfg<P>;
-    using M = TetMma<P>;
     int r = ensure_attrs<P>();
     if (r) return r;
     TetSmall<double, P> sm;
@@ -1303,14 +1445,12 @@ int launch_jacdiag(hp_tet_ctx *c) {
         sm.z0[i] = t.z0[i];
     }
     const double beta0 = c->ph.beta[0];
-    const long n1 = ((long)c->mesh.ntet + 1) / 2, n2 = ((long)c->mesh.ntet * NV * C::T + 1) / 2;
-    k_tet_rsdl_mma<P, 1><<<std::min(nblk(n1, M::WPC), c->nsm * 32), M::WPC * 32, M::SMEM, c->stream>>>(
-        c->projB, c->intB, sm, c->mesh, c->fields(c->U), c->fields(c->RES), c->fields(c->RR), c->tau, c->ph.rho,
-        c->ph.mu, beta0, c->rbar, c->fields(c->JD), nullptr, 0.f);
+    const bool re = beta0 > 0.0;
+    if (re) go_rsdl<P, 1, true>(c, sm, beta0, nullptr, 0.f);
+    else go_rsdl<P, 1, false>(c, sm, beta0, nullptr, 0.f);
     TCK(cudaMemsetAsync(c->JD, 0, 8 * c->ltot, c->stream));
-    k_tet_rsdl_mma<P, 2><<<std::min(nblk(n2, M::WPC), c->nsm * 32), M::WPC * 32, M::SMEM, c->stream>>>(
-        c->projB, c->intB, sm, c->mesh, c->fields(c->U), c->fields(c->RES), c->fields(c->RR), c->tau, c->ph.rho,
-        c->ph.mu, beta0, c->rbar, c->fields(c->JD), c->lsc, c->lsc_clamp);
+    if (re) go_rsdl<P, 2, true>(c, sm, beta0, c->lsc, c->lsc_clamp);
+    else go_rsdl<P, 2, false>(c, sm, beta0, c->lsc, c->lsc_clamp);
     TCK(cudaGetLastError());
     return HP_OK;
 }

@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 from hpb.tet import TetGPU, TetProblem
-from hpb.tetmesh import cube_tets
+from hpb.tetmesh import TetMesh, cube_tets
 from oracle.oracle import OracleTet
 
 pytestmark = pytest.mark.gpu
@@ -258,3 +258,26 @@ def test_tet_exact_steady_solutions_have_zero_residual_on_gpu(p, case, mesh):
     rng = np.random.default_rng(3)
     pert = [a + 1e-3 * rng.uniform(-1, 1, a.shape) for a in pr.state]
     assert free_max(pr.state) < 1e-9 * free_max(pert)
+
+
+@pytest.mark.parametrize("p,ntet", [(1, 1), (2, 1), (3, 1), (4, 1), (1, 6), (2, 5), (3, 2), (3, 3), (4, 3), (3, 297),
+                                    (1, 4737), (2, 4735), (3, 3551), (3, 3553), (4, 1777)])
+def test_tet_rsdl_at_the_edges_of_its_work_split(p, ntet):
+    """k_tet_rsdl_mma takes tetrahedra in pairs, one CTA an SM: a missing second one, fewer pairs than
+    SMs, fewer and a few more than the resident warps (148 SMs of 16 warps, 12 at p = 3, 6 at p = 4).
+    The Jacobian diagonal's items are (tetrahedron, mode, variable). Tolerances as above."""
+    full = cube_tets(10)
+    tp = full.tet_pnt[:ntet] if ntet > 6 else full.tet_pnt[3:3 + ntet]
+    used, inv = np.unique(tp, return_inverse=True)
+    pr = TetProblem(TetMesh(full.pnts[used], inv.reshape(-1, 4)), p, mu=0.01).set_beltrami()
+    assert pr.mesh.ntet == ntet
+    g, o = TetGPU(pr), OracleTet(pr)
+    assert g.setup_preconditioner() == 0 and o.setup_preconditioner() == 0
+    for stage in (pr.phys.nstage, 0, 1, 2):
+        g.rsdl(stage)
+        o.rsdl(stage)
+        assert relerr(g.residual(), o.residual()) < 1e-12, f"res stage {stage}"
+        assert relerr(g.residual(1), o.residual_r()) < 1e-12, f"res_r stage {stage}"
+    if ntet < 10:
+        assert relerr(g.jacobian_diagonal(), o.jacobian_diagonal()) < 1e-7
+    g.close()
