@@ -306,6 +306,7 @@ __global__ void __launch_bounds__(LineCfg<R, P, PHYS, DIFF, RE>::NTHR, LineCfg<R
     };
     const int step = gridDim.x;
     int b = blockIdx.x, slot = 0;
+    chain_next();
     fetch_idx(b, 0);
     fetch_idx(b + step, 1);
     cp_async_wait();

@@ -917,6 +917,12 @@ static void launch_elem(hp_gpu_ctx *c, const Launchers<R> &L, const void *tab, c
         L.elem(tab, c->mesh, st, ph, stage, zero_rr, diff, c->nsm, tune_of(c, R()), c->stream);
 }
 
+// Whether launch_elem ends in the line kernel on the level's stream, so that the next kernel may be
+// chained to it (with curved triangles it ends in a wait for their stream).
+static bool elem_chains(const hp_gpu_ctx *c, const Phys &ph, int diff) {
+    return !(c->emat_on && c->emat_built && ph.physics == HP_PHYS_CD && !diff) && c->elem_kind != HP_ELEM_SCALAR && !c->side;
+}
+
 // Stream-ordered body of rsdl(stage) (no sync, capturable), either precision.
 template <typename R>
 static void enqueue_rsdl_t(hp_gpu_ctx *c, const Launchers<R> &L, const void *tab, const State<R> &st, const Phys &ph,
@@ -931,8 +937,9 @@ static void enqueue_rsdl_t(hp_gpu_ctx *c, const Launchers<R> &L, const void *tab
         if (c->elem_kind == HP_ELEM_SCALAR) L.bflux(tab, c->mesh, st, ph, diff, c->stream);
         const long n = (long)(c->lv + c->ls);
         const int with_b = (ph.physics == HP_PHYS_INS && c->nbseg > 0) ? 1 : 0;
-        k_assemble<R><<<std::min(nblk(n, 256), c->nsm * 16), 256, 0, c->stream>>>(
-            c->mesh, st, c->NV, c->sm, (R)omb, zero_rr, ph.beta[stage] > 0.0 ? 1 : 0, with_b, fold);
+        // chained to the line kernel: residual of 8192 triangles, p = 4, 16.5 -> 15.8 us
+        launch_chained(elem_chains(c, ph, diff), k_assemble<R>, std::min(nblk(n, 256), c->nsm * 16), 256, 0, c->stream,
+                       c->mesh, st, c->NV, c->sm, (R)omb, zero_rr, ph.beta[stage] > 0.0 ? 1 : 0, with_b, fold);
         return;
     }
     const long n = (long)(c->lv + c->ls);
@@ -964,7 +971,8 @@ static void p1_slots(hp_gpu_ctx *c, State<float> &st) {
 // residual with res_r and the source folded in.
 template <typename R>
 static void enqueue_p1_stage(hp_gpu_ctx *c, const Launchers<R> &L, const void *tab, const State<R> &st0, const Phys &ph,
-                             int stage, int diff, R *in, const R *u0, R *out, R *res, unsigned long long *slot) {
+                             int stage, int diff, R *in, const R *u0, R *out, R *res, int chained,
+                             unsigned long long *slot) {
     State<R> st = st0;
     P1Stage<R> s;
     s.u_in = in;
@@ -982,7 +990,7 @@ static void enqueue_p1_stage(hp_gpu_ctx *c, const Launchers<R> &L, const void *t
     s.re = ph.beta[stage] > 0.0 ? 1 : 0;
     s.slot = slot;
     if (p1_small<R>(c->mesh, c->nsm)) {
-        p1_stage<R>(p1_ops_of(c, R()), c->mesh, s, ph, diff, c->nsm, c->stream);
+        p1_stage<R>(p1_ops_of(c, R()), c->mesh, s, ph, diff, c->nsm, chained, c->stream);
         return;
     }
     p1_slots(c, st);
@@ -996,7 +1004,7 @@ template <typename R>
 static void enqueue_rsdl_folded(hp_gpu_ctx *c, const Launchers<R> &L, const void *tab, const State<R> &st,
                                 const Phys &ph, int stage, int diff) {
     if (p1_fused(c))
-        enqueue_p1_stage<R>(c, L, tab, st, ph, stage, diff, st.ugv, (const R *)nullptr, (R *)nullptr, st.resv, nullptr);
+        enqueue_p1_stage<R>(c, L, tab, st, ph, stage, diff, st.ugv, (const R *)nullptr, (R *)nullptr, st.resv, 0, nullptr);
     else enqueue_rsdl_t<R>(c, L, tab, st, ph, stage, diff, 1);
 }
 
@@ -1011,7 +1019,7 @@ static void enqueue_p1_update(hp_gpu_ctx *c, const Launchers<R> &L, const void *
     for (int k = 0; k < ns; ++k) {
         const bool last = k == ns - 1;
         enqueue_p1_stage<R>(c, L, tab, st, ph, k, diff, ns == 1 ? b : k == 0 ? a : (k & 1) ? b : d, ns == 1 ? b : a,
-                            last ? a : (k & 1) ? d : b, last ? st.resv : (R *)nullptr, last ? slot : nullptr);
+                            last ? a : (k & 1) ? d : b, last ? st.resv : (R *)nullptr, k > 0, last ? slot : nullptr);
     }
 }
 

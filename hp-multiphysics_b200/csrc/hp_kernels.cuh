@@ -12,6 +12,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include "hp_chain.cuh"
 
 namespace hpb {
 
@@ -954,6 +955,7 @@ __global__ void k_assemble(Mesh mesh, State<R> st, int NV, int SM, R omb, int ze
                            int fold) {
     const unsigned nv = (unsigned)mesh.npnt * NV, lps = (unsigned)SM * NV, n0 = nv + (unsigned)mesh.nseg * lps;
     const size_t soff = (size_t)3 * mesh.ntri * NV;  // side section of the buffers
+    chain_wait();
     for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k < n0; k += gridDim.x * blockDim.x) {
         R sim = (R)0, sre = (R)0;
         if (k < nv) {

@@ -1,6 +1,7 @@
 // Operators and launcher of the fused p = 1 stage kernel (hp_stage_p1.cuh).
 #include <algorithm>
 
+#include "hp_chain.cuh"
 #include "hp_line.h"
 #include "hp_stage_p1.cuh"
 
@@ -36,16 +37,16 @@ template void p1_ops<double>(const hp_basis_tables &, P1Ops<double> &);
 template void p1_ops<float>(const hp_basis_tables &, P1Ops<float> &);
 
 template <typename R>
-void p1_stage(const P1Ops<R> *ops, const Mesh &m, const P1Stage<R> &s, const Phys &ph, int diff, int nsm,
+void p1_stage(const P1Ops<R> *ops, const Mesh &m, const P1Stage<R> &s, const Phys &ph, int diff, int nsm, int chained,
               cudaStream_t st) {
-    const int blocks = std::min((m.npnt + 3) / 4, nsm * (sizeof(R) == 8 ? 5 : 6));
-    if (ph.physics == HP_PHYS_CD) k_stage_p1<R, 0, false><<<blocks, 128, 0, st>>>(ops, m, s, ph);
-    else if (diff) k_stage_p1<R, 1, true><<<blocks, 128, 0, st>>>(ops, m, s, ph);
-    else k_stage_p1<R, 1, false><<<blocks, 128, 0, st>>>(ops, m, s, ph);
+    const unsigned blocks = std::min((m.npnt + 3) / 4, nsm * (sizeof(R) == 8 ? 5 : 6));
+    if (ph.physics == HP_PHYS_CD) launch_chained(chained, k_stage_p1<R, 0, false>, blocks, 128, 0, st, ops, m, s, ph);
+    else if (diff) launch_chained(chained, k_stage_p1<R, 1, true>, blocks, 128, 0, st, ops, m, s, ph);
+    else launch_chained(chained, k_stage_p1<R, 1, false>, blocks, 128, 0, st, ops, m, s, ph);
 }
 template void p1_stage<double>(const P1Ops<double> *, const Mesh &, const P1Stage<double> &, const Phys &, int, int,
-                               cudaStream_t);
-template void p1_stage<float>(const P1Ops<float> *, const Mesh &, const P1Stage<float> &, const Phys &, int, int,
+                               int, cudaStream_t);
+template void p1_stage<float>(const P1Ops<float> *, const Mesh &, const P1Stage<float> &, const Phys &, int, int, int,
                               cudaStream_t);
 
 template <typename R>

@@ -42,8 +42,11 @@ bool p1_small(const Mesh &m, int nsm) {
     return m.npnt <= 2 * nsm * (sizeof(R) == 8 ? 20 : 24);
 }
 
+// chained (hp_chain.cuh): the kernel before it on the stream is the same update's previous stage. An
+// update of 512 triangles 30.9 -> 28.8 us, cd 20.6 -> 16.5, 11k triangles 53.3 -> 50.1.
 template <typename R>
-void p1_stage(const P1Ops<R> *dev_ops, const Mesh &, const P1Stage<R> &, const Phys &, int diff, int nsm, cudaStream_t);
+void p1_stage(const P1Ops<R> *dev_ops, const Mesh &, const P1Stage<R> &, const Phys &, int diff, int nsm, int chained,
+              cudaStream_t);
 
 // k_vert_p1 after the element kernel.
 template <typename R>

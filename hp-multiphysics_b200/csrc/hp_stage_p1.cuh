@@ -17,6 +17,7 @@
 // 131k triangles 212 -> 367 us, where the element kernel and k_vert_p1 take 141 (hence the rule). Bound by latency (vertex -> incidence -> state
 // loads, then the FP64 chain of a point).
 #pragma once
+#include "hp_chain.cuh"
 #include "hp_p1.h"
 
 namespace hpb {
@@ -73,6 +74,20 @@ __global__ void __launch_bounds__(128, sizeof(R) == 8 ? 5 : 6)
     const R as2_jj = ops->AS2[j][j], as2_jo = ops->AS2[j][1 - j], n0j = ops->N0[j];
     R rmax = (R)0;
     const int nwarp = (gridDim.x * blockDim.x) >> 5;
+    // The next stage may start its CTAs; this one, while the stage before it ends, brings in what no
+    // stage writes: the operators and the incidences and geometry of its first vertices.
+    chain_next();
+    {
+        const int v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+        if (v < mesh.npnt) {
+            const int v0 = mesh.vt_ptr[v], k = lane >> 2, kk = v0 + (k < mesh.vt_ptr[v + 1] - v0 ? k : 0);
+            const double *tg = mesh.tgeo + (size_t)8 * (mesh.vt_idx[kk] >> 2);
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(tg));
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(mesh.vt_pnt + 3 * kk));
+            if (PHYS == 1 && mesh.nbseg > 0) asm volatile("prefetch.global.L1 [%0];" ::"l"(mesh.vb_idx + 2 * v));
+        }
+    }
+    chain_wait();
     for (int v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < mesh.npnt; v += nwarp) {
         const int v0 = mesh.vt_ptr[v], nt = mesh.vt_ptr[v + 1] - v0;
         R im[NV], re[NV];
