@@ -14,8 +14,8 @@ the same metric through the C-ABI with host buffers (pinned state upload + rsdl 
 residual download every step). `time_to_tol` runs W-cycles from the initial state to a
 1e-10 drop of the FP64 residual: plain FP64, FP32 smoothing inside FP64 defect
 correction, and that plus the learned preconditioner correction. `roofline` relates the
-element kernel to the FP64 tensor-core (DMMA) throughput measured in the same run, with
-the HBM fraction of the compulsory bytes beside it.
+element kernel to the FP64 throughput (the DMMA rate; DMMA and DFMA share one pipe) measured in
+the same run, with the HBM fraction of the compulsory bytes beside it.
 
 --gpus N > 1 runs N independent replicas (the path does not shard across GPUs in this
 tier): value = sum over ranks.
@@ -704,8 +704,8 @@ def time_to_tolerance(hpb, dev):
 
 
 def kernel_sweep(hpb, dev, n, ps, steps, timed, stream):
-    """FP64 element-kernel time per p on the lid cavity (n x n split squares): the tensor-core
-    (DMMA) and the scalar warp kernel, with the algorithmic flop rate (oracle op count) and
+    """FP64 element-kernel time per p on the lid cavity (n x n split squares): the default (line)
+    kernel, named by its switch "tensor", and the scalar warp kernel, with the algorithmic flop rate (oracle op count) and
     the FP64 tensor-core peak measured in the same run."""
     from hpb._lib import check
     peak = ctypes.c_double()
@@ -897,18 +897,18 @@ def c3_headline(args, torch, dist, rank, world, dev, stream):
                "sample": f"oracle rsdl(nstage) on a 512 x {STRIP_ROWS}-square strip of the C3 mesh "
                          f"({2 * C3_N * STRIP_ROWS} triangles, p={C3_P}, lid-cavity state), {reps} evaluations "
                          "in 10 s, 1 core"}
-    # element kernel (k_rsdl_ins_mma or k_rsdl_elem), k_bdry_flux_ins, k_assemble, and the k_rsdl_fold
-    # that hp_gpu_enqueue_rsdl adds (res += res_r for the caller, nstage.cpp:76-82)
-    launches_per_step = 4
+    # k_rsdl_line (boundary fluxes inside), k_assemble (res += res_r inside, nstage.cpp:76-82); the
+    # scalar kernel has k_bdry_flux_ins beside it
+    launches_per_step = 3 if args.elem == "scalar" else 2
     line = {
         "metric": METRIC, "value": value, "unit": "GDoF/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": t_ms / args.steps, "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": "f64", "data": "synthetic", "config": c3_config(),
-        "roofline": {"bound": "tensor", "achieved": achieved, "peak": peak.value, "unit": "TFLOP/s",
+        "roofline": {"bound": "fp64", "achieved": achieved, "peak": peak.value, "unit": "TFLOP/s",
                      "frac": achieved / peak.value, "traffic": traffic, "kernel": "element residual (fine level)",
                      "kernel_ms": k_ms, "flops_per_element": fl_el, "flops_source": fl_src,
-                     "peak_source": "FP64 tensor-core (DMMA) rate measured in this run by hp_tet_fp64_mma_peak "
-                                    "(MEASURED_PEAKS.json has no FP64 figure)",
+                     "peak_source": "FP64 rate measured in this run by hp_tet_fp64_mma_peak (DMMA, on the pipe of "
+                                    "the DFMAs; MEASURED_PEAKS.json has no FP64 figure)",
                      "hbm": {"compulsory_bytes": comp_bytes, "achieved_gbs": comp_bytes / (k_ms * 1e-3) / 1e9,
                              "peak_gbs": hbm, "frac": comp_bytes / (k_ms * 1e-3) / 1e9 / hbm,
                              "peak_source": hbm_src,
@@ -1201,7 +1201,7 @@ def main():
         cv, n = run_cpu(1, 10.0)
         cpu = {"value": cv, "unit": "GDoF/s", "cores": 1, "kind": "port",
                "sample": f"oracle rsdl(nstage) on a {n}x{n} split-square mesh, p={P}, 10 s, 1 core"}
-    launches_per_step = 3  # k_rsdl_pre, k_rsdl_emat, k_rsdl_fold (cd has no boundary-flux kernel)
+    launches_per_step = 2  # k_rsdl_emat, k_assemble (cd has no boundary-flux kernel)
     cfg = workload_config()
     cfg["element_operators"] = ("stored: built once by the element kernel on unit vectors "
                                 f"({build_ms:.1f} ms, {2 * op_bytes / 1e9:.2f} GB FP64 + FP32 copy), "

@@ -23,12 +23,13 @@
 // 37.0 TFLOP/s against 34.5 for DFMA, and 31 in sum when mixed), so the dense per-point operators
 // that a fragment needs (98k flops per triangle at p = 6 with the padding) lose to the
 // sum-factorised form (about 40k). Measured, FP64, 131k triangles, full residual, against two
-// triangles per warp on mma.m8n8k4.f64: p = 3 157 -> 89 us, p = 4 308 -> 171, p = 5 503 -> 246,
-// p = 6 719 -> 403, p = 8 1884 -> 1169; p = 2 against the scalar warp kernel 197 -> 52. Bound by
+// triangles per warp on mma.m8n8k4.f64: p = 3 157 -> 91 us, p = 4 308 -> 166, p = 5 503 -> 246,
+// p = 6 719 -> 413, p = 8 1884 -> 1169; p = 2 against the scalar warp kernel 197 -> 50 (the boundary
+// fluxes, a kernel of their own before, included). Bound by
 // issue: the FP64 pipe is busy 33 % (p = 6) to 41 % (p = 3) of the time; 7 to 16 warps an SM fit.
 // FP32: the same form beats TF32 fragments (mma.m16n8k8, operands rounded to 10 bits), and in
-// full FP32: an update of the FP32 smoother, 131k triangles, p = 3 728 -> 522 us, p = 4 1202 ->
-// 854, p = 6 2625 -> 2031, p = 8 7305 -> 4032, p = 2 against the scalar warp kernel 670 -> 269; in
+// full FP32: an update of the FP32 smoother, 131k triangles, p = 3 728 -> 482 us, p = 4 1202 ->
+// 820, p = 6 2625 -> 2020, p = 8 7305 -> 3893, p = 2 against the scalar warp kernel 670 -> 247; in
 // plain form against the scalar warp kernel p = 6 4475 -> 1885. Bound by issue, too: half of the
 // instructions are FMAs. cd against the scalar warp kernel, an FP64 update of 80k triangles: p = 1
 // 126 -> 68 us (with k_vert_p1), p = 2 282 -> 121, p = 4 739 -> 322; p = 6 of 20k 626 -> 330.

@@ -35,8 +35,8 @@ void p1_ops(const hp_basis_tables &, P1Ops<R> &);
 
 // Whether a level's stage runs vertex by vertex (k_stage_p1): its vertices, one warp each, are two
 // waves of the resident warps at most. Measured per update (five stages), vertex by vertex / element
-// kernel and k_vert_p1: FP64 4225 vertices 51 / 54 us, 66k vertices 367 / 141; FP32 4225 vertices
-// 41 / 57, 66k vertices 251 / 116.
+// kernel and k_vert_p1: FP64 4225 vertices 48 / 54 us, 66k vertices 367 / 141; FP32 4225 vertices
+// 38 / 57, 66k vertices 251 / 116.
 template <typename R>
 bool p1_small(const Mesh &m, int nsm) {
     return m.npnt <= 2 * nsm * (sizeof(R) == 8 ? 20 : 24);

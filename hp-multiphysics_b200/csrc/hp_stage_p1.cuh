@@ -4,8 +4,7 @@
 // boundary fluxes (hp_edge_bdry::rsdl, hp_boundary.cpp:973-1049), tri_hp::minvrt
 // (setup_preconditioner.cpp:102-373) and the stage update (nstage.cpp:387-409) of a vertex need
 // only the triangles around it. A warp takes a vertex: lane 4 e + q evaluates Gauss point
-// q = 2 i + j of the vertex's triangle e (eight at a time) with the dense per-point operators, as
-// k_rsdl_ins_p1 does, and keeps its share of the one test function that belongs to the vertex; the
+// q = 2 i + j of the vertex's triangle e (eight at a time) with the dense per-point operators, and keeps its share of the one test function that belongs to the vertex; the
 // shares are summed by shuffles in a fixed order and lane n finishes variable n. A triangle is
 // evaluated three times, once for each of its vertices, and nothing goes through memory between
 // the element loop and the update: the separate kernels (element, boundary flux, assembly, vertex
@@ -13,7 +12,7 @@
 // from one buffer and written to another (neighbours are read), see p1_update.
 // For small levels (p1_small); larger ones take the element kernel and
 // k_vert_p1, since the threefold evaluation then costs more than the launch it saves.
-// Measured per FP64 update (five stages): 512 triangles 86 -> 31 us, 8192 triangles 89 -> 51 us,
+// Measured per FP64 update (five stages): 512 triangles 86 -> 29 us, 8192 triangles 89 -> 48 us,
 // 131k triangles 212 -> 367 us, where the element kernel and k_vert_p1 take 141 (hence the rule). Bound by latency (vertex -> incidence -> state
 // loads, then the FP64 chain of a point).
 #pragma once
