@@ -1219,7 +1219,7 @@ def main():
         "elem_operator_build_ms": build_ms,
         "update_ms": u_ms, "update_gdofs_per_stage": ndof * ns / (u_ms * 1e-3) / 1e9,
         "fp32_update_ms": u32_ms,
-        "matrix_free": {"value": ndof / (mf_ms * 1e-3) / 1e9, "ms_per_step": mf_ms, "kernel": "k_rsdl_elem",
+        "matrix_free": {"value": ndof / (mf_ms * 1e-3) / 1e9, "ms_per_step": mf_ms, "kernel": "k_rsdl_line",
                         "kernel_ms": mf_k, "fp64_tflops": fl / (mf_k * 1e-3) / 1e12, "flops_per_launch": fl,
                         "update_ms": mf_u},
         "time_to_tol": tol,

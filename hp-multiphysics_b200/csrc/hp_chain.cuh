@@ -6,7 +6,7 @@
 // us a kernel (figures at the launches). A chain begins with an ordinary launch, and whatever does not
 // know the kernel before it launches an ordinary one. Only the vertex kernels of small p = 1 levels and
 // the assembly after the line kernel are chained: the preconditioner's phases and the persistent line
-// kernel after them lose what they gain (p = 6 cavity, 8 sweeps with all of it chained 6640 us against
+// kernel after them lose what they gain (p = 6 cavity, 2 sweeps with all of it chained 6640 us against
 // 6287; an FP32-smoothed solve 830 ms against 782), since their CTAs then sit on the SMs early.
 #pragma once
 #include <cuda_runtime.h>
