@@ -131,7 +131,7 @@ struct Launchers {
                  int threads, cudaStream_t);
     void (*intr)(const Mesh &, const State<R> &, const DevMinv<R> *, double cfla, int upd, int threads, cudaStream_t);
     void (*vert)(const Mesh &, const State<R> &, const DevMinv<R> *, int sm, int im, double cfla, int upd, int fold,
-                 unsigned long long *slot, int threads, cudaStream_t);
+                 unsigned long long *slot, int threads, int nsm, cudaStream_t);
     int elem_smem;
     cudaError_t (*set_smem)();
     // cd element operators: length of one operator array, build, apply
@@ -262,13 +262,21 @@ struct LaunchImpl {
             k_minv_int_flat<R, NV, SM, IM><<<nblk((long)m.ntri * NV, th), th, 0, st>>>(m, s, mt, (R)cfla, upd);
     }
     static void vert(const Mesh &m, const State<R> &s, const DevMinv<R> *mt, int sm, int im, double cfla, int upd,
-                     int fold, unsigned long long *slot, int th, cudaStream_t st) {
+                     int fold, unsigned long long *slot, int th, int nsm, cudaStream_t st) {
         if constexpr (SM > 0) {
-            // a lane group per vertex, sized to the vertex's removal terms (about 6 sides x SM
-            // and 6 triangles x IM)
-            constexpr int LPV = SM + IM >= 8 ? 32 : (SM + IM >= 3 ? 8 : 4);
-            k_minv_vert_coop<R, NV, SM, IM, LPV><<<nblk((long)m.npnt * LPV, th), th, 0, st>>>(m, s, mt, (R)cfla, upd,
-                                                                                             fold, slot);
+            // a lane group per vertex for its removal terms (about 6 sides x SM and 6 triangles x IM),
+            // wide on small levels, where it shortens a vertex's chain of loads, and narrow on the
+            // others, where it saves instructions: fewer shuffles, and the lanes that finish a vertex
+            // are a larger share. An FP64 update, cavity, wide / narrow: p = 3 4k vertices 159 / 162 us,
+            // 9k 200 / 198, 66k 736 / 675; p = 4 4k 217 / 222, 17k 379 / 375, 66k 1215 / 1160; p = 6 4k
+            // 356 / 355, 9k 548 / 523, 66k 3120 / 2942. p = 2: 2 lanes always (4 are 100 / 97 at 4k).
+            constexpr int WIDE = SM + IM >= 8 ? 32 : (SM + IM >= 3 ? 8 : 2), NARROW = SM + IM >= 8 ? 8 : 2;
+            if (m.npnt <= 48 * nsm)
+                k_minv_vert_coop<R, NV, SM, IM, WIDE><<<nblk((long)m.npnt * WIDE, th), th, 0, st>>>(m, s, mt, (R)cfla, upd,
+                                                                                                   fold, slot);
+            else
+                k_minv_vert_coop<R, NV, SM, IM, NARROW><<<nblk((long)m.npnt * NARROW, th), th, 0, st>>>(
+                    m, s, mt, (R)cfla, upd, fold, slot);
         } else {
             k_minv_vert<R, NV><<<nblk(m.npnt, th), th, 0, st>>>(m, s, mt, sm, im, (R)cfla, upd, fold, slot);
         }
@@ -1028,7 +1036,7 @@ template <typename R>
 static void enqueue_minvrt_t(hp_gpu_ctx *c, const Launchers<R> &L, const State<R> &st, const DevMinv<R> *mt,
                              double cfla, int upd, int fold, unsigned long long *slot) {
     const int th = tune_of(c, R()).minv_threads;
-    L.vert(c->mesh, st, mt, c->sm, c->im, cfla, upd, fold, slot, th, c->stream);
+    L.vert(c->mesh, st, mt, c->sm, c->im, cfla, upd, fold, slot, th, c->nsm, c->stream);
     for (int mode = 0; mode < c->sm; ++mode) L.side(c->mesh, st, mt, c->im, mode, cfla, upd, fold, th, c->stream);
     if (c->im > 0) L.intr(c->mesh, st, mt, cfla, upd, th, c->stream);
 }

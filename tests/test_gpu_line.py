@@ -112,3 +112,19 @@ def test_p1_updates_match_oracle(mesh, nstage, physics):
     o.rsdl(nstage)
     assert relerr(g.residual(), o.residual()) < 1e-9  # (the residual has dropped below its terms)
     g.close()
+
+
+@pytest.mark.parametrize("physics,p,n", [("ins", p, n) for p in (2, 3, 4, 6) for n in (83, 84)] +
+                         [("cd", 3, 84), ("ins", 2, 3), ("ins", 5, 5), ("cd", 7, 4)])
+def test_update_at_the_two_forms_of_the_vertex_phase(physics, p, n):
+    """An update (minvrt's vertex phase with wide and narrow lane groups: 7056 and 7225 vertices lie
+    on the two sides of the size that divides them on 148 SMs, 7104) against the oracle, tolerance
+    as above for a third of the updates."""
+    pr = _problem(hpb.square_mesh(n), p, physics)
+    g, o = pr.gpu(), Oracle(pr)
+    assert g.setup_preconditioner() == 0 and o.setup_preconditioner() == 0
+    hist = g.iterate(1)
+    o.update()
+    assert abs(hist[0] - o.maxres()[0]) <= 1e-9 * o.maxres()[0]
+    assert relerr(g.state(), o.state()) < 1e-11
+    g.close()
