@@ -79,10 +79,12 @@ __global__ void __launch_bounds__(128, sizeof(R) == 8 ? 5 : 6)
     {
         const int v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
         if (v < mesh.npnt) {
-            const int v0 = mesh.vt_ptr[v], k = lane >> 2, kk = v0 + (k < mesh.vt_ptr[v + 1] - v0 ? k : 0);
-            const double *tg = mesh.tgeo + (size_t)8 * (mesh.vt_idx[kk] >> 2);
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(tg));
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(mesh.vt_pnt + 3 * kk));
+            const int v0 = mesh.vt_ptr[v], nt = mesh.vt_ptr[v + 1] - v0, k = lane >> 2, kk = v0 + (k < nt ? k : 0);
+            if (nt > 0) {  // a last vertex without triangles has v0 past the end of the incidences
+                const double *tg = mesh.tgeo + (size_t)8 * (mesh.vt_idx[kk] >> 2);
+                asm volatile("prefetch.global.L1 [%0];" ::"l"(tg));
+                asm volatile("prefetch.global.L1 [%0];" ::"l"(mesh.vt_pnt + 3 * kk));
+            }
             if (PHYS == 1 && mesh.nbseg > 0) asm volatile("prefetch.global.L1 [%0];" ::"l"(mesh.vb_idx + 2 * v));
         }
     }
