@@ -196,11 +196,14 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_al
 // where a mode lies and its sign are looked up (TetLoc), not worked out per value; the phases
 // between the MMAs give a lane a line along x of its own tetrahedron, whose geometry it holds and
 // whose x sums take each value once. Before: two warps a CTA, 8 warps an SM, the convective fluxes
-// in shared memory. 197k tetrahedra, p = 3, full residual 1760 -> 1230 us, without the real part
-// 1100 -> 441; p = 2 763 -> 540 and 436 -> 182; p = 1 219 -> 169 and 124 -> 71; p = 4 (25k) 1221 ->
-// 640 and 585 -> 214; the p = 3 Jacobian diagonal 137 -> 104 ms. The derivatives stay modal: taken
+// in shared memory. 197k tetrahedra, p = 3, full residual 1760 -> 1270 us, without the real part
+// 1100 -> 442; p = 2 762 -> 599 and 436 -> 183; p = 1 218 -> 172 and 124 -> 71; p = 4 (25k) 1222 ->
+// 686 and 583 -> 214; the p = 3 Jacobian diagonal 137 -> 107 ms. The derivatives stay modal: taken
 // from the point values by the 1D operators they would save 120 of 448 MMAs, but their error is
-// 1.6e-15 instead of 4e-17 (the collapsed coordinates amplify it).
+// 1.6e-15 instead of 4e-17 (the collapsed coordinates amplify it). The viscous fluxes stay apart from
+// the convective ones: one exchange of the total fluxes of all variables, the viscous ones got back
+// as total minus convective, took 1234, 538, 169 and 639 us, but left res_r a rounding of the size of
+// eps times the convective terms (at mu = 1e-6 without stabilisation 1e-11 of res_r instead of 5e-16).
 template <int P, bool RE>
 struct TetMma {
     using C = TetCfg<P>;
@@ -214,18 +217,17 @@ struct TetMma {
     static constexpr int QP = pad4(C::Q);       // u, v, w, p at the points [NV][QP]
     static constexpr int VS = pad4(3 * C::Q);   // fluxes [NV][VS], component c at c * Q
     // a warp's area: gathered modes [2][NV T], vertex coordinates and tau [2][14], both of the next
-    // pair from the moment this pair's are in registers; u, v, w, p [2][NV][QP]; total fluxes, then
-    // the real ones [2][NV][VS]; indices
-    // of three pairs [3][2][25]
+    // pair from the moment this pair's are in registers; u, v, w, p [2][NV][QP]; velocity derivatives,
+    // then viscous fluxes, then all real ones [2][NV][VS]; indices of three pairs [3][2][25]
     static constexpr int U = 0, XY = U + 2 * NV * C::T, UQ = XY + 28, FR = UQ + 2 * NV * QP,
                          IDX = FR + (RE ? 2 * NV * VS : 0), S_WARP = IDX + 76;
     static_assert(UQ % 2 == 0 && FR % 2 == 0 && S_WARP % 2 == 0, "pairs of doubles are stored at once");
     static constexpr int NG = NT < 8 ? NT : 8;  // projection n-tiles accumulated together
     static constexpr size_t PROJ_LEN = (size_t)4 * NT * KS * 32, INT_LEN = (size_t)NT2 * QK * 3 * 32;
     static constexpr int fit = (227 * 1024 / 8) / S_WARP;  // warps an SM, one CTA
-    // as many as fit (12 at p = 3 with the real part: 1640, 1460, 1230 us with 10, 11, 12 at 197k
+    // as many as fit (12 at p = 3 with the real part: 1460, 1360, 1270 us with 10, 11, 12 at 197k
     // tetrahedra), up to 16: without the real part 20 are 444 against 441 us at p = 3, 301 against 214
-    // at p = 4 (25k), 16 with it 540 against 556 with 12 at p = 2
+    // at p = 4 (25k), at p = 2 12 are 195 against 183 (with it 594 against 597)
     static constexpr int WPC = fit < 16 ? fit : 16;
     static constexpr size_t SMEM = (size_t)S_WARP * WPC * sizeof(double);
 };
@@ -476,31 +478,20 @@ __global__ void __launch_bounds__(TetMma<P, RE>::WPC * 32, 1)
             const double *const uq = base + M::UQ + e * NV * QP;
             double *const fr = base + M::FR + e * NV * VS;
             const double cjcbi = mu / cj;
-            // the convective and pressure flux of the momentum at a point, f3 the mass flux
-            auto conv = [&](const double (&uu)[4], double (&f3)[3], double (&f)[3][3]) {
-                const double fx = rho * uu[0], fy = rho * uu[1], fz = rho * uu[2];
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    f3[c] = d[c][0] * fx + d[c][1] * fy + d[c][2] * fz;
-#pragma unroll
-                    for (int k = 0; k < 3; ++k) f[k][c] = uu[k] * f3[c] + d[c][k] * uu[3];
-                }
-            };
             constexpr int NL = (GG + 15) / 16;  // x lines of a lane; at p = 1 there are lanes for each half of one
             constexpr int SP = 2 * GG <= 16 ? 2 : 1, NI = G / SP;
             const int l16 = lane & 15, i0 = SP > 1 && l16 >= GG ? NI : 0, r0 = SP > 1 && l16 >= GG ? l16 - GG : l16;
+            auto mine = [&](int r) { return SP > 1 ? l16 < SP * GG : r < GG; };
             double rsd[NL][NI][NV];
-            // ---- total fluxes, in the place of the velocity derivatives; lanes own lines along x
+            // ---- viscous fluxes, in the place of the velocity derivatives; lanes own lines along x
 #pragma unroll
             for (int it = 0; it < NL; ++it) {
                 const int r = r0 + 16 * it;
-                if (SP > 1 ? l16 >= SP * GG : r >= GG) break;
+                if (!mine(r)) break;
 #pragma unroll
                 for (int ii = 0; ii < NI; ++ii) {
                     const int q = (i0 + ii) * GG + r;
-                    const double uu[4] = {uq[q], uq[QP + q], uq[2 * QP + q], uq[3 * QP + q]};
-                    double f3[3], f[3][3], du[3][3], h[3][3];
-                    conv(uu, f3, f);
+                    double du[3][3], h[3][3];
 #pragma unroll
                     for (int k = 0; k < 3; ++k)
 #pragma unroll
@@ -514,76 +505,104 @@ __global__ void __launch_bounds__(TetMma<P, RE>::WPC * 32, 1)
                     for (int k = 0; k < 3; ++k)
 #pragma unroll
                         for (int c = 0; c < 3; ++c)
-                            fr[k * VS + c * Q + q] =
-                                f[k][c] - cjcbi * (d[c][0] * (h[k][0] + h[0][k]) + d[c][1] * (h[k][1] + h[1][k]) +
-                                                   d[c][2] * (h[k][2] + h[2][k]));
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) fr[3 * VS + c * Q + q] = f3[c];
+                            fr[k * VS + c * Q + q] = -cjcbi * (d[c][0] * (h[k][0] + h[0][k]) + d[c][1] * (h[k][1] + h[1][k]) +
+                                                               d[c][2] * (h[k][2] + h[2][k]));
                 }
             }
-            __syncwarp();
-            // ---- strong residual at the lane's points
+            // ---- strong residual at the lane's points, two variables at a time: the total fluxes of
+            //      one are exchanged in the place of its viscous ones, which the lane holds meanwhile,
+            //      those of the other in the place of variable 3, which has no viscous ones. (Got back
+            //      as total minus convective, the viscous fluxes would carry the rounding of the
+            //      convective ones, 1 / mu of their own.)
 #pragma unroll
-            for (int it = 0; it < NL; ++it) {
-                const int r = r0 + 16 * it;
-                if (SP > 1 ? l16 >= SP * GG : r >= GG) break;
-                const int j = r / G, kk = r - j * G;
-                const double zz = s1d[3 * GG + G + kk], yz = s1d[3 * GG + j] * zz;
+            for (int m = 0; m < NV; m += 2) {
+                double vis[NL][NI][3];
 #pragma unroll
-                for (int i = 0; i < NI; ++i)
+                for (int it = 0; it < NL; ++it) {
+                    const int r = r0 + 16 * it;
+                    if (!mine(r)) break;
 #pragma unroll
-                    for (int m = 0; m < NV; ++m) rsd[it][i][m] = 0.0;
+                    for (int ii = 0; ii < NI; ++ii) {
+                        const int q = (i0 + ii) * GG + r;
+                        const double u0 = uq[q], u1 = uq[QP + q], u2 = uq[2 * QP + q], prs = uq[3 * QP + q];
 #pragma unroll
-                for (int l = 0; l < G; ++l)
-#pragma unroll
-                    for (int m = 0; m < NV; ++m) {
-                        const double *fx = fr + m * VS + l * GG + r;
-                        const double f0 = fx[0], f12 = fx[Q] + fx[2 * Q];
-#pragma unroll
-                        for (int i = 0; i < NI; ++i)
-                            if constexpr (SP == 1) rsd[it][i][m] += sm.Ax[i][l] * f0 + sm.Bx[i][l] * f12;
-                            else rsd[it][i][m] += s1d[3 * GG + 2 * G + (i0 + i) * G + l] * f0 + s1d[4 * GG + 2 * G + (i0 + i) * G + l] * f12;
+                        for (int c = 0; c < 3; ++c) {
+                            const double f3 = d[c][0] * (rho * u0) + d[c][1] * (rho * u1) + d[c][2] * (rho * u2);
+                            vis[it][ii][c] = fr[m * VS + c * Q + q];
+                            fr[m * VS + c * Q + q] = ((m == 0 ? u0 : u2) * f3 + d[c][m] * prs) + vis[it][ii][c];
+                            fr[3 * VS + c * Q + q] = m == 0 ? (u1 * f3 + d[c][1] * prs) + fr[VS + c * Q + q] : f3;
+                        }
                     }
+                }
+                __syncwarp();
 #pragma unroll
-                for (int ii = 0; ii < NI; ++ii) {
-                    const int i = i0 + ii;
-                    double ay[NV], az[NV];
+                for (int it = 0; it < NL; ++it) {
+                    const int r = r0 + 16 * it;
+                    if (!mine(r)) break;
+                    const int j = r / G, kk = r - j * G;
+                    const double zz = s1d[3 * GG + G + kk], yz = s1d[3 * GG + j] * zz;
+                    const double *const tot[2] = {fr + m * VS, fr + 3 * VS};
+                    double x[2][NI], ay[2][NI], az[2][NI];
 #pragma unroll
-                    for (int m = 0; m < NV; ++m) ay[m] = az[m] = 0.0;
+                    for (int h = 0; h < 2; ++h)
+#pragma unroll
+                        for (int i = 0; i < NI; ++i) x[h][i] = ay[h][i] = az[h][i] = 0.0;
+#pragma unroll
+                    for (int l = 0; l < G; ++l)
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const double *fx = tot[h] + l * GG + r;
+                            const double f0 = fx[0], f12 = fx[Q] + fx[2 * Q];
+#pragma unroll
+                            for (int i = 0; i < NI; ++i)
+                                if constexpr (SP == 1) x[h][i] += sm.Ax[i][l] * f0 + sm.Bx[i][l] * f12;
+                                else x[h][i] += s1d[3 * GG + 2 * G + (i0 + i) * G + l] * f0 + s1d[4 * GG + 2 * G + (i0 + i) * G + l] * f12;
+                        }
 #pragma unroll
                     for (int l = 0; l < G; ++l) {
                         const double cay = s1d[j * G + l], cby = s1d[GG + j * G + l], caz = s1d[2 * GG + kk * G + l];
-                        const double *fy = fr + (i * G + l) * G + kk, *fz = fr + (i * G + j) * G + l;
 #pragma unroll
-                        for (int m = 0; m < NV; ++m) {
-                            ay[m] += cay * fy[m * VS + Q] + cby * fy[m * VS + 2 * Q];
-                            az[m] += caz * fz[m * VS + 2 * Q];
+                        for (int ii = 0; ii < NI; ++ii) {
+                            const int qy = ((i0 + ii) * G + l) * G + kk, qz = ((i0 + ii) * G + j) * G + l;
+#pragma unroll
+                            for (int h = 0; h < 2; ++h) {
+                                ay[h][ii] += cay * tot[h][Q + qy] + cby * tot[h][2 * Q + qy];
+                                az[h][ii] += caz * tot[h][2 * Q + qz];
+                            }
                         }
                     }
 #pragma unroll
-                    for (int m = 0; m < NV; ++m) rsd[it][ii][m] = yz * rsd[it][ii][m] + zz * ay[m] + az[m];
+                    for (int ii = 0; ii < NI; ++ii)
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) rsd[it][ii][m + h] = yz * x[h][ii] + zz * ay[h][ii] + az[h][ii];
+                }
+                __syncwarp();
+#pragma unroll
+                for (int it = 0; it < NL; ++it) {
+                    const int r = r0 + 16 * it;
+                    if (!mine(r)) break;
+#pragma unroll
+                    for (int ii = 0; ii < NI; ++ii)
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) fr[m * VS + c * Q + (i0 + ii) * GG + r] = vis[it][ii][c];
                 }
             }
-            __syncwarp();
             // ---- viscous + SUPG fluxes (variable 3: the continuity SUPG term)
 #pragma unroll
             for (int it = 0; it < NL; ++it) {
                 const int r = r0 + 16 * it;
-                if (SP > 1 ? l16 >= SP * GG : r >= GG) break;
+                if (!mine(r)) break;
 #pragma unroll
                 for (int ii = 0; ii < NI; ++ii) {
                     const int q = (i0 + ii) * GG + r;
-                    const double uu[4] = {uq[q], uq[QP + q], uq[2 * QP + q], uq[3 * QP + q]};
+                    const double uu[3] = {uq[q], uq[QP + q], uq[2 * QP + q]};
                     const double tr[4] = {tau0 * rsd[it][ii][0], tau0 * rsd[it][ii][1], tau0 * rsd[it][ii][2], tau3 * rsd[it][ii][3]};
-                    double f3[3], f[3][3];
-                    conv(uu, f3, f);
 #pragma unroll
                     for (int c = 0; c < 3; ++c) {
                         const double du = d[c][0] * uu[0] + d[c][1] * uu[1] + d[c][2] * uu[2];
                         const double dt = d[c][0] * tr[0] + d[c][1] * tr[1] + d[c][2] * tr[2];
 #pragma unroll
-                        for (int m = 0; m < 3; ++m)
-                            fr[m * VS + c * Q + q] = (fr[m * VS + c * Q + q] - f[m][c]) - (du * tr[m] + dt * uu[m] + d[c][m] * tr[3]);
+                        for (int m = 0; m < 3; ++m) fr[m * VS + c * Q + q] -= du * tr[m] + dt * uu[m] + d[c][m] * tr[3];
                         fr[3 * VS + c * Q + q] = -dt;
                     }
                 }
