@@ -903,12 +903,17 @@ static void launch_line(hp_gpu_ctx *c, const State<float> &st, const Phys &ph, i
     c->line32.launch(c->line_tab32.data(), c->d_tab32, c->mesh, st, ph, stage, zero_rr, diff, c->nsm, c->stream);
 }
 
+// Whether the element part is the stored cd operators.
+static bool emat_used(const hp_gpu_ctx *c, const Phys &ph, int diff) {
+    return c->emat_on && c->emat_built && ph.physics == HP_PHYS_CD && !diff;
+}
+
 // Element part of rsdl(stage): the stored cd element operators once built, else the
 // matrix-free element kernel.
 template <typename R>
 static void launch_elem(hp_gpu_ctx *c, const Launchers<R> &L, const void *tab, const State<R> &st, const Phys &ph,
                         int stage, int zero_rr, int diff) {
-    if (c->emat_on && c->emat_built && ph.physics == HP_PHYS_CD && !diff)
+    if (emat_used(c, ph, diff))
         L.emat_apply(emat_of(c, R()), c->mesh, st, ph, stage, zero_rr, c->nsm, tune_of(c, R()), c->stream);
     else if (c->elem_kind != HP_ELEM_SCALAR) {
         // the curved triangles beside the straight ones, on a stream of their own (other slots)
@@ -928,7 +933,7 @@ static void launch_elem(hp_gpu_ctx *c, const Launchers<R> &L, const void *tab, c
 // Whether launch_elem ends in the line kernel on the level's stream, so that the next kernel may be
 // chained to it (with curved triangles it ends in a wait for their stream).
 static bool elem_chains(const hp_gpu_ctx *c, const Phys &ph, int diff) {
-    return !(c->emat_on && c->emat_built && ph.physics == HP_PHYS_CD && !diff) && c->elem_kind != HP_ELEM_SCALAR && !c->side;
+    return !emat_used(c, ph, diff) && c->elem_kind != HP_ELEM_SCALAR && !c->side;
 }
 
 // Stream-ordered body of rsdl(stage) (no sync, capturable), either precision.
@@ -997,7 +1002,7 @@ static void enqueue_p1_stage(hp_gpu_ctx *c, const Launchers<R> &L, const void *t
     s.cfla = (R)(ph.alpha[stage] * ph.cfl);
     s.re = ph.beta[stage] > 0.0 ? 1 : 0;
     s.slot = slot;
-    if (p1_small<R>(c->mesh, c->nsm)) {
+    if (p1_small<R>(c->mesh, c->nsm) && !emat_used(c, ph, diff)) {
         p1_stage<R>(p1_ops_of(c, R()), c->mesh, s, ph, diff, c->nsm, chained, c->stream);
         return;
     }
@@ -2207,7 +2212,7 @@ static int tune_prec(hp_gpu_ctx *c, const Launchers<R> &L, const void *tab, cons
     auto elem = [&]() { launch_elem<R>(c, L, tab, st, ph, ns, 1, diff); };
     Tune keep = tn;
     float best = 1e30f;
-    if (c->emat_on && c->emat_built && ph.physics == HP_PHYS_CD && !diff) {
+    if (emat_used(c, ph, diff)) {
         const int tpps[2] = {1, 2}, ctas[3] = {0, 4, 2};
         for (int a : tpps)
             for (int b : ctas) {

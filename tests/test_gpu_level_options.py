@@ -1,0 +1,43 @@
+"""Options of a level that choose what its residual runs on: the stored operators at p = 1.
+
+Tolerance of the residuals: 1e-12 of the largest value, as in test_gpu_parity.py."""
+import numpy as np
+import pytest
+
+import hpb
+from oracle.oracle import Oracle
+from test_gpu_parity import relerr
+
+pytestmark = pytest.mark.gpu
+
+
+def _vec(arrays):
+    return np.concatenate([a.ravel() for a in arrays])
+
+
+@pytest.mark.parametrize("n", [7, 83, 84])
+def test_stored_operators_are_applied_at_p1(n):
+    """n = 7 and 84 lie on the two sides of the size that divides the two forms of a p = 1 stage, n = 83
+    between the sizes of FP64 and FP32. The stored operators sum an element's products in another
+    order than the matrix-free kernels: the residuals agree to rounding and are not the same bit by
+    bit, in either precision."""
+    pr = hpb.cd_sinsin(n=n, p=1, kcond=1e-2, src=0.7)
+    a, b, o = pr.gpu(), pr.gpu(), Oracle(pr)
+    assert a.setup_preconditioner() == 0 and b.setup_preconditioner() == 0 and o.setup_preconditioner() == 0
+    b.element_matrices(True)
+    ns = pr.phys.nstage
+    for prec, tol in ((0, 1e-12), (1, 1e-5)):
+        a.rsdl(ns, prec)
+        b.rsdl(ns, prec)
+        o.rsdl(ns)
+        assert relerr(b.residual(), o.residual()) < tol and relerr(a.residual(), o.residual()) < tol
+        assert not np.array_equal(_vec(a.residual()), _vec(b.residual()))
+    a.iterate(3)
+    b.iterate(3)
+    assert relerr(b.state(), a.state()) < 1e-11 and not np.array_equal(_vec(a.state()), _vec(b.state()))
+    b.element_matrices(False)
+    b.upload(pr.ugv, pr.ugs, pr.ugi)
+    b.iterate(3)
+    assert np.array_equal(_vec(a.state()), _vec(b.state()))
+    a.close()
+    b.close()
