@@ -1189,10 +1189,6 @@ extern "C" int hp_gpu_l2error(hp_gpu_ctx *c, const hp_field *fld, double *l2, do
 
 extern "C" int hp_gpu_set_element_kernel(hp_gpu_ctx *c, int kind) {
     if (!c || (kind != HP_ELEM_SCALAR && kind != HP_ELEM_TENSOR && kind != HP_ELEM_POINT)) return HP_EINVAL;
-    if (kind == HP_ELEM_TENSOR && c->ph.physics != HP_PHYS_INS) {
-        set_err("the line element kernel is built for ins only");
-        return HP_ENOTSUP;
-    }
     if (kind == HP_ELEM_POINT && (c->ph.physics != HP_PHYS_INS || c->p != 1)) {
         set_err("HP_ELEM_POINT is for ins at p = 1 only");
         return HP_ENOTSUP;

@@ -269,8 +269,8 @@ class GPULevel:
         return K
 
     def element_kernel(self, kind):
-        """Element kernel (hp_gpu_set_element_kernel): "tensor" or "point" (ins, at
-        p = 1): the line kernel, the default; "scalar": the warp kernel."""
+        """Element kernel (hp_gpu_set_element_kernel): "tensor" or, for ins at p = 1, "point": the
+        line kernel, the default; "scalar": the warp kernel."""
         L.check(self.lib.hp_gpu_set_element_kernel(self.h, {"scalar": 0, "tensor": 1, "point": 2}[kind]),
                 "set_element_kernel")
 

@@ -200,10 +200,11 @@ int hp_gpu_resnorm(hp_gpu_ctx *ctx, double *l2, double *linf);
  * tri_hp/nstage.cpp:52-73). The default of both physics is the
  * line kernel, sum-factorised with one lane per triangle and one warp per line of the
  * tensor-product points; at p = 1 updates and residuals fuse it with the vertex phase, on
- * small levels vertex by vertex. HP_ELEM_TENSOR selects it for ins, HP_ELEM_POINT for ins
- * at p = 1; HP_ELEM_SCALAR: the sum-factorised warp kernel, one warp or lane group per
- * triangle. All give the reference's residual up to rounding. HP_ENOTSUP when the kernel
- * cannot be selected for the context's physics and p. */
+ * small levels vertex by vertex. HP_ELEM_TENSOR selects it (the names are those of the kernels
+ * that the values selected at first), and so does HP_ELEM_POINT for ins at p = 1;
+ * HP_ELEM_SCALAR: the sum-factorised warp kernel, one warp or lane group per
+ * triangle. All give the reference's residual up to rounding. HP_ENOTSUP for HP_ELEM_POINT
+ * on cd or at p > 1. */
 #define HP_ELEM_SCALAR 0
 #define HP_ELEM_TENSOR 1
 #define HP_ELEM_POINT 2

@@ -1,4 +1,5 @@
-"""Options of a level that choose what its residual runs on: the stored operators at p = 1.
+"""Options of a level that choose what its residual runs on: the stored operators at p = 1, the element
+kernel of cd.
 
 Tolerance of the residuals: 1e-12 of the largest value, as in test_gpu_parity.py."""
 import numpy as np
@@ -41,3 +42,20 @@ def test_stored_operators_are_applied_at_p1(n):
     assert np.array_equal(_vec(a.state()), _vec(b.state()))
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("p", [1, 2, 4])
+def test_cd_returns_from_the_scalar_kernel(p):
+    pr = hpb.cd_sinsin(n=7, p=p, kcond=1e-2, src=0.7)
+    g, o = pr.gpu(), Oracle(pr)
+    assert g.setup_preconditioner() == 0 and o.setup_preconditioner() == 0
+    res = []
+    for kind in (None, "scalar", "tensor"):
+        if kind:
+            g.element_kernel(kind)
+        g.rsdl(pr.phys.nstage)
+        o.rsdl(pr.phys.nstage)
+        res.append(_vec(g.residual()))
+        assert relerr(g.residual(), o.residual()) < 1e-12, kind
+    assert np.array_equal(res[0], res[2])
+    g.close()
