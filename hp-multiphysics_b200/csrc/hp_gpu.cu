@@ -113,7 +113,7 @@ inline int nblk(long n, int t) { return (int)((n + t - 1) / t); }
 
 // Launch shapes chosen per context (per mesh level) and precision by hp_gpu_autotune.
 struct Tune {
-    int elem_cap = 16;       // matrix-free element kernel: CTAs per SM at most
+    int elem_cap = 16;       // scalar element kernel: CTAs per SM at most
     int emat_tpp = 1;        // stored-operator kernel: tiles per pipeline phase (1 or 2)
     int emat_ctas = 0;       // stored-operator kernel: CTAs per SM (0 = as many as fit)
     int minv_threads = 128;  // minvrt kernels: threads per CTA
@@ -2184,7 +2184,7 @@ extern "C" int hp_gpu_solve_mg_mixed(hp_gpu_ctx **levels, int nlevels, double dr
 // ---------------------------------------------------------------------------
 // Launch-shape autotuner. Each context is one mesh level at one p, so the best
 // shapes differ between the levels of a hierarchy: the tuner times the candidate
-// shapes of this context's element part (matrix-free kernel: CTAs per SM; stored
+// shapes of this context's element part (scalar kernel, where one runs: CTAs per SM; stored
 // operators: tiles per phase x CTAs per SM) and of its minvrt kernels (threads per
 // CTA) on its own mesh, in FP64 and FP32, and keeps the fastest of each.
 // ---------------------------------------------------------------------------
@@ -2205,10 +2205,14 @@ static int tune_prec(hp_gpu_ctx *c, const Launchers<R> &L, const void *tab, cons
         return ms / reps;
     };
     const int ns = ph.nstage;
-    auto elem = [&]() { launch_elem<R>(c, L, tab, st, ph, ns, 1, diff); };
+    const bool emat = emat_used(c, ph, diff), fused = p1_fused(c) && !emat;
+    auto elem = [&]() {
+        if (fused) enqueue_rsdl_folded<R>(c, L, tab, st, ph, ns, diff);
+        else launch_elem<R>(c, L, tab, st, ph, ns, 1, diff);
+    };
     Tune keep = tn;
     float best = 1e30f;
-    if (emat_used(c, ph, diff)) {
+    if (emat) {
         const int tpps[2] = {1, 2}, ctas[3] = {0, 4, 2};
         for (int a : tpps)
             for (int b : ctas) {
@@ -2217,13 +2221,15 @@ static int tune_prec(hp_gpu_ctx *c, const Launchers<R> &L, const void *tab, cons
                 const float t = time(elem);
                 if (t < best) { best = t; keep = tn; }
             }
-    } else {
+    } else if (c->elem_kind == HP_ELEM_SCALAR || c->ncurved > 0) {
         const int caps[3] = {4, 8, 16};
         for (int a : caps) {
             tn.elem_cap = a;
             const float t = time(elem);
             if (t < best) { best = t; keep = tn; }
         }
+    } else {
+        best = time(elem);  // the line kernel and the p = 1 stage have one launch shape
     }
     tn = keep;
     ms_out[0] = best;

@@ -340,9 +340,12 @@ int hp_gpu_fp32_updates(hp_gpu_ctx *ctx, int n);
  * per-level tile-shape choice). Each context is one mesh level at one p, so the
  * fastest launch shapes differ between the levels of a hierarchy. Times, on this
  * context's own mesh, `reps` launches of each candidate shape of
- *   the element part: matrix-free kernel CTAs per SM in {4, 8, 16}, or with stored
- *     cd operators tiles per pipeline phase {1, 2} x CTAs per SM {all that fit, 4, 2};
- *   the minvrt kernels: threads per CTA {64, 128, 256};
+ *   the element part: CTAs per SM of the scalar kernel in {4, 8, 16} where it runs
+ *     (HP_ELEM_SCALAR, curved triangles), or with stored cd operators tiles per pipeline
+ *     phase {1, 2} x CTAs per SM {all that fit, 4, 2}; the line kernel and the p = 1 stage
+ *     have one shape, which is timed (the stage with its vertex phase);
+ *   the minvrt kernels: threads per CTA {64, 128, 256} (at p = 1 of hp_gpu_minvrt and
+ *     HP_ELEM_SCALAR);
  * in FP64 and in FP32 (allocating the FP32 smoother state), and keeps the fastest
  * for every later launch of that precision. Results do not depend on the shapes
  * beyond rounding of the atomic scatter. Needs setup_preconditioner(); leaves the

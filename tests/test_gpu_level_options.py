@@ -1,5 +1,5 @@
 """Options of a level that choose what its residual runs on: the stored operators at p = 1, the element
-kernel of cd.
+kernel of cd, the launch shapes of the tuner.
 
 Tolerance of the residuals: 1e-12 of the largest value, as in test_gpu_parity.py."""
 import numpy as np
@@ -58,4 +58,29 @@ def test_cd_returns_from_the_scalar_kernel(p):
         res.append(_vec(g.residual()))
         assert relerr(g.residual(), o.residual()) < 1e-12, kind
     assert np.array_equal(res[0], res[2])
+    g.close()
+
+
+@pytest.mark.parametrize("kind,p,tuned", [("ins", 1, False), ("ins", 4, False), ("cd", 2, False),
+                                          ("scalar", 3, True), ("cylinder", 2, True)])
+def test_tuner_keeps_shapes_that_no_kernel_reads(kind, p, tuned):
+    """The CTAs an SM of the scalar kernel are tuned where it runs (asked for, or curved triangles),
+    and stay at the default elsewhere, however the timings fall."""
+    if kind == "cylinder":
+        pr = hpb.channel_cylinder_ins(scale=8.0, p=p)
+    else:
+        pr = hpb.cd_sinsin(n=9, p=p, kcond=1e-2) if kind == "cd" else hpb.kovasznay_ins(n=9, p=p)
+    g = pr.gpu()
+    if kind == "scalar":
+        g.element_kernel("scalar")
+    assert g.setup_preconditioner() == 0
+    default = {prec: t["elem_cap"] for prec, t in g.tuning().items()}
+    for _ in range(4):
+        t = g.autotune(reps=1)
+        for prec in ("fp64", "fp32"):
+            assert t[prec]["elem_ms"] > 0 and t[prec]["minv_ms"] > 0
+            if tuned:
+                assert t[prec]["elem_cap"] in (4, 8, 16)
+            else:
+                assert t[prec]["elem_cap"] == default[prec]
     g.close()
