@@ -1019,7 +1019,12 @@ __global__ void k_prcn_gather(Mesh mesh, State<R> st, int NV, int with_s, R vdia
     }
 }
 
-// Order-preserving key of a non-negative floating value (for atomicMax).
+// The larger of two values, NaN where one of them is: residual maxima, which must not lose a diverged
+// vertex. (A vertex without triangles has no residual, 0 / 0 in its place, and is left out of them.)
+template <typename R>
+__device__ __forceinline__ R max_nan(R a, R b) { return a > b || a != a ? a : b; }
+
+// Order-preserving key of a non-negative floating value (for atomicMax); NaN lies above all others.
 __device__ __forceinline__ unsigned long long ord_key(double v) { return (unsigned long long)__double_as_longlong(v); }
 __device__ __forceinline__ unsigned long long ord_key(float v) { return (unsigned long long)__double_as_longlong((double)v); }
 
@@ -1075,11 +1080,8 @@ __global__ void k_minv_vert(Mesh mesh, State<R> st, const DevMinv<R> *__restrict
     }
     if (maxres_slot) {
         for (int n = 0; n < NV; ++n) {
-            R a = active ? fabs(r[n]) : (R)0;
-            for (int o = 16; o > 0; o >>= 1) {
-                R b = __shfl_xor_sync(0xffffffffu, a, o);
-                a = a > b ? a : b;
-            }
+            R a = active && mesh.vt_ptr[v + 1] > mesh.vt_ptr[v] ? fabs(r[n]) : (R)0;
+            for (int o = 16; o > 0; o >>= 1) a = max_nan(a, __shfl_xor_sync(0xffffffffu, a, o));
             if ((threadIdx.x & 31) == 0) atomicMax(&maxres_slot[n], ord_key(a));
         }
     }
@@ -1154,11 +1156,8 @@ __global__ void k_minv_vert_coop(Mesh mesh, State<R> st, const DevMinv<R> *__res
     if (maxres_slot) {
 #pragma unroll
         for (int n = 0; n < NV; ++n) {
-            R a = fabs(r[n]);
-            for (int o = 16; o > 0; o >>= 1) {
-                R b = __shfl_xor_sync(0xffffffffu, a, o);
-                a = a > b ? a : b;
-            }
+            R a = mesh.vt_ptr[v + 1] > mesh.vt_ptr[v] ? fabs(r[n]) : (R)0;
+            for (int o = 16; o > 0; o >>= 1) a = max_nan(a, __shfl_xor_sync(0xffffffffu, a, o));
             if ((threadIdx.x & 31) == 0) atomicMax(&maxres_slot[n], ord_key(a));
         }
     }
@@ -1609,8 +1608,7 @@ static __global__ void k_hist_advance(unsigned long long *slot, double *hist, in
     if (threadIdx.x == 0 && blockIdx.x == 0) {
         double mx = 0.0;
         for (int n = 0; n < NV; ++n) {
-            const double v = __longlong_as_double((long long)slot[n]);
-            mx = v > mx ? v : mx;
+            mx = max_nan(mx, __longlong_as_double((long long)slot[n]));
             slot[n] = 0ull;
         }
         const int k = *it;

@@ -235,8 +235,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 8 ? 5 : 6)
                 r *= s.vprcn[g];
                 if (mesh.vess[v] & (1 << lane)) r = (R)0;
                 s.u_out[g] = s.u0[g] - s.cfla * r;
-                const R ar = fabs(r);
-                rmax = ar > rmax ? ar : rmax;
+                if (nt > 0) rmax = max_nan(rmax, (R)fabs(r));
             }
             if (s.res) s.res[g] = r;
         }
@@ -247,7 +246,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 8 ? 5 : 6)
         __syncthreads();
         if (threadIdx.x < NV) {
             R a = sm[0][threadIdx.x];
-            for (int w = 1; w < 4; ++w) a = sm[w][threadIdx.x] > a ? sm[w][threadIdx.x] : a;
+            for (int w = 1; w < 4; ++w) a = max_nan(a, sm[w][threadIdx.x]);
             atomicMax(&s.slot[threadIdx.x], ord_key(a));
         }
     }
@@ -287,7 +286,7 @@ __global__ void __launch_bounds__(128)
             r *= s.vprcn[g];
             if (mesh.vess[v] & (1 << n)) r = (R)0;
             s.u_out[g] = s.u0[g] - s.cfla * r;
-            ar = fabs(r);
+            if (j1 > mesh.vt_ptr[v]) ar = fabs(r);
         }
         if (s.res) s.res[g] = r;
     }
