@@ -135,7 +135,7 @@ __global__ void k_mlp_backward(Dims d, const float *__restrict__ pbf, const floa
 // A warp takes 32 samples, two fragments of 16: each layer's C fragments (+ bias, ReLU, rounded to
 // BF16) are the next layer's A fragments as they sit in the registers (n-tiles 2t and 2t + 1 of
 // the output are k-step t of the next product); the weights are the B operands, in fragment order
-// (k_pack_frag, whenever the weights change) so that a CTA copies them to shared memory as they
+// (k_round_pack, whenever the weights change) so that a CTA copies them to shared memory as they
 // are and one 16-byte load per lane feeds four products; the 64 -> 1 output layer is a dot product
 // per sample summed over the four lanes that hold a row. Same arithmetic as forward_one up to the
 // order of the FP32 sums. Bound by the issue of the products and of the ReLU and rounding between
@@ -159,22 +159,6 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const unsigned (&a)[4], 
 
 // k-steps of the hidden layers: two for the inputs (K padded to 32), four for each further layer
 __host__ __device__ inline int frag_steps(const Dims &d) { return 2 + 4 * (d.L - 2); }
-
-// The hidden layers' weights in B-fragment order: lane (g, t) of n-tile nt, k-step ks holds
-// W[8 nt + g][16 ks + 2 t + {0, 1}] and W[8 nt + g][16 ks + 8 + 2 t + {0, 1}] (zero beyond the inputs).
-__global__ void k_pack_frag(Dims d, const float *__restrict__ pbf, uint4 *__restrict__ frag) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= frag_steps(d) * kFragStep) return;
-    const int lane = k & 31, pr = (k >> 5) & 3, s = k >> 7, g = lane >> 2, t = lane & 3;
-    const int l = s < 2 ? 0 : 1 + (s - 2) / 4, ks = s < 2 ? s : (s - 2) % 4, ni = d.n[l];
-    unsigned w[4];
-    for (int q = 0; q < 4; ++q) {
-        const float *row = pbf + d.woff[l] + ((2 * pr + (q >> 1)) * 8 + g) * ni;
-        const int i = ks * 16 + (q & 1) * 8 + 2 * t;
-        w[q] = pack_bf16(i < ni ? row[i] : 0.f, i + 1 < ni ? row[i + 1] : 0.f);
-    }
-    frag[k] = make_uint4(w[0], w[1], w[2], w[3]);
-}
 
 __global__ void __launch_bounds__(128, 3) k_mlp_forward_mma(Dims d, const float *__restrict__ pbf,
                                                             const uint4 *__restrict__ frag,
@@ -314,9 +298,23 @@ static size_t mma_smem(const Dims &d) {
            (size_t)4 * 32 * d.n[0] * 4;
 }
 
-__global__ void k_round_bf16(const float *w, float *wb, int n) {
+// The BF16 forms of the weights, in one launch (a launch of its own for the fragments made a training
+// step of a small network 212 -> 220 us): wb, the parameters rounded, and frag (mma_shape, else
+// NULL), the hidden layers' weights in B-fragment order: lane (g, t) of n-tile nt, k-step ks holds
+// W[8 nt + g][16 ks + 2 t + {0, 1}] and W[8 nt + g][16 ks + 8 + 2 t + {0, 1}] (zero beyond the inputs).
+__global__ void k_round_pack(Dims d, const float *__restrict__ w, float *__restrict__ wb, uint4 *__restrict__ frag) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < n) wb[k] = bf(w[k]);
+    if (k < d.nparam) wb[k] = bf(w[k]);
+    if (!frag || k >= frag_steps(d) * kFragStep) return;
+    const int lane = k & 31, pr = (k >> 5) & 3, s = k >> 7, g = lane >> 2, t = lane & 3;
+    const int l = s < 2 ? 0 : 1 + (s - 2) / 4, ks = s < 2 ? s : (s - 2) % 4, ni = d.n[l];
+    unsigned v[4];
+    for (int q = 0; q < 4; ++q) {
+        const float *row = w + d.woff[l] + ((2 * pr + (q >> 1)) * 8 + g) * ni;
+        const int i = ks * 16 + (q & 1) * 8 + 2 * t;
+        v[q] = pack_bf16(i < ni ? row[i] : 0.f, i + 1 < ni ? row[i + 1] : 0.f);
+    }
+    frag[k] = make_uint4(v[0], v[1], v[2], v[3]);
 }
 
 __global__ void k_adam(float *w, const float *g, float *m, float *v, int n, float lr, float b1, float b2, float eps,
@@ -356,12 +354,8 @@ static int merr(int code, const char *m) {
 
 // The BF16 forms of the weights after they changed (stream 0).
 static void refresh_bf16(hp_mlp *net) {
-    const int P = net->d.nparam;
-    k_round_bf16<<<(P + 255) / 256, 256>>>(net->w, net->wb, P);
-    if (net->frag) {
-        const int nf = frag_steps(net->d) * kFragStep;
-        k_pack_frag<<<(nf + 127) / 128, 128>>>(net->d, net->wb, net->frag);
-    }
+    const int n = std::max(net->d.nparam, net->frag ? frag_steps(net->d) * kFragStep : 0);
+    k_round_pack<<<(n + 127) / 128, 128>>>(net->d, net->w, net->wb, net->frag);
 }
 
 extern "C" int hp_mlp_create(int nlayers, const int *widths, unsigned long long seed, hp_mlp **out) {
