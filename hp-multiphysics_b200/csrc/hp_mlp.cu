@@ -337,6 +337,7 @@ struct hp_mlp {
           *loss = nullptr;
     uint4 *frag = nullptr;  // the hidden layers' weights in fragment order (mma_shape)
     int step = 0;
+    int nsm = 148;  // of the network's device
 };
 
 extern "C" const char *hp_mlp_last_error(void) { return g_mlp_err.c_str(); }
@@ -361,6 +362,10 @@ static void refresh_bf16(hp_mlp *net) {
 extern "C" int hp_mlp_create(int nlayers, const int *widths, unsigned long long seed, hp_mlp **out) {
     if (!widths || !out || nlayers < 1 || nlayers > kMaxLayers) return merr(HP_EINVAL, "bad layer count");
     hp_mlp *net = new hp_mlp();
+    int device = 0, nsm = 0;
+    cudaGetDevice(&device);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
+    if (nsm > 0) net->nsm = nsm;
     Dims &d = net->d;
     d.L = nlayers;
     int off = 0;
@@ -456,7 +461,7 @@ extern "C" int hp_mlp_forward(hp_mlp *net, const float *d_x, int n, float *d_y, 
             MCK(cudaFuncSetAttribute(k_mlp_forward_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smm));
         // as many CTAs as are resident: the weights are staged once per CTA
         const long groups = ((long)n + 31) / 32;
-        const int blocks = (int)std::min<long>((groups + 3) / 4, 148L * 3);
+        const int blocks = (int)std::min<long>((groups + 3) / 4, 3L * net->nsm);
         k_mlp_forward_mma<<<blocks, 128, smm, st>>>(net->d, net->wb, net->frag, net->mean, net->istd, d_x, n, d_y);
         MCK(cudaGetLastError());
         return HP_OK;
