@@ -1267,7 +1267,7 @@ __global__ void k_minv_int_flat(Mesh mesh, State<R> st, const DevMinv<R> *__rest
     // the tables in shared memory, staged per block
     __shared__ R s_bfmi[3 + 3 * SM][IM], s_idiag[IM][2];
     for (int x = threadIdx.x; x < (3 + 3 * SM) * IM; x += blockDim.x) s_bfmi[x / IM][x % IM] = mt->bfmi[x / IM][x % IM];
-    for (int x = threadIdx.x; x < 2 * IM; x += blockDim.x) s_idiag[x / 2][x % 2] = x % 2 ? (R)1 / mt->idiag[x / 2][1] : mt->idiag[x / 2][0];
+    for (int x = threadIdx.x; x < 2 * IM; x += blockDim.x) s_idiag[x / 2][x % 2] = mt->idiag[x / 2][x % 2];
     __syncthreads();
     const long gid = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (gid >= (long)mesh.ntri * NV) return;
@@ -1275,20 +1275,19 @@ __global__ void k_minv_int_flat(Mesh mesh, State<R> st, const DevMinv<R> *__rest
     R b[IM];
 #pragma unroll
     for (int k = 0; k < IM; ++k) b[k] = st.resi[((size_t)t * IM + k) * NV + n];
-    // (s_idiag[i][1] holds the reciprocal: a thread had 3 IM divisions)
 #pragma unroll
     for (int i = 0; i < IM; ++i) {
         if (i >= 1) b[i] -= s_idiag[i][0] * b[0];
-        b[i] *= s_idiag[i][1];
+        b[i] /= s_idiag[i][1];
     }
 #pragma unroll
     for (int i = IM - 1; i >= 0; --i) {
-        b[i] *= s_idiag[i][1];
+        b[i] /= s_idiag[i][1];
         if (i >= 1) b[0] -= s_idiag[i][0] * b[i];
     }
-    const R tp = (R)1 / st.tprcn[t * NV + n];
+    const R tp = st.tprcn[t * NV + n];
 #pragma unroll
-    for (int k = 0; k < IM; ++k) b[k] *= tp;
+    for (int k = 0; k < IM; ++k) b[k] /= tp;
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
         const R u = st.resv[mesh.tri_pnt[3 * t + i] * NV + n];
