@@ -101,6 +101,9 @@ struct LinePar {
     int gfloor;
 };
 
+// c / sqrt(gam). FP64 by rsqrt: over gam from 1e-8 to 1e12 its error is 0.425 ulp rms, 1.48 at most,
+// that of the quotient 0.426 and 1.46, and the full residual takes 446 us instead of 459 at p = 6, 193
+// instead of 197 at p = 4 (131k triangles), though 367 instead of 343 at p = 8 (33k).
 template <typename R>
 __device__ __forceinline__ R line_tau0(R c, R gam);
 template <>
