@@ -2,8 +2,9 @@
 //
 // tri_hp::rsdl's element loop (tri_hp/nstage.cpp:52-73: ugtouht, element_rsdl, lftog) with
 // tri_hp_ins::element_rsdl's straight-element branch (tri_hp/ins/rsdl.cpp:259-433) or
-// tri_hp_cd::element_rsdl (tri_hp/cd/rsdl.cpp:14-154, CONST_A) and the tri_basis operators it calls (proj.cpp:22-119, intgrt.cpp:81-158, derivr / derivs
-// proj.cpp:339-402), FP64 or FP32, plain or correction form.
+// tri_hp_cd::element_rsdl (tri_hp/cd/rsdl.cpp:14-154, CONST_A) and the tri_basis operators they
+// call (proj.cpp:22-119, intgrt.cpp:81-158, derivr / derivs proj.cpp:339-402), FP64 or FP32, plain
+// or correction form.
 //
 // A CTA takes batches of 32 triangles, lane = triangle, and has one warp per eta point j: a
 // thread owns the line (triangle, j) of the tensor-product points. Everything that is not per
@@ -22,17 +23,19 @@
 // Why vector FMAs: on B200 the FP64 tensor instruction runs on the FP64 pipe at its rate (measured
 // 37.0 TFLOP/s against 34.5 for DFMA, and 31 in sum when mixed), so the dense per-point operators
 // that a fragment needs (98k flops per triangle at p = 6 with the padding) lose to the
-// sum-factorised form (about 40k). Measured, FP64, 131k triangles, full residual, against two
-// triangles per warp on mma.m8n8k4.f64: p = 3 157 -> 91 us, p = 4 308 -> 166, p = 5 503 -> 246,
-// p = 6 719 -> 413, p = 8 1884 -> 1169; p = 2 against the scalar warp kernel 197 -> 50 (the boundary
-// fluxes, a kernel of their own before, included). Bound by
-// issue: the FP64 pipe is busy 33 % (p = 6) to 41 % (p = 3) of the time; 7 to 16 warps an SM fit.
+// sum-factorised form (43.6k as the reference's loops are counted). Measured, FP64, 131k triangles,
+// full residual, against two triangles per warp on mma.m8n8k4.f64: p = 3 157 -> 91 us, p = 4
+// 308 -> 168, p = 5 503 -> 249, p = 6 719 -> 409, p = 8 1884 -> 1236; p = 2 against the scalar warp
+// kernel 197 -> 50 (the boundary fluxes, a kernel of their own before, included). Bound by latency
+// (fixed-length instructions, shared memory) at the 7 to 16 warps an SM that fit: at p = 6 the FP64
+// pipe is 36 % busy and the schedulers issue in 33 % of the cycles, at p = 3 the pipe is 41 % busy.
 // FP32: the same form beats TF32 fragments (mma.m16n8k8, operands rounded to 10 bits), and in
-// full FP32: an update of the FP32 smoother, 131k triangles, p = 3 728 -> 482 us, p = 4 1202 ->
-// 820, p = 6 2625 -> 2020, p = 8 7305 -> 3893, p = 2 against the scalar warp kernel 670 -> 247; in
-// plain form against the scalar warp kernel p = 6 4475 -> 1885. Bound by issue, too: half of the
-// instructions are FMAs. cd against the scalar warp kernel, an FP64 update of 80k triangles: p = 1
-// 126 -> 68 us (with k_vert_p1), p = 2 282 -> 121, p = 4 739 -> 322; p = 6 of 20k 626 -> 330.
+// full FP32: an update of the FP32 smoother, 131k triangles, p = 3 728 -> 464 us, p = 4 1202 ->
+// 796, p = 6 2625 -> 1901, p = 8 7305 -> 3835, p = 2 against the scalar warp kernel 670 -> 236; in
+// plain form against the scalar warp kernel p = 6 4475 -> 1741. Half of the instructions are FMAs.
+// cd against the scalar warp kernel, an FP64 update of 80k triangles: p = 1 126 -> 68 us (with
+// k_vert_p1), p = 2 282 -> 118, p = 4 739 -> 308; p = 6 of 20k 626 -> 320. (The pairs at the choices
+// below were measured together, when each choice was made.)
 #pragma once
 #include <utility>
 #include "hp_line.h"
@@ -46,7 +49,7 @@ struct LineCfg {
     static constexpr int NTHR = 32 * G;
     // FP64, p = 6, a stage without the real part: the modes are gathered into the exchange area, once
     // that has been read, instead of into an area of their own, so that a second CTA fits an SM (its
-    // 128 registers a thread hold what such a stage keeps; 131k triangles: 246 -> 159 us). With the
+    // 128 registers a thread hold what such a stage keeps; 131k triangles: 246 -> 160 us). With the
     // real part the point data do not fit: 404 us with two CTAs against 413, 30 against 22 us on 2k
     // triangles. p = 7, 8 need more than half of the shared memory, p <= 5 have two CTAs as it is.
     static constexpr bool TIGHT = PHYS == 1 && G == 7 && sizeof(R) == 8 && !RE;
@@ -54,7 +57,7 @@ struct LineCfg {
     static constexpr int U = NV * T * 33;                   // gathered modes [NV T][33]
     static constexpr int EX = TIGHT ? U : 2 * NV * T * 33;  // s fluxes [NV][G][G][32], then A, B [NV][2][X][G][32]
     static constexpr int LEN = EX + 2 * NV * X * G * 32;
-    static constexpr int IDX = 16 * 32;        // connectivity of a batch: pnt, seg, sgn, vpos, spos [32][3] each, tri_cv [32]
+    static constexpr int IDX = 16 * 32;  // connectivity of a batch: pnt, seg, sgn, vpos, spos [32][3], tri_cv [32]
     static constexpr int LPS = SM > 0 ? SM * NV : 1, LPI = IM > 0 ? IM * NV : 1;  // values of a side, of an interior
     static constexpr int XH = NV == 1 ? X : (X + 1) / 2;  // columns whose x sums share the registers
     static constexpr int SMEM = LEN * (int)sizeof(R) + 3 * IDX * 4;
@@ -65,8 +68,9 @@ struct LineCfg {
     // 4932, 4052
     static constexpr int by_cd = G <= 2 ? 8 : G <= 4 ? 6 : G == 5 ? 5 : G == 6 ? 4 : G == 7 ? 3 : 2;
     static constexpr int by_regs = PHYS == 0 ? (sizeof(R) == 8 ? by_cd : 2 * by_cd)
-                                 : sizeof(R) == 8 ? (G == 2 ? 8 : G == 3 ? 5 : G == 4 ? 4 : G == 5 ? 3 : G == 6 || TIGHT ? 2 : 1)
-                                                  : (G == 2 ? 12 : G == 3 ? 8 : G <= 5 ? 5 : G == 6 ? 4 : G == 7 ? 3 : 2);
+                                 : sizeof(R) == 8
+                                     ? (G == 2 ? 8 : G == 3 ? 5 : G == 4 ? 4 : G == 5 ? 3 : G == 6 || TIGHT ? 2 : 1)
+                                     : (G == 2 ? 12 : G == 3 ? 8 : G <= 5 ? 5 : G == 6 ? 4 : G == 7 ? 3 : 2);
     static constexpr int MINB = by_smem < by_regs ? (by_smem < 1 ? 1 : by_smem) : by_regs;
 };
 
@@ -262,7 +266,11 @@ __global__ void __launch_bounds__(LineCfg<R, P, PHYS, DIFF, RE>::NTHR, LineCfg<R
                 if (mesh.tri_cv) cp_async<4>(d + w, mesh.tri_cv + min(b * 32 + r, last));
                 continue;
             }
-            const int *src = a == 0 ? mesh.tri_pnt : a == 1 ? mesh.tri_seg : a == 2 ? mesh.tri_sgn : a == 3 ? mesh.vpos : mesh.spos;
+            const int *src = a == 0   ? mesh.tri_pnt
+                             : a == 1 ? mesh.tri_seg
+                             : a == 2 ? mesh.tri_sgn
+                             : a == 3 ? mesh.vpos
+                                      : mesh.spos;
             cp_async<4>(d + w, src + min(b * 96 + r, 3 * last + r % 3));
         }
     };
@@ -325,9 +333,11 @@ __global__ void __launch_bounds__(LineCfg<R, P, PHYS, DIFF, RE>::NTHR, LineCfg<R
         const R d00 = (R)lg[0], d01 = (R)lg[32], d10 = (R)lg[64], d11 = (R)lg[96];
         // ins: -mu / |J|, 2 nu / h, adis h / |J|
         const R cm = INS && RE ? (R)(-par.mu * lg[128]) : (R)0;
-        const R c5 = INS && RE ? (R)(par.nu2 * lg[192]) : (R)0, c6 = INS && RE ? (R)(par.adis * lg[160] * lg[128]) : (R)0;
+        const R c5 = INS && RE ? (R)(par.nu2 * lg[192]) : (R)0;
+        const R c6 = INS && RE ? (R)(par.adis * lg[160] * lg[128]) : (R)0;
         // cd: the velocity's r and s components, the diffusion tensor, -|J| src, tau
-        const R sr = INS ? (R)0 : d11 * (R)par.ax - d01 * (R)par.ay, ss = INS ? (R)0 : d00 * (R)par.ay - d10 * (R)par.ax;
+        const R sr = INS ? (R)0 : d11 * (R)par.ax - d01 * (R)par.ay;
+        const R ss = INS ? (R)0 : d00 * (R)par.ay - d10 * (R)par.ax;
         R k00 = (R)0, k01 = (R)0, k11 = (R)0, msrc = (R)0, taue = (R)0;
         if constexpr (!INS && RE) {
             const R kc = (R)(par.kcond * lg[128]);
@@ -517,31 +527,32 @@ __global__ void __launch_bounds__(LineCfg<R, P, PHYS, DIFF, RE>::NTHR, LineCfg<R
                     pr[0][i] = xx[i] - sr * tres + tab.x0[i] * fs;
                     ps[0][i] = fs;
                 } else {
-                R u = uq[i], v = vq[i], qv;
-                if constexpr (DIFF) {
-                    qv = bu[i] * bu[i] + bv[i] * bv[i];
-                    u += bu[i];
-                    v += bv[i];
-                } else {
-                    qv = u * u + v * v;
-                }
-                R gam = (R)3 * qv + c5 * c5;
-                if (par.gfloor) gam = gam > (R)0.1 ? gam : (R)0.1;
-                const R tau0 = line_tau0<R>(c6, gam), tau2 = sqrt(qv) * tau0;
-                const R a0 = tau0 * (n0 * res[0][i] + ex[(i * G) * 32]), a1 = tau0 * (n0 * res[1][i] + ex[((G + i) * G) * 32]),
-                        a2 = tau2 * (n0 * res[2][i] + ex[((2 * G + i) * G) * 32]);
-                // physical SUPG fluxes: x-momentum (2 u a0 + a2, v a0 + u a1), y-momentum
-                // (v a0 + u a1, 2 v a1 + a2), continuity (a0, a1)
-                const R sxx = xx[i] - ((u + u) * a0 + a2), sxy = xy[i] - (v * a0 + u * a1),
-                        syy = yy[i] - ((v + v) * a1 + a2);
-                pr[0][i] = d11 * sxx - d01 * sxy;
-                ps[0][i] = d00 * sxy - d10 * sxx;
-                pr[1][i] = d11 * sxy - d01 * syy;
-                ps[1][i] = d00 * syy - d10 * sxy;
-                pr[2][i] = d01 * a1 - d11 * a0;
-                ps[2][i] = d10 * a0 - d00 * a1;
+                    R u = uq[i], v = vq[i], qv;
+                    if constexpr (DIFF) {
+                        qv = bu[i] * bu[i] + bv[i] * bv[i];
+                        u += bu[i];
+                        v += bv[i];
+                    } else {
+                        qv = u * u + v * v;
+                    }
+                    R gam = (R)3 * qv + c5 * c5;
+                    if (par.gfloor) gam = gam > (R)0.1 ? gam : (R)0.1;
+                    const R tau0 = line_tau0<R>(c6, gam), tau2 = sqrt(qv) * tau0;
+                    const R a0 = tau0 * (n0 * res[0][i] + ex[(i * G) * 32]);
+                    const R a1 = tau0 * (n0 * res[1][i] + ex[((G + i) * G) * 32]);
+                    const R a2 = tau2 * (n0 * res[2][i] + ex[((2 * G + i) * G) * 32]);
+                    // physical SUPG fluxes: x-momentum (2 u a0 + a2, v a0 + u a1), y-momentum
+                    // (v a0 + u a1, 2 v a1 + a2), continuity (a0, a1)
+                    const R sxx = xx[i] - ((u + u) * a0 + a2), sxy = xy[i] - (v * a0 + u * a1),
+                            syy = yy[i] - ((v + v) * a1 + a2);
+                    pr[0][i] = d11 * sxx - d01 * sxy;
+                    ps[0][i] = d00 * sxy - d10 * sxx;
+                    pr[1][i] = d11 * sxy - d01 * syy;
+                    ps[1][i] = d00 * syy - d10 * sxy;
+                    pr[2][i] = d01 * a1 - d11 * a0;
+                    ps[2][i] = d10 * a0 - d00 * a1;
 #pragma unroll
-                for (int n = 0; n < 3; ++n) pr[n][i] += tab.x0[i] * ps[n][i];
+                    for (int n = 0; n < 3; ++n) pr[n][i] += tab.x0[i] * ps[n][i];
                 }
             }
             __syncthreads();  // A, B take the place of the exchanged rows

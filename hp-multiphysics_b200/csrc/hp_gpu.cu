@@ -267,9 +267,9 @@ struct LaunchImpl {
             // a lane group per vertex for its removal terms (about 6 sides x SM and 6 triangles x IM),
             // wide on small levels, where it shortens a vertex's chain of loads, and narrow on the
             // others, where it saves instructions: fewer shuffles, and the lanes that finish a vertex
-            // are a larger share. An FP64 update, cavity, wide / narrow: p = 3 4k vertices 159 / 162 us,
-            // 9k 200 / 198, 66k 736 / 675; p = 4 4k 217 / 222, 17k 379 / 375, 66k 1215 / 1160; p = 6 4k
-            // 356 / 355, 9k 548 / 523, 66k 3120 / 2942. p = 2: 2 lanes always (4 are 100 / 97 at 4k).
+            // are a larger share. An FP64 update, cavity, wide / narrow: p = 3 4k vertices 160 / 162 us,
+            // 9k 200 / 199, 66k 733 / 671; p = 4 4k 217 / 223, 17k 380 / 377, 66k 1220 / 1166; p = 6 4k
+            // 365 / 366, 9k 557 / 531, 66k 3177 / 2999. p = 2: 2 lanes always (4 are 100 / 97 at 4k).
             constexpr int WIDE = SM + IM >= 8 ? 32 : (SM + IM >= 3 ? 8 : 2), NARROW = SM + IM >= 8 ? 8 : 2;
             if (m.npnt <= 48 * nsm)
                 k_minv_vert_coop<R, NV, SM, IM, WIDE><<<nblk((long)m.npnt * WIDE, th), th, 0, st>>>(m, s, mt, (R)cfla, upd,
@@ -1802,7 +1802,7 @@ extern "C" int hp_gpu_mg_prolongate(hp_gpu_ctx *coarse) {
 // block::cycle (tri_mesh/blocks.cpp:1267-1348) over levels[0] (finest) .. levels[n-1]. The count of
 // bad elements is read at every set-up, before anything uses the preconditioner: a level that has some
 // stops the cycle there, with the states above it as they were. (Read once after the whole cycle it saved
-// the waits, 4 % of a p = 6 W-cycle, 5 % of a cd p = 2 V-cycle, but the cycle then smoothed with stale
+// the waits, 5 % of a p = 6 W-cycle and of a cd p = 2 V-cycle, but the cycle then smoothed with stale
 // preconditioners and prolongated the result.)
 static int cycle(hp_gpu_ctx **lv, int n, int lvl, int vw, int itercrsn, int iterrfne, int eval_prcn) {
     hp_gpu_ctx *c = lv[lvl];

@@ -85,14 +85,15 @@ struct Impl {
         return e;
     }
     template <bool DIFF, bool RE>
-    static void go(const void *tab, const void *gtab, const Mesh &m, const State<R> &s, const LinePar &par, int nsm, cudaStream_t st) {
+    static void go(const void *tab, const void *gtab, const Mesh &m, const State<R> &s, const LinePar &par, int nsm,
+                   cudaStream_t st) {
         using C = LineCfg<R, P, PHYS, DIFF, RE>;
         const int nb = (m.ntri + 31) / 32;
         k_rsdl_line<R, P, PHYS, DIFF, RE><<<std::min(nb, nsm * C::MINB), C::NTHR, C::SMEM, st>>>(
             *static_cast<const LineTab<R, P> *>(tab), static_cast<const DevTables<R, P> *>(gtab), m, s, par);
     }
-    static void launch(const void *tab, const void *gtab, const Mesh &m, const State<R> &s, const Phys &ph, int stage, int zero_rr,
-                       int diff, int nsm, cudaStream_t st) {
+    static void launch(const void *tab, const void *gtab, const Mesh &m, const State<R> &s, const Phys &ph, int stage,
+                       int zero_rr, int diff, int nsm, cudaStream_t st) {
         LinePar par;
         par.beta = ph.beta[stage];
         par.omb = zero_rr ? 0.0 : (double)((R)1 - (R)ph.beta[stage]);

@@ -37,8 +37,8 @@ struct LineLaunch {
     // level's DevTables on the device (ins at p > 1: the boundary fluxes, too)
     void (*build)(const hp_basis_tables &, std::vector<unsigned char> &tab) = nullptr;
     cudaError_t (*set_smem)() = nullptr;
-    void (*launch)(const void *tab, const void *dev_tables, const Mesh &, const State<R> &, const Phys &, int stage, int zero_rr, int diff,
-                   int nsm, cudaStream_t) = nullptr;
+    void (*launch)(const void *tab, const void *dev_tables, const Mesh &, const State<R> &, const Phys &, int stage,
+                   int zero_rr, int diff, int nsm, cudaStream_t) = nullptr;
     // FP32: the base state's point values of the correction form (State::bpt), their number
     void (*base_pts)(const void *dev_tables, const Mesh &, const State<R> &, R *bpt, cudaStream_t) = nullptr;
     size_t (*bpt_len)(int ntri) = nullptr;

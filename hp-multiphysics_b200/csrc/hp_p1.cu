@@ -57,8 +57,8 @@ void p1_vert(const P1Ops<R> *ops, const Mesh &m, const R *elim, const R *elre, c
     else if (diff) k_vert_p1<R, 1, true><<<blocks, 128, 0, str>>>(ops, m, elim, elre, s, ph);
     else k_vert_p1<R, 1, false><<<blocks, 128, 0, str>>>(ops, m, elim, elre, s, ph);
 }
-template void p1_vert<double>(const P1Ops<double> *, const Mesh &, const double *, const double *, const P1Stage<double> &,
-                              const Phys &, int, cudaStream_t);
+template void p1_vert<double>(const P1Ops<double> *, const Mesh &, const double *, const double *,
+                              const P1Stage<double> &, const Phys &, int, cudaStream_t);
 template void p1_vert<float>(const P1Ops<float> *, const Mesh &, const float *, const float *, const P1Stage<float> &,
                              const Phys &, int, cudaStream_t);
 

@@ -7,9 +7,11 @@
 
 namespace hpb {
 
-// The operators at p = 1 (G = 2, T = 3) as dense arrays, q = 2 i + j, as InsP1Ops, with the weights
-// of intgrt W0[q][m] and the boundary side's tables at its Gauss points: values and derivatives of
-// the two end functions BG, BD [k][end], integration weights BW [k][end].
+// The operators at p = 1 (G = 2, T = 3) as dense arrays over the points q = 2 i + j: values V and
+// derivatives DR, DS of the modes, weights of the r and s fluxes WR, WS, those of intgrt W0; the 1D
+// derivative operators AR, AS1, AS2 and factors N0 of the strong residual; the boundary side's
+// tables at its Gauss points: values and derivatives of the two end functions BG, BD [k][end],
+// integration weights BW [k][end].
 template <typename R>
 struct P1Ops {
     R V[4][3], DR[4][3], DS[4][3], WR[4][3], WS[4][3], W0[4][3];
@@ -35,8 +37,8 @@ void p1_ops(const hp_basis_tables &, P1Ops<R> &);
 
 // Whether a level's stage runs vertex by vertex (k_stage_p1): its vertices, one warp each, are two
 // waves of the resident warps at most. Measured per update (five stages), vertex by vertex / element
-// kernel and k_vert_p1: FP64 4225 vertices 48 / 54 us, 66k vertices 367 / 141; FP32 4225 vertices
-// 38 / 57, 66k vertices 251 / 116.
+// kernel and k_vert_p1: FP64 4225 vertices 49 / 55 us, 66k vertices 390 / 143; FP32 4225 vertices
+// 38 / 57, 66k vertices 252 / 116.
 template <typename R>
 bool p1_small(const Mesh &m, int nsm) {
     return m.npnt <= 2 * nsm * (sizeof(R) == 8 ? 20 : 24);

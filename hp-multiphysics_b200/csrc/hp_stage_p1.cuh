@@ -4,17 +4,18 @@
 // boundary fluxes (hp_edge_bdry::rsdl, hp_boundary.cpp:973-1049), tri_hp::minvrt
 // (setup_preconditioner.cpp:102-373) and the stage update (nstage.cpp:387-409) of a vertex need
 // only the triangles around it. A warp takes a vertex: lane 4 e + q evaluates Gauss point
-// q = 2 i + j of the vertex's triangle e (eight at a time) with the dense per-point operators, and keeps its share of the one test function that belongs to the vertex; the
-// shares are summed by shuffles in a fixed order and lane n finishes variable n. A triangle is
-// evaluated three times, once for each of its vertices, and nothing goes through memory between
-// the element loop and the update: the separate kernels (element, boundary flux, assembly, vertex
-// phase) were a chain of four launches of 5 to 10 us each, latency and not work. The state is read
-// from one buffer and written to another (neighbours are read), see p1_update.
-// For small levels (p1_small); larger ones take the element kernel and
-// k_vert_p1, since the threefold evaluation then costs more than the launch it saves.
-// Measured per FP64 update (five stages): 512 triangles 86 -> 29 us, 8192 triangles 89 -> 48 us,
-// 131k triangles 212 -> 367 us, where the element kernel and k_vert_p1 take 141 (hence the rule). Bound by latency (vertex -> incidence -> state
-// loads, then the FP64 chain of a point).
+// q = 2 i + j of the vertex's triangle e (eight at a time) with the dense per-point operators, and
+// keeps its share of the one test function that belongs to the vertex; the shares are summed by
+// shuffles in a fixed order and lane n finishes variable n. A triangle is evaluated three times,
+// once for each of its vertices, and nothing goes through memory between the element loop and the
+// update: the separate kernels (element, boundary flux, assembly, vertex phase) were a chain of four
+// launches of 5 to 10 us each, latency and not work. The state is read from one buffer and written
+// to another (neighbours are read), see enqueue_p1_update.
+// For small levels (p1_small); larger ones take the element kernel and k_vert_p1, since the
+// threefold evaluation then costs more than the launch it saves.
+// Measured per FP64 update (five stages): 512 triangles 86 -> 29 us, 8192 triangles 89 -> 49 us,
+// 131k triangles 212 -> 390 us, where the element kernel and k_vert_p1 take 143 (hence the rule).
+// Bound by latency (vertex -> incidence -> state loads, then the FP64 chain of a point).
 #pragma once
 #include "hp_chain.cuh"
 #include "hp_p1.h"
@@ -158,7 +159,8 @@ __global__ void __launch_bounds__(128, sizeof(R) == 8 ? 5 : 6)
 #pragma unroll
                     for (int n = 0; n < 3; ++n) {
                         const R fr = fir[n] + fxr[n], fs = fis[n] + fxs[n];
-                        const R fr_oi = __shfl_xor_sync(0xffffffffu, fr, 2), fs_oi = __shfl_xor_sync(0xffffffffu, fs, 2);
+                        const R fr_oi = __shfl_xor_sync(0xffffffffu, fr, 2);
+                        const R fs_oi = __shfl_xor_sync(0xffffffffu, fs, 2);
                         const R fs_oj = __shfl_xor_sync(0xffffffffu, fs, 1);
                         res[n] = n0j * (ar_ii * fr + ar_io * fr_oi + as1_ii * fs + as1_io * fs_oi) +
                                  (as2_jj * fs + as2_jo * fs_oj);

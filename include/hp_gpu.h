@@ -223,7 +223,8 @@ int hp_gpu_enqueue_update(hp_gpu_ctx *ctx);
 int hp_gpu_enqueue_upload_state(hp_gpu_ctx *ctx, const double *ugv, const double *ugs, const double *ugi);
 int hp_gpu_enqueue_download_residual(hp_gpu_ctx *ctx, double *resv, double *ress, double *resi);
 /* The element-residual kernel alone (the loop over elements of tri_hp::rsdl,
- * nstage.cpp:52-73: ugtouht, element_rsdl, lftog), for timing it in isolation. */
+ * nstage.cpp:52-73: ugtouht, element_rsdl, lftog), for timing it in isolation. The line
+ * kernel of ins at p > 1 evaluates the boundary fluxes, too. */
 int hp_gpu_enqueue_element_rsdl(hp_gpu_ctx *ctx, int stage);
 
 /* Stored element operators for the linear cd residual. No counterpart in the
@@ -233,7 +234,11 @@ int hp_gpu_enqueue_element_rsdl(hp_gpu_ctx *ctx, int stage);
  * so on = 1 builds A_im, A_re, b_re of every element once (FP64 by the element
  * kernel applied to unit vectors, plus an FP32 copy for the FP32 smoother), and
  * every later rsdl of either precision becomes a streamed batched mat-vec with
- * the same result up to rounding. The build needs tau: it runs
+ * the same result up to rounding. It pays at p = 1 on large levels and about breaks even at
+ * p = 2; from p = 3 on the matrix-free line kernel is the faster one. 80,000 triangles, matrix-free /
+ * stored: FP64 rsdl p = 1 17 / 11 us, p = 2 21 / 19, p = 3 29 / 46, p = 4 41 / 81, p = 6 114 / 200,
+ * p = 8 250 / 480; an FP32 update 71 / 55, 142 / 131, 224 / 237, 311 / 386, 599 / 826, 1174 / 1550;
+ * on 512 triangles at p = 1 rsdl 6 / 10. The build needs tau: it runs
  * setup_preconditioner() first when that has not run (cd tau depends on the
  * geometry and the fixed parameters only, so the operators stay valid for every
  * later state). on = 0 returns to the matrix-free kernel (the storage is kept
@@ -290,7 +295,9 @@ int hp_gpu_mg_prolongate(hp_gpu_ctx *coarse);
 /* block::cycle (tri_mesh/blocks.cpp:1267-1348) over levels[0] (finest) ..
  * levels[nlevels-1], each attached to the previous one: vw cycles per level,
  * itercrsn updates before and iterrfne after the coarse-grid correction,
- * setup_preconditioner() on entry to each level when eval_prcn. */
+ * setup_preconditioner() on entry to each level when eval_prcn. A set-up that meets bad
+ * elements ends the cycle with HP_ESTATE ahead of that level's updates: the levels above
+ * keep the states they had then. */
 int hp_gpu_vcycle(hp_gpu_ctx **levels, int nlevels, int vw, int itercrsn, int iterrfne, int eval_prcn);
 /* Cycles until ||R64|| on levels[0] (as in hp_gpu_solve) drops by `drop` or
  * max_cycles ran; preconditioners on the first cycle and every prcn_every
